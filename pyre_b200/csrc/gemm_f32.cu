@@ -2,27 +2,47 @@
 //
 // IEEE fp32 multiply-add on the CUDA cores, no tensor-core or TF32 mode anywhere.  W has
 // the layout of a linear layer's weight ([out, in], in-dim contiguous, pyre/model.py:84-87
-// via nn.Linear).  Every output element is summed in two levels: a chain
-// part = fma(a[k], w[k], part) over each run of 32 consecutive k (from k = 0, ascending),
-// and the runs' sums added in ascending order.  The rounding error then grows with
-// K / 32 + 32 terms instead of K.  The grouping depends on k alone, whatever tile shape
-// computes it: a row's result is bit-identical for any M and any batch composition.
+// via nn.Linear).  Every output element is summed in three levels:
+//   * a run is 32 consecutive k; its even and its odd k are two chains part = fma(a[k], w[k], part), ascending, and the
+//     run's sum is even + odd (a float4 of each operand then is two fma.rn.f32x2, without a move);
+//   * chain c of eight adds the sums of the runs c, c + 8, c + 16, ... in ascending order;
+//   * the eight chains are added in ascending order.
+// The rounding error grows with 16 + K / 256 + 8 terms instead of K.  The grouping depends on k alone, whatever kernel
+// or tile shape computes it: a row's result is bit-identical for any M and any batch composition.  The chains are
+// what the kernels divide among threads (few rows) or CTAs (few tiles) without changing a bit.
 //
 // Three kernels, the same arithmetic in each:
-//   * many rows, rows of both operands 16-byte aligned and K a multiple of 4: 128 x 128 tiles, 8 x 8 per thread,
-//     16 k per step fetched as float4 into registers one step ahead and stored transposed into the other half of a
-//     double-buffered shared-memory tile (one barrier per step);
-//   * up to 32 rows (decode), same alignment: a CTA of 128 threads owns 16 output features and streams their
-//     weight rows in runs of 32 k through a four-stage cp.async ring (a weight stream: many small CTAs keep the
-//     memory system busy, where one 128-wide tile per CTA left most SMs without work);
+//   * many rows, rows of both operands 16-byte aligned and K a multiple of 4: 64 x 64 tiles, one CTA per tile or a
+//     cluster of eight, one per chain;
+//   * up to 32 rows (decode), same alignment: a weight stream, 16 output features per CTA, the chains in different threads;
 //   * anything else: the plain tile kernel with scalar loads.
 #include "common.cuh"
 
-template <int BM, int BN, int BK, int TM, int TN>
+namespace {
+constexpr int RUN = 32, CHAINS = 8;       // the grouping of the sums, see above
+
+typedef unsigned long long f32x2;         // two floats in one 64-bit register: the even k below, the odd k above
+
+__device__ __forceinline__ void fma2(f32x2& d, f32x2 a, f32x2 b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ float run_sum(f32x2 p) {      // even + odd
+    return __uint_as_float((uint32_t)p) + __uint_as_float((uint32_t)(p >> 32));
+}
+// a 16-byte copy into shared memory, or 16 bytes of zeros
+__device__ __forceinline__ void copy16(float* dst, const float* src, bool live) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = live ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+}  // namespace
+
+template <int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 sgemm_nt_kernel(const float* A, long long lda, const float* W, long long ldw,
                 float* C, long long ldc, const float* bias, int M, int N, int K) {
-    constexpr int THREADS = (BM / TM) * (BN / TN);
+    constexpr int THREADS = (BM / TM) * (BN / TN), BK = 8;
+    static_assert(RUN % BK == 0 && BK % 2 == 0, "a run ends at a tile's end, a tile holds whole even-odd pairs");
     __shared__ float As[BK][BM + 4];
     __shared__ float Ws[BK][BN + 4];
     pdl_trigger();
@@ -31,50 +51,62 @@ sgemm_nt_kernel(const float* A, long long lda, const float* W, long long ldw,
     const int tx = tid % (BN / TN);  // column group
     const int ty = tid / (BN / TN);  // row group
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int n_runs = (K + RUN - 1) / RUN;
 
-    constexpr int RUN = 32;  // k per first-level sum; a multiple of both tile depths
-    static_assert(RUN % BK == 0, "a run of the first level must end at a tile's end");
-    float acc[TM][TN], part[TM][TN];
+    float total[TM][TN];
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = part[i][j] = 0.f;
+        for (int j = 0; j < TN; ++j) total[i][j] = 0.f;
 
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        // tile loads: consecutive threads read consecutive k of one row
-        for (int e = tid; e < BM * BK; e += THREADS) {
-            const int r = e / BK, kk = e % BK;
-            const int gm = m0 + r, gk = k0 + kk;
-            As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
-        }
-        for (int e = tid; e < BN * BK; e += THREADS) {
-            const int r = e / BK, kk = e % BK;
-            const int gn = n0 + r, gk = k0 + kk;
-            Ws[kk][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
-        }
-        __syncthreads();
+    for (int c = 0; c < CHAINS && c < n_runs; ++c) {
+        float acc[TM][TN];
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float a[TM], w[TN];
+        for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+        for (int run = c; run < n_runs; run += CHAINS) {
+            float part[2][TM][TN];
 #pragma unroll
             for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < TN; ++j) part[i][j] = fmaf(a[i], w[j], part[i][j]);
-        }
-        if ((k0 + BK) % RUN == 0 || k0 + BK >= K) {
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) {
-                    acc[i][j] += part[i][j];
-                    part[i][j] = 0.f;
+                for (int j = 0; j < TN; ++j) part[0][i][j] = part[1][i][j] = 0.f;
+            for (int k0 = run * RUN; k0 < run * RUN + RUN; k0 += BK) {
+                // tile loads: consecutive threads read consecutive k of one row
+                for (int e = tid; e < BM * BK; e += THREADS) {
+                    const int r = e / BK, kk = e % BK;
+                    const int gm = m0 + r, gk = k0 + kk;
+                    As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
                 }
+                for (int e = tid; e < BN * BK; e += THREADS) {
+                    const int r = e / BK, kk = e % BK;
+                    const int gn = n0 + r, gk = k0 + kk;
+                    Ws[kk][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
+                }
+                __syncthreads();
+#pragma unroll
+                for (int kk = 0; kk < BK; ++kk) {
+                    float a[TM], w[TN];
+#pragma unroll
+                    for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
+#pragma unroll
+                    for (int i = 0; i < TM; ++i)
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) part[kk & 1][i][j] = fmaf(a[i], w[j], part[kk & 1][i][j]);
+                }
+                __syncthreads();
+            }
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] += part[0][i][j] + part[1][i][j];
         }
-        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) total[i][j] += acc[i][j];
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
@@ -83,128 +115,211 @@ sgemm_nt_kernel(const float* A, long long lda, const float* W, long long ldw,
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
             const int gn = n0 + tx * TN + j;
-            if (gn < N) C[(size_t)gm * ldc + gn] = bias ? acc[i][j] + bias[gn] : acc[i][j];
+            if (gn < N) C[(size_t)gm * ldc + gn] = bias ? total[i][j] + bias[gn] : total[i][j];
         }
     }
 }
 
 // ---------------------------------------------------------------------------
-// Many rows: float4 loads along k, register prefetch, double-buffered shared memory.
-// A thread's 8 rows (columns) are two groups of 4, 64 apart, so that the float4 reads of eight neighbouring threads
-// cover 128 consecutive bytes of shared memory.
+// Many rows.  Bound by the FMA pipe: fma.rn.f32x2 alone, out of registers, reaches 49 TFLOP/s on this chip; a thread owns 8 x 4
+// outputs as even-odd pairs, four k cost it 12 reads of 16 bytes from shared memory and 64 fma.rn.f32x2.  128 threads on a
+// 64 x 64 tile and 168 registers put three CTAs on an SM, whose barriers and first loads hide behind one another; operands
+// arrive by cp.async, 16 k at a time and two steps ahead, in rows of 20 floats (reads of 16 bytes by eight neighbouring
+// threads cover all banks).  Measured (M x N x K): 509 x 37888 x 3584: 3905 -> 3386 us (35 -> 41 TFLOP/s); 509 x 3584 x
+// 18944: 2565 -> 1997 us; 40 x 3584 x 18944: 2505 -> 310 us (the tiles were 128 x 128, a CTA each, 8 x 8 outputs per
+// thread).  8 x 8 outputs per thread here (255 registers): 3713 us for the first, scalar fmaf in their place 3597 us.
+//
+// PARTS == 1: a CTA walks the chains one after the other (runs c, c + 8, ...) and keeps the sum of the finished ones
+// in shared memory.  PARTS == 8: the CTAs of a cluster take a chain each and add them up through distributed shared memory.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+constexpr int TILE = 64, TILE_STAGES = 3;
+
+template <int PARTS>
+__global__ void __launch_bounds__(128, 3)
 sgemm_nt_tiles_kernel(const float* A, long long lda, const float* W, long long ldw,
-                      float* C, long long ldc, const float* bias, int M, int N, int K) {
-    constexpr int BM = 128, BN = 128, BK = 16, RUN = 32;
-    __shared__ __align__(16) float As[2][BK][BM + 4];
-    __shared__ __align__(16) float Ws[2][BK][BN + 4];
+                      float* C, long long ldc, const float* bias, int M, int N, int K, int tiles_m) {
+    constexpr int BM = TILE, BN = TILE, TN = BN / 16, BK = 16, PITCH = BK + 4, STAGES = TILE_STAGES, STAGE = (BM + BN) * PITCH;
+    static_assert(PARTS == 1 || PARTS == CHAINS, "all chains in one CTA, or one in each");
+    extern __shared__ __align__(16) float tiles[];      // STAGES x STAGE, then total: BM x BN
+    float* const total = tiles + STAGES * STAGE;
     pdl_trigger();
-    pdl_wait();
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    // loads: 128 rows x 4 float4 per operand and step; a thread fetches rows lr and lr + 64, k quad lq
+    const int rank = PARTS > 1 ? blockIdx.x % PARTS : 0, tile = blockIdx.x / PARTS;
+    // the tiles of one block of weight rows follow one another: their weights come out of the L2 cache
+    const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
+    const int n_runs = (K + RUN - 1) / RUN;
+    // copies: per step 128 rows of 4 quads; a thread fetches quad lq of the rows lr, lr + 32 of both operands
     const int lr = tid >> 2, lq = tid & 3;
-    float acc[8][8], part[8][8];
+    int f_chain = rank, f_run = rank, f_half = 0, f_stage = 0;      // where the next fetch stands
+    auto fetch = [&]() {
+        if (f_run < n_runs) {
+            const int gk = f_run * RUN + f_half * BK + 4 * lq;
+            const bool in_k = gk < K;
+            float* dst = tiles + f_stage * STAGE + lr * PITCH + 4 * lq;
+            // rows outside the matrices are not stored: whatever their sums are
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+            for (int h = 0; h < BM / 32; ++h) {
+                const int gm = m0 + lr + 32 * h;
+                if (gm < M) copy16(dst + 32 * h * PITCH, in_k ? A + (size_t)gm * lda + gk : A, in_k);
+            }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = part[i][j] = 0.f;
-    float4 ra[2], rw[2];
-    auto fetch = [&](int k0) {
-        const int gk = k0 + 4 * lq;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int gm = m0 + lr + 64 * h, gn = n0 + lr + 64 * h;
-            ra[h] = (gm < M && gk < K) ? *reinterpret_cast<const float4*>(A + (size_t)gm * lda + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
-            rw[h] = (gn < N && gk < K) ? *reinterpret_cast<const float4*>(W + (size_t)gn * ldw + gk) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int h = 0; h < BN / 32; ++h) {
+                const int gn = n0 + lr + 32 * h;
+                if (gn < N) copy16(dst + (BM + 32 * h) * PITCH, in_k ? W + (size_t)gn * ldw + gk : W, in_k);
+            }
+            f_half ^= 1;
+            if (f_half == 0) {
+                f_run += CHAINS;
+                if (PARTS == 1 && f_run >= n_runs && f_chain + 1 < CHAINS) f_run = ++f_chain;
+            }
         }
+        f_stage = f_stage == STAGES - 1 ? 0 : f_stage + 1;
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    auto stash = [&](int buf) {
+    pdl_wait();
+    for (int s = 0; s < STAGES - 1; ++s) fetch();
+    float acc[8][TN];
+    int stage = 0;
+#pragma unroll 1
+    for (int chain = rank; chain < (PARTS == 1 ? CHAINS : rank + 1); ++chain) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = lr + 64 * h;
-            As[buf][4 * lq + 0][r] = ra[h].x; As[buf][4 * lq + 1][r] = ra[h].y;
-            As[buf][4 * lq + 2][r] = ra[h].z; As[buf][4 * lq + 3][r] = ra[h].w;
-            Ws[buf][4 * lq + 0][r] = rw[h].x; Ws[buf][4 * lq + 1][r] = rw[h].y;
-            Ws[buf][4 * lq + 2][r] = rw[h].z; Ws[buf][4 * lq + 3][r] = rw[h].w;
-        }
-    };
-    const int n_steps = (K + BK - 1) / BK;
-    fetch(0);
-    stash(0);
-    __syncthreads();
-    for (int t = 0; t < n_steps; ++t) {
-        const int buf = t & 1;
-        if (t + 1 < n_steps) fetch((t + 1) * BK);
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][kk][4 * ty]), a1 = *reinterpret_cast<const float4*>(&As[buf][kk][64 + 4 * ty]);
-            const float4 w0 = *reinterpret_cast<const float4*>(&Ws[buf][kk][4 * tx]), w1 = *reinterpret_cast<const float4*>(&Ws[buf][kk][64 + 4 * tx]);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+#pragma unroll 1
+        for (int run = chain; run < n_runs; run += CHAINS) {
+            f32x2 part[8][TN];
 #pragma unroll
             for (int i = 0; i < 8; ++i)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) part[i][j] = fmaf(a[i], w[j], part[i][j]);
-        }
-        if (((t + 1) * BK) % RUN == 0 || t + 1 == n_steps) {
+                for (int j = 0; j < TN; ++j) part[i][j] = 0ull;
+#pragma unroll 1
+            for (int half = 0; half < RUN / BK; ++half) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+                __syncthreads();      // this step has landed for every thread; the stage filled below was read a step ago
+                fetch();
+                const float* as = tiles + stage * STAGE + ty * PITCH;
+                const float* ws = tiles + stage * STAGE + (BM + tx) * PITCH;
+                stage = stage == STAGES - 1 ? 0 : stage + 1;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+                for (int q = 0; q < BK / 4; ++q) {
+                    ulonglong2 w[TN];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    acc[i][j] += part[i][j];
-                    part[i][j] = 0.f;
+                    for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(ws + 16 * j * PITCH + 4 * q);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + 8 * i * PITCH + 4 * q);
+#pragma unroll
+                        for (int j = 0; j < TN; ++j) {
+                            fma2(part[i][j], a.x, w[j].x);
+                            fma2(part[i][j], a.y, w[j].y);
+                        }
+                    }
                 }
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[i][j] += run_sum(part[i][j]);
         }
-        if (t + 1 < n_steps) stash(buf ^ 1);
-        __syncthreads();
+        if constexpr (PARTS == 1) {
+            // the finished chains' sum: this thread's own sums
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float4* t = reinterpret_cast<float4*>(total) + i * 128 + tid;
+                float4 v = chain == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : *t;
+                v.x += acc[i][0]; v.y += acc[i][1]; v.z += acc[i][2]; v.w += acc[i][3];
+                *t = v;
+            }
+        }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if constexpr (PARTS == 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int gm = m0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + i - 4);
-        if (gm >= M) continue;
+        for (int i = 0; i < 8; ++i) {
+            const int gm = m0 + ty + 8 * i;
+            if (gm >= M) continue;
+            const float4 v = reinterpret_cast<const float4*>(total)[i * 128 + tid];
+            const float out[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int gn = n0 + (j < 4 ? 4 * tx + j : 64 + 4 * tx + j - 4);
-            if (gn < N) C[(size_t)gm * ldc + gn] = bias ? acc[i][j] + bias[gn] : acc[i][j];
+            for (int j = 0; j < TN; ++j) {
+                const int gn = n0 + tx + 16 * j;
+                if (gn < N) C[(size_t)gm * ldc + gn] = bias ? out[j] + bias[gn] : out[j];
+            }
         }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < TN; ++j) total[(ty + 8 * i) * BN + tx + 16 * j] = acc[i][j];
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // eight rows of the tile per CTA, four neighbouring columns at a time; the chains in ascending order
+        for (int e = tid; e < (BM / PARTS) * (BN / 4); e += 128) {
+            const int row = rank * (BM / PARTS) + e / (BN / 4), col = 4 * (e % (BN / 4));
+            const uint32_t mine = (uint32_t)__cvta_generic_to_shared(total + row * BN + col);
+            float out[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int c = 0; c < PARTS; ++c) {
+                uint32_t at;
+                float4 v;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(mine), "r"(c));
+                asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+                out[0] += v.x; out[1] += v.y; out[2] += v.z; out[3] += v.w;
+            }
+            const int gm = m0 + row;
+            if (gm >= M) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int gn = n0 + col + j;
+                if (gn < N) C[(size_t)gm * ldc + gn] = bias ? out[j] + bias[gn] : out[j];
+            }
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");     // no CTA leaves while another reads its tile
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
 
 // ---------------------------------------------------------------------------
-// Few rows (MT = 8 or 32 of them per CTA): 16 output features per CTA, their weight rows and the rows of A in runs of
-// 32 k through a four-stage cp.async ring.  Thread (feature tn, row group tg) owns MT / 8 outputs; one stage is one
-// run of the first level, so a stage ends with acc += part.
+// Few rows: bound by reading the weights.  A CTA owns 16 output features; a stage is 256 k (a run of each chain: 1 KB
+// of every weight row and of every row of A) in a ring of cp.async copies, 16 KB of weights each, so that even a
+// product of few features has some 50 KB in flight on every SM.  A thread owns one chain of F features x MR rows.  Shared
+// memory is what comes next after the memory: runs are 36 floats apart and rows 292, so that eight
+// neighbouring threads (features of one run) and the runs of a warp fall on different banks.  Measured (M x N x K, weights
+// read at): 4 x 37888 x 3584: 226 -> 119 us (4.6 TB/s); 4 x 3584 x 18944: 185 -> 70 us (3.9 TB/s); 8 x 3584 x 18944: 184 -> 97 us;
+// 12 x 3584 x 18944: 723 -> 138 us; 32 x 3584 x 18944: 441 -> 213 us (a stage was one run of 32 k, a CTA's threads all walked it).
 // ---------------------------------------------------------------------------
-template <int MT>
-__global__ void __launch_bounds__(128)
+template <int MR, int F, int GROUPS, int STAGES>
+__global__ void __launch_bounds__(CHAINS * 16 / F * GROUPS)
 sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long ldw,
                        float* C, long long ldc, const float* bias, int M, int N, int K) {
-    constexpr int FN = 16, RUN = 32, STAGES = 4, PITCH = RUN + 4, PER = MT / 8;
-    __shared__ __align__(16) float Ws[STAGES][FN][PITCH];
-    __shared__ __align__(16) float As[STAGES][MT][PITCH];
+    constexpr int FN = 16, FT = FN / F, MT = MR * GROUPS, THREADS = CHAINS * FT * GROUPS;
+    constexpr int RUN_PITCH = RUN + 4, ROW = CHAINS * RUN_PITCH + 4, KS = RUN * CHAINS;
+    constexpr int STAGE = (FN + MT) * ROW, STEP = THREADS / 64;
+    static_assert(CHAINS * MT * FN <= STAGE * STAGES && THREADS % 64 == 0 && FN % STEP == 0, "copies and the last sum fit");
+    extern __shared__ __align__(16) float ring[];
     pdl_trigger();
-    const int tid = threadIdx.x, tn = tid & 15, tg = tid >> 4;
-    const int n0 = blockIdx.x * FN, m0 = blockIdx.y * MT;
-    const int n_runs = (K + RUN - 1) / RUN;
-    // a 16-byte copy, or 16 bytes of zeros where the source lies outside the matrix
-    auto copy16 = [](float* dst, const float* src, bool live) {
-        const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-        const int bytes = live ? 16 : 0;
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+    const int tid = threadIdx.x;
+    const int ft = tid % FT, chain = tid / FT % CHAINS, group = tid / (FT * CHAINS);
+    const int n0 = blockIdx.x * FN;
+    const int n_steps = (K + KS - 1) / KS;
+    // copies: a thread fetches quad cq of the rows cr, cr + STEP, ...
+    const int cq = tid & 63, cr = tid >> 6;
+    float* const to = ring + (cq >> 3) * RUN_PITCH + (cq & 7) * 4;
+    auto load_w = [&](int t, int st) {
+        const int gk = t * KS + 4 * cq;
+        const bool live = gk < K;
+        if (t >= n_steps) return;
+#pragma unroll
+        for (int r = cr; r < FN; r += STEP)      // rows outside the matrices are not stored: whatever their sums are
+            if (n0 + r < N) copy16(to + st * STAGE + r * ROW, live ? W + (size_t)(n0 + r) * ldw + gk : W, live);
     };
-    auto load_w = [&](int run, int st) {      // 16 rows x 8 quads: one per thread
-        const int r = tid >> 3, q = tid & 7, gk = run * RUN + 4 * q, gn = n0 + r;
-        const bool live = run < n_runs && gn < N && gk < K;
-        copy16(&Ws[st][r][4 * q], live ? W + (size_t)gn * ldw + gk : W, live);
-    };
-    auto load_a = [&](int run, int st) {      // MT rows x 8 quads
-        for (int e = tid; e < MT * 8; e += 128) {
-            const int r = e >> 3, q = e & 7, gk = run * RUN + 4 * q, gm = m0 + r;
-            const bool live = run < n_runs && gm < M && gk < K;
-            copy16(&As[st][r][4 * q], live ? A + (size_t)gm * lda + gk : A, live);
-        }
+    auto load_a = [&](int t, int st) {
+        const int gk = t * KS + 4 * cq;
+        const bool live = gk < K;
+        if (t >= n_steps) return;
+        for (int r = cr; r < MT; r += STEP)
+            if (r < M) copy16(to + st * STAGE + (FN + r) * ROW, live ? A + (size_t)r * lda + gk : A, live);
     };
     // the weights depend on no earlier kernel: their first stages are on their way before the wait
     for (int s = 0; s < STAGES - 1; ++s) load_w(s, s);
@@ -213,43 +328,122 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
         load_a(s, s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    float acc[PER], part[PER];
+    float acc[MR][F];
 #pragma unroll
-    for (int i = 0; i < PER; ++i) acc[i] = part[i] = 0.f;
-    for (int run = 0; run < n_runs; ++run) {
-        const int st = run % STAGES;
+    for (int i = 0; i < MR; ++i)
+#pragma unroll
+        for (int j = 0; j < F; ++j) acc[i][j] = 0.f;
+    int st = 0, fill = STAGES - 1;
+    for (int t = 0; t < n_steps; ++t) {
         asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-        __syncthreads();      // this run's stage has landed for every thread; the stage refilled below was read a run ago
-        load_w(run + STAGES - 1, (run + STAGES - 1) % STAGES);
-        load_a(run + STAGES - 1, (run + STAGES - 1) % STAGES);
+        __syncthreads();      // this stage has landed for every thread; the stage refilled below was read a step ago
+        load_w(t + STAGES - 1, fill);
+        load_a(t + STAGES - 1, fill);
+        fill = fill == STAGES - 1 ? 0 : fill + 1;
         asm volatile("cp.async.commit_group;" ::: "memory");
+        const float* ws = ring + st * STAGE + ft * ROW + chain * RUN_PITCH;
+        const float* as = ring + st * STAGE + (FN + group * MR) * ROW + chain * RUN_PITCH;
+        st = st == STAGES - 1 ? 0 : st + 1;
+        f32x2 part[MR][F];
+#pragma unroll
+        for (int i = 0; i < MR; ++i)
+#pragma unroll
+            for (int j = 0; j < F; ++j) part[i][j] = 0ull;
 #pragma unroll
         for (int q = 0; q < RUN / 4; ++q) {
-            const float4 w = *reinterpret_cast<const float4*>(&Ws[st][tn][4 * q]);
+            ulonglong2 w[F];
 #pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                const float4 a = *reinterpret_cast<const float4*>(&As[st][tg * PER + i][4 * q]);
-                part[i] = fmaf(a.x, w.x, part[i]);
-                part[i] = fmaf(a.y, w.y, part[i]);
-                part[i] = fmaf(a.z, w.z, part[i]);
-                part[i] = fmaf(a.w, w.w, part[i]);
+            for (int j = 0; j < F; ++j) w[j] = *reinterpret_cast<const ulonglong2*>(ws + j * FT * ROW + 4 * q);
+#pragma unroll
+            for (int i = 0; i < MR; ++i) {
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(as + i * ROW + 4 * q);
+#pragma unroll
+                for (int j = 0; j < F; ++j) {
+                    fma2(part[i][j], a.x, w[j].x);
+                    fma2(part[i][j], a.y, w[j].y);
+                }
             }
         }
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            acc[i] += part[i];
-            part[i] = 0.f;
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const int gn = n0 + tn;
-    if (gn < N) {
+        for (int i = 0; i < MR; ++i)
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const int gm = m0 + tg * PER + i;
-            if (gm < M) C[(size_t)gm * ldc + gn] = bias ? acc[i] + bias[gn] : acc[i];
-        }
+            for (int j = 0; j < F; ++j) acc[i][j] += run_sum(part[i][j]);
     }
+    // the chains in ascending order, through the ring's memory
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MR; ++i)
+#pragma unroll
+        for (int j = 0; j < F; ++j) ring[(chain * MT + group * MR + i) * FN + ft + j * FT] = acc[i][j];
+    __syncthreads();
+    for (int e = tid; e < MT * FN; e += THREADS) {
+        const int m = e / FN, n = n0 + e % FN;
+        if (m >= M || n >= N) continue;
+        float out = 0.f;
+#pragma unroll
+        for (int c = 0; c < CHAINS; ++c) out += ring[c * MT * FN + e];
+        C[(size_t)m * ldc + n] = bias ? out + bias[n] : out;
+    }
+}
+
+template <int MR, int F, int GROUPS, int STAGES>
+static int launch_stream(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
+                         const float* bias, int M, int N, int K, cudaStream_t stream) {
+    constexpr int BYTES = STAGES * (16 + MR * GROUPS) * (CHAINS * (RUN + 4) + 4) * 4;
+    static_assert(BYTES <= 232448, "the ring does not fit into shared memory");
+    static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attribute is per device
+    bool& configured = configured_on[pyre_current_device()];
+    auto kernel = sgemm_nt_stream_kernel<MR, F, GROUPS, STAGES>;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    return (int)pyre_launch(kernel, dim3(ceil_div(N, 16)), dim3(CHAINS * 16 / F * GROUPS), (size_t)BYTES, stream,
+                            A, lda, W, ldw, C, ldc, bias, M, N, K);
+}
+
+template <int PARTS>
+static int launch_tiles_as(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
+                           const float* bias, int M, int N, int K, cudaStream_t stream) {
+    constexpr int BYTES = (TILE_STAGES * 2 * TILE * 20 + TILE * TILE) * 4;
+    static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attribute is per device
+    bool& configured = configured_on[pyre_current_device()];
+    auto kernel = sgemm_nt_tiles_kernel<PARTS>;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int tiles_m = ceil_div(M, TILE);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((long long)tiles_m * ceil_div(N, TILE) * PARTS));
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = PARTS;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = pyre_pdl_enabled() ? attr : attr + 1;
+    cfg.numAttrs = (pyre_pdl_enabled() ? 1 : 0) + (PARTS > 1 ? 1 : 0);
+    return (int)cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, bias, M, N, K, tiles_m);
+}
+
+static int launch_tiles(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
+                        const float* bias, int M, int N, int K, cudaStream_t stream) {
+    const long long tiles = (long long)ceil_div(M, TILE) * ceil_div(N, TILE);
+    const int sms = pyre_sm_count();
+    // A CTA per chain where whole tiles would leave the SMs unevenly loaded (the busiest has ceil(tiles / SMs) of them) and
+    // a chain is long enough (four runs) to pay for the cluster's meeting
+    const long long busiest = (tiles + sms - 1) / sms;
+    if (K >= 4 * RUN * CHAINS && busiest * sms * 10 > tiles * 11)
+        return launch_tiles_as<CHAINS>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    return launch_tiles_as<1>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
 }
 
 PYRE_API int pyre_sgemm_nt(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
@@ -258,22 +452,17 @@ PYRE_API int pyre_sgemm_nt(const float* A, long long lda, const float* W, long l
     if (K < 0) return PYRE_ERR_BAD_ARG;
     // float4 loads and 16-byte copies need aligned rows in both operands
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)A & 15) && !((uintptr_t)W & 15);
-    if (vec && M <= 8) {
-        dim3 grid(ceil_div(N, 16), 1);
-        pyre_launch(sgemm_nt_stream_kernel<8>, dim3(grid), dim3(128), 0, stream, A, lda, W, ldw, C, ldc, bias, M, N, K);
-    } else if (vec && M <= 32) {
-        dim3 grid(ceil_div(N, 16), 1);
-        pyre_launch(sgemm_nt_stream_kernel<32>, dim3(grid), dim3(128), 0, stream, A, lda, W, ldw, C, ldc, bias, M, N, K);
-    } else if (vec) {
-        dim3 grid(ceil_div(N, 128), ceil_div(M, 128));
-        pyre_launch(sgemm_nt_tiles_kernel, dim3(grid), dim3(256), 0, stream, A, lda, W, ldw, C, ldc, bias, M, N, K);
-    } else if (M > 32) {
-        dim3 grid(ceil_div(N, 128), ceil_div(M, 128));
-        pyre_launch(sgemm_nt_kernel<128, 128, 8, 8, 8>, dim3(grid), dim3(256), 0, stream, A, lda, W, ldw, C, ldc, bias, M, N, K);
-    } else {
-        dim3 grid(ceil_div(N, 128), ceil_div(M, 32));
-        pyre_launch(sgemm_nt_kernel<32, 128, 16, 2, 8>, dim3(grid), dim3(256), 0, stream, A, lda, W, ldw, C, ldc, bias, M, N, K);
-    }
+    int rc = 0;
+    if (vec && M <= 4) rc = launch_stream<4, 1, 1, 4>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    else if (vec && M <= 8) rc = launch_stream<8, 1, 1, 4>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    else if (vec && M <= 16) rc = launch_stream<8, 2, 2, 3>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    else if (vec && M <= 32) rc = launch_stream<8, 2, 4, 2>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    else if (vec) rc = launch_tiles(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    else if (M > 32) rc = (int)pyre_launch(sgemm_nt_kernel<64, 128, 4, 8>, dim3(ceil_div(N, 128), ceil_div(M, 64)), dim3(256), 0, stream,
+                                           A, lda, W, ldw, C, ldc, bias, M, N, K);
+    else rc = (int)pyre_launch(sgemm_nt_kernel<32, 128, 2, 8>, dim3(ceil_div(N, 128), ceil_div(M, 32)), dim3(256), 0, stream,
+                               A, lda, W, ldw, C, ldc, bias, M, N, K);
+    if (rc) return rc;
     PYRE_LAUNCH_CHECK();
     return 0;
 }
