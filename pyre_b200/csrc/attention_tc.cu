@@ -565,60 +565,52 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
 }
 
-// The shares of a (query tile, head) put together: out = sum_i O_i 2^(m_i - M) / sum_i l_i 2^(m_i - M) over the
-// shares that saw a key (l_i > 0).  One CTA per query tile and head as in the main kernel, a warp per row, a lane per
-// four head dimensions.
+// The shares of a row put together: out = sum_i O_i 2^(m_i - M) / sum_i l_i 2^(m_i - M) over the shares that saw a key
+// (l_i > 0).  A warp per (token, head), a lane per four head dimensions: bound by reading the shares, which have
+// just been written and mostly lie in the L2 cache, so what counts is that all of them are asked for at once.  (With a CTA per
+// query tile and head, as in the main kernel, a warp walked 32 rows one after the other: 500 tokens of 28 heads in five
+// shares, 36 MB, 97 -> 8.7 us.)
 template <int HD>
 __global__ void __launch_bounds__(128)
-combine_shares_kernel(const TcParams p) {
+combine_shares_kernel(const TcParams p, int n_tokens) {
     pdl_trigger();
     pdl_wait();
-    int tile = blockIdx.y, seq = -1, tok0 = 0, n_tok = 0;
-    for (int b = 0; b < p.n_seqs; ++b) {
-        const int begin = p.cu_seqlens[b], len = p.cu_seqlens[b + 1] - begin;
-        if (len < p.min_len) continue;
-        const int nt = (len + BM - 1) / BM;
-        if (tile < nt) {
-            const int qt = nt - 1 - tile;
-            seq = b;
-            tok0 = begin + qt * BM;
-            n_tok = min(BM, len - qt * BM);
-            break;
-        }
-        tile -= nt;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, S = p.key_splits;
+    const long long item = (long long)blockIdx.x * 4 + warp;
+    if (item >= (long long)n_tokens * p.nh) return;
+    const int token = (int)(item / p.nh), head = (int)(item - (long long)token * p.nh);
+    int b = 0;
+    while (b + 1 < p.n_seqs && p.cu_seqlens[b + 1] <= token) ++b;
+    if (p.cu_seqlens[b + 1] - p.cu_seqlens[b] < p.min_len) return;      // the other attention kernel's rows
+    const size_t at = (size_t)item * S;
+    float m = -INFINITY, l = 0.f;
+    if (lane < S) {
+        m = p.part_ml[(at + lane) * 2];
+        l = p.part_ml[(at + lane) * 2 + 1];
+        if (!(l > 0.f)) { m = -INFINITY; l = 0.f; }
     }
-    if (seq < 0) return;
-    const int head = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, S = p.key_splits;
-    for (int row = warp; row < n_tok; row += 4) {
-        const size_t at = ((size_t)(tok0 + row) * p.nh + head) * S;
-        float m = -INFINITY, l = 0.f;
-        if (lane < S) {
-            m = p.part_ml[(at + lane) * 2];
-            l = p.part_ml[(at + lane) * 2 + 1];
-            if (!(l > 0.f)) { m = -INFINITY; l = 0.f; }
-        }
-        float top = m;
+    float top = m;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-        const float w = l > 0.f ? ex2(m - top) : 0.f;
-        float denom = l * w;
+    for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    const float w = l > 0.f ? ex2(m - top) : 0.f;
+    float denom = l * w;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) denom += __shfl_xor_sync(0xffffffffu, denom, o);
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int i = 0; i < S; ++i) {
-            const float wi = __shfl_sync(0xffffffffu, w, i);
-            if (wi > 0.f && lane < HD / 4) {
-                const float4 o = *reinterpret_cast<const float4*>(p.part_o + (at + i) * HD + 4 * lane);
-                acc.x = fmaf(wi, o.x, acc.x); acc.y = fmaf(wi, o.y, acc.y); acc.z = fmaf(wi, o.z, acc.z); acc.w = fmaf(wi, o.w, acc.w);
-            }
+    for (int o = 16; o > 0; o >>= 1) denom += __shfl_xor_sync(0xffffffffu, denom, o);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int i = 0; i < S; ++i) {
+        const float wi = __shfl_sync(0xffffffffu, w, i);
+        const float4 o = *reinterpret_cast<const float4*>(p.part_o + (at + i) * HD + 4 * (lane % (HD / 4)));
+        if (wi > 0.f) {      // a share that saw no key has left nothing there
+            acc.x = fmaf(wi, o.x, acc.x); acc.y = fmaf(wi, o.y, acc.y); acc.z = fmaf(wi, o.z, acc.z); acc.w = fmaf(wi, o.w, acc.w);
         }
-        if (lane < HD / 4) {
-            const float inv = denom > 0.f ? 1.0f / (denom + ex2((p.head_sinks ? p.head_sinks[head] * 1.44269504088896341f : p.sink_l2) - top)) : 0.f;
-            uint2 packed;
-            packed.x = pack_bf16(acc.x * inv, acc.y * inv);
-            packed.y = pack_bf16(acc.z * inv, acc.w * inv);
-            *reinterpret_cast<uint2*>(p.out + ((size_t)(tok0 + row) * p.nh + head) * HD + 4 * lane) = packed;
-        }
+    }
+    if (lane < HD / 4) {
+        const float inv = denom > 0.f ? 1.0f / (denom + ex2((p.head_sinks ? p.head_sinks[head] * 1.44269504088896341f : p.sink_l2) - top)) : 0.f;
+        uint2 packed;
+        packed.x = pack_bf16(acc.x * inv, acc.y * inv);
+        packed.y = pack_bf16(acc.z * inv, acc.w * inv);
+        *reinterpret_cast<uint2*>(p.out + (size_t)item * HD + 4 * lane) = packed;
     }
 }
 
@@ -652,7 +644,7 @@ bool make_map(CUtensorMap* map, const void* ptr, long long rows, long long cols,
 }
 
 template <int HD, bool KEEP>
-int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const TcParams& p, int tiles_bound, cudaStream_t stream) {
+int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const TcParams& p, int tiles_bound, int n_tokens, cudaStream_t stream) {
     using L = Smem<HD>;
     static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attributes are per device
     bool& configured = configured_on[pyre_current_device()];
@@ -664,7 +656,7 @@ int launch(const CUtensorMap& mq, const CUtensorMap& mkv, const TcParams& p, int
     cudaError_t e = pyre_launch(attention_tc_kernel<HD, KEEP>, dim3(p.nh, tiles_bound, p.key_splits), dim3(THREADS), (size_t)L::TOTAL, stream, mq, mkv, p);
     if (e != cudaSuccess) return (int)e;
     if (p.key_splits > 1) {
-        e = pyre_launch(combine_shares_kernel<HD>, dim3(p.nh, tiles_bound), dim3(128), 0, stream, p);
+        e = pyre_launch(combine_shares_kernel<HD>, dim3((unsigned)(((long long)n_tokens * p.nh + 3) / 4)), dim3(128), 0, stream, p, n_tokens);
         if (e != cudaSuccess) return (int)e;
     }
     return (int)cudaGetLastError();
@@ -706,6 +698,6 @@ PYRE_API int pyre_attention_prefill_tc(const void* q, const void* cache, void* o
     const int tiles_bound = n_long_tokens / BM + n_seqs;
     if (tiles_bound > 65535) return PYRE_ERR_BAD_ARG;   // grid.y
     if (p.keep_first > 0)
-        return hd == 128 ? launch<128, true>(mq, mkv, p, tiles_bound, stream) : launch<64, true>(mq, mkv, p, tiles_bound, stream);
-    return hd == 128 ? launch<128, false>(mq, mkv, p, tiles_bound, stream) : launch<64, false>(mq, mkv, p, tiles_bound, stream);
+        return hd == 128 ? launch<128, true>(mq, mkv, p, tiles_bound, n_tokens, stream) : launch<64, true>(mq, mkv, p, tiles_bound, n_tokens, stream);
+    return hd == 128 ? launch<128, false>(mq, mkv, p, tiles_bound, n_tokens, stream) : launch<64, false>(mq, mkv, p, tiles_bound, n_tokens, stream);
 }
