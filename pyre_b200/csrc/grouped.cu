@@ -10,7 +10,8 @@
 //
 // One CTA computes a 64 x 64 tile of a group's result (128 x 128 for bfloat16 groups of many rows).  float32: FFMA, one chain per output element over k in
 // ascending order, so a row's result does not depend on which other rows share its tile or its launch.
-// bfloat16 operands: the same tiles on the tensor cores (mma.sync m16n8k16, fp32 accumulators).
+// bfloat16 operands: on the tensor cores with fp32 accumulators, groups of few rows by mma.sync m16n8k16 (a weight stream:
+// its tiles grow with the rows in steps of 16), groups of many rows by tcgen05.mma.
 // `dtype`: type of x and w (0 = float32, 1 = bfloat16); `out_f32`: the result stays fp32, else it is rounded to dtype.
 #include "common.cuh"
 
@@ -41,19 +42,31 @@ __device__ __forceinline__ bool grouped_tile(const GroupedArgs& a, int& g, int& 
         return count > 0;
     }
     __shared__ int found[3];
-    if (threadIdx.x == 0) {
-        int tile = blockIdx.x, gg = 0;
-        found[0] = -1;
-        for (; gg < a.G; ++gg) {
-            const int lo = a.offsets[gg], n = a.offsets[gg + 1] - lo;
+    if (threadIdx.x < 32) {
+        // a lane per group, 32 groups at a time: the tiles before a group by a scan over the lanes (one thread that walked
+        // the groups waited for a load per group: some 8 us of a decode step's product at 32 groups)
+        const int lane = threadIdx.x;
+        int before = 0;
+        if (lane == 0) found[0] = -1;
+        __syncwarp();
+        for (int g0 = 0; g0 < a.G; g0 += 32) {
+            const int gg = g0 + lane;
+            const int lo = gg < a.G ? a.offsets[gg] : 0, n = gg < a.G ? a.offsets[gg + 1] - lo : 0;
             const int tiles = (n + GB_M - 1) / GB_M;
-            if (tile < tiles) {
+            int upto = tiles;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, upto, o);
+                if (lane >= o) upto += v;
+            }
+            const int tile = (int)blockIdx.x - before - (upto - tiles);       // within this lane's group
+            if (tile >= 0 && tile < tiles) {
                 found[0] = gg;
                 found[1] = lo + tile * GB_M;
                 found[2] = min(GB_M, n - tile * GB_M);
-                break;
             }
-            tile -= tiles;
+            before += __shfl_sync(0xffffffffu, upto, 31);
+            if (before > (int)blockIdx.x) break;
         }
     }
     __syncthreads();
@@ -129,10 +142,16 @@ __global__ void __launch_bounds__(256) grouped_linear_kernel(GroupedArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// bfloat16 on the tensor cores: the same 64 x 64 tile, K in steps of 32 through shared memory, four warps of
-// 32 x 32 each (2 x 4 MMAs of m16n8k16 per k-step of 16).  Needs K % 8 == 0 and 16-byte aligned rows of x and w.
+// bfloat16, groups of few rows: a 64 x 64 tile by mma.sync, bound by reading the weights (a decoded token's experts have a row
+// or two each).  K in steps of 64 through a ring of four stages filled by cp.async, so that a CTA has 24 KB of weights in
+// flight and three CTAs fit on an SM; each of the four warps owns 16 output features and as many 16-row pieces as the
+// tile has rows, so that two rows do not cost the multiplications of 64.  Measured inside a decode step of 4 tokens (16
+// places of 32 experts, 2048 x 2048 and 2048 x 1024 weights): 95 -> 28 us and 50 -> 16 us (64-row
+// tiles whatever the rows, one step ahead through registers); 64 tokens: 111 -> 70 us.
+// Needs K % 8 == 0 and 16-byte aligned rows of x and w.
 // ---------------------------------------------------------------------------
-constexpr int GT_K = 32, GT_LD = GT_K + 8;   // padded rows: 80 bytes, conflict-free for ldmatrix
+constexpr int GT_K = 64, GT_LD = GT_K + 8, GT_STAGES = 4;   // padded rows: 144 bytes, conflict-free for ldmatrix
+constexpr int GT_STAGE = (GB_M + GB_N) * GT_LD, GT_SMEM = GT_STAGES * GT_STAGE * 2;
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* p) {
     const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
@@ -145,15 +164,59 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(128) grouped_linear_mma_kernel(GroupedArgs a) {
-    __shared__ __align__(16) __nv_bfloat16 xs[2][GB_M][GT_LD];
-    __shared__ __align__(16) __nv_bfloat16 ws[2][GB_N][GT_LD];
+// a 16-byte copy into shared memory, or 16 bytes of zeros
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool live) {
+    const int bytes = live ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// Two neighbouring results of a row: one store where the row allows it.
+__device__ __forceinline__ void store_pair(const GroupedArgs& a, size_t at, int n, float v0, float v1) {
+    if (a.out_f32) {
+        float* o = (float*)a.out + at;
+        if (n + 1 < a.N && ((uintptr_t)o & 7) == 0) *reinterpret_cast<float2*>(o) = make_float2(v0, v1);
+        else {
+            if (n < a.N) o[0] = v0;
+            if (n + 1 < a.N) o[1] = v1;
+        }
+    } else {
+        __nv_bfloat16* o = (__nv_bfloat16*)a.out + at;
+        if (n + 1 < a.N && ((uintptr_t)o & 3) == 0) *reinterpret_cast<__nv_bfloat162*>(o) = __floats2bfloat162_rn(v0, v1);
+        else {
+            if (n < a.N) o[0] = __float2bfloat16_rn(v0);
+            if (n + 1 < a.N) o[1] = __float2bfloat16_rn(v1);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs a) {
+    extern __shared__ __align__(16) __nv_bfloat16 g_ring[];      // [stages][64 rows of x, 64 rows of w][GT_LD]
     __shared__ int src_row[GB_M], dst_row[GB_M];
     pdl_trigger();
-    pdl_wait();
-    int g, first, count;
-    if (!grouped_tile(a, g, first, count)) return;
     const int n0 = blockIdx.y * GB_N;
+    const int n_steps = (a.K + GT_K - 1) / GT_K;
+    const int lr = threadIdx.x >> 3, lk = (threadIdx.x & 7) * 8;        // copies: rows lr, lr + 16, ..., eight threads to a row
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(g_ring);
+    auto load_w = [&](const __nv_bfloat16* w, int s) {
+        if (s >= n_steps) return;
+        const uint32_t to = ring + ((s % GT_STAGES) * GT_STAGE + GB_M * GT_LD) * 2;
+        const int k = s * GT_K + lk;
+        const bool in_k = k < a.K;
+#pragma unroll
+        for (int r = lr; r < GB_N; r += 16)      // features past the end are not stored: whatever their sums are
+            if (n0 + r < a.N) copy16(to + (r * GT_LD + lk) * 2, in_k ? w + (size_t)(n0 + r) * a.K + k : w, in_k);
+    };
+    int g = 0, first = 0, count = 0;
+    if (!a.offsets) {      // the weights are known before the kernels before this one finish
+        g = blockIdx.z;
+        const __nv_bfloat16* w = (const __nv_bfloat16*)a.w + (size_t)g * a.w_group_stride;
+        for (int s = 0; s < GT_STAGES - 1; ++s) load_w(w, s);
+    }
+    pdl_wait();
+    if (!grouped_tile(a, g, first, count)) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        return;
+    }
     if (threadIdx.x < GB_M) {
         const int p = first + threadIdx.x;
         const bool live = (int)threadIdx.x < count;
@@ -164,85 +227,126 @@ __global__ void __launch_bounds__(128) grouped_linear_mma_kernel(GroupedArgs a) 
     const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + (size_t)g * a.x_group_stride;
     const __nv_bfloat16* w = (const __nv_bfloat16*)a.w + (size_t)g * a.w_group_stride;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-    float acc[2][4][4];
+    const int m_tiles = (count + 15) / 16;
+    auto load_x = [&](int s) {
+        if (s >= n_steps) return;
+        const uint32_t to = ring + (s % GT_STAGES) * GT_STAGE * 2;
+        const int k = s * GT_K + lk;
+        const bool in_k = k < a.K;
+        for (int r = lr; r < count; r += 16)
+            copy16(to + (r * GT_LD + lk) * 2, in_k ? x + (size_t)src_row[r] * a.x_row_stride + k : x, in_k);
+    };
+    for (int s = 0; s < GT_STAGES - 1; ++s) {
+        if (a.offsets) load_w(w, s);
+        load_x(s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float acc[4][2][4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-
-    // a stage: 64 rows x 32 k of each operand = 256 vectors of 8 per operand, two per thread and operand
-    auto load_stage = [&](int st, int k0) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int idx = threadIdx.x + u * 128;
-            const int r = idx >> 2, k = (idx & 3) * 8;
-            const int sr = src_row[r];
-            uint4 xv = make_uint4(0, 0, 0, 0), wv = make_uint4(0, 0, 0, 0);
-            if (sr >= 0 && k0 + k < a.K) xv = *reinterpret_cast<const uint4*>(x + (size_t)sr * a.x_row_stride + k0 + k);
-            if (n0 + r < a.N && k0 + k < a.K) wv = *reinterpret_cast<const uint4*>(w + (size_t)(n0 + r) * a.K + k0 + k);
-            *reinterpret_cast<uint4*>(&xs[st][r][k]) = xv;
-            *reinterpret_cast<uint4*>(&ws[st][r][k]) = wv;
-        }
-    };
-    const int n_steps = (a.K + GT_K - 1) / GT_K;
-    load_stage(0, 0);
-    __syncthreads();
     for (int s = 0; s < n_steps; ++s) {
-        const int st = s & 1;
-        if (s + 1 < n_steps) load_stage(st ^ 1, (s + 1) * GT_K);
+        asm volatile("cp.async.wait_group %0;" ::"n"(GT_STAGES - 2) : "memory");
+        __syncthreads();      // this step has landed for every thread; the stage filled below was read a step ago
+        load_w(w, s + GT_STAGES - 1);
+        load_x(s + GT_STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const __nv_bfloat16* xs = g_ring + (s % GT_STAGES) * GT_STAGE;
+        const __nv_bfloat16* ws = xs + (GB_M + warp * 16) * GT_LD;
 #pragma unroll
         for (int kk = 0; kk < GT_K; kk += 16) {
-            uint32_t af[2][4], bf[2][4];
+            uint32_t bf[4];      // 16 n-rows: two 8-wide n tiles, both k halves
+            ldmatrix_x4(bf, ws + ((lane & 7) + ((lane >> 4) << 3)) * GT_LD + kk + ((lane >> 3) & 1) * 8);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-                ldmatrix_x4(af[i], &xs[st][wm + i * 16 + (lane & 15)][kk + (lane >> 4) * 8]);
-#pragma unroll
-            for (int j = 0; j < 2; ++j)   // 16 n-rows per ldmatrix: two 8-wide n tiles, both k halves
-                ldmatrix_x4(bf[j], &ws[st][wn + j * 16 + (lane & 7) + ((lane >> 4) << 3)][kk + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
+            for (int i = 0; i < 4; ++i) {
+                if (i < m_tiles) {
+                    uint32_t af[4];
+                    ldmatrix_x4(af, xs + (i * 16 + (lane & 15)) * GT_LD + kk + (lane >> 4) * 8);
+                    mma_bf16(acc[i][0], af, bf[0], bf[1]);
+                    mma_bf16(acc[i][1], af, bf[2], bf[3]);
+                }
+            }
         }
-        __syncthreads();
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            const int dr = dst_row[wm + i * 16 + (lane >> 2) + half * 8];
+            const int dr = dst_row[i * 16 + (lane >> 2) + half * 8];
             if (dr < 0) continue;
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int n = n0 + wn + j * 8 + (lane & 3) * 2 + e;
-                    if (n >= a.N) continue;
-                    const size_t at = (size_t)dr * a.out_row_stride + (size_t)g * a.out_group_stride + n;
-                    const float v = acc[i][j][half * 2 + e];
-                    if (a.out_f32) ((float*)a.out)[at] = v;
-                    else ((__nv_bfloat16*)a.out)[at] = __float2bfloat16_rn(v);
-                }
+            for (int j = 0; j < 2; ++j) {
+                const int n = n0 + warp * 16 + j * 8 + (lane & 3) * 2;
+                store_pair(a, (size_t)dr * a.out_row_stride + (size_t)g * a.out_group_stride + n, n, acc[i][j][half * 2], acc[i][j][half * 2 + 1]);
+            }
         }
 }
 
 // ---------------------------------------------------------------------------
-// The same product for groups of many rows: 128 x 128 tiles, eight warps of 64 x 32 each (16 MMAs per four A and two B
-// fragment loads), K in steps of 32 through two buffers filled by cp.async while the other is multiplied.
+// The same product for groups of many rows, on the 5th-generation tensor cores: 128 rows x 128 features per CTA, fp32
+// accumulators in tensor memory, K in steps of 64 through a ring of three 32 KB stages; two CTAs fit on an SM, so that one
+// drains its result while the other multiplies.
+//   warps 0..3 : bring the rows of x (gathered) and of w into the ring by cp.async, 128-byte rows with the 128-byte swizzle
+//                (16-byte piece c of row r lies at c ^ (r & 7)), and tell the MMA thread when a stage has landed; then the
+//                epilogue, a row per thread.  (TMA would need a tensor map per launch and cannot gather rows cheaper.)
+//   warp 4     : allocates tensor memory; one thread issues tcgen05.mma (M = 128, N = 128, four of K = 16 per stage).
+// Bound by what an SM can load: 32 KB per 128 x 128 x 64 products.  Measured: 2,240 tokens, top 4 of
+// 32 experts, 2048 x 2048: 336 -> 126 us (559 TFLOP/s), 2048 x 1024: 195 -> 72 us (mma.sync before); handing a stage over two
+// copies later instead of one costs 155 us, six stages and one CTA per SM 208 us.  2,240 tokens x 16 heads of 256 x 128: 29 -> 14 us.
+// Every wait on an mbarrier is bounded; if one runs out, the error flag is raised, nothing is stored, and the tensor
+// memory is freed.
 // ---------------------------------------------------------------------------
-constexpr int GL_M = 128, GL_N = 128;
+constexpr int GL_M = 128, GL_N = 128, GL_K = 64, GL_STAGES = 3, GL_THREADS = 160;
+constexpr int GL_AHEAD = 1;      // a stage is handed over once the next one's copies are on their way
+constexpr int GL_STAGE = (GL_M + GL_N) * GL_K * 2;                 // bytes
+constexpr int GL_BARS = GL_STAGES * GL_STAGE;                      // full[], empty[], accumulator full
+constexpr int GL_SMEM = GL_BARS + (2 * GL_STAGES + 1) * 8 + 1024;  // and what brings the ring to a 1024-byte boundary
+constexpr int GL_ERR_TIMEOUT = 2;
 
-__global__ void __launch_bounds__(256) grouped_linear_mma_large_kernel(GroupedArgs a) {
-    __shared__ __align__(16) __nv_bfloat16 xs[2][GL_M][GT_LD];
-    __shared__ __align__(16) __nv_bfloat16 ws[2][GL_N][GT_LD];
+__device__ __forceinline__ bool gl_try_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool gl_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err_flag) {
+    if (gl_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (uint32_t it = 1;; ++it) {
+        if (gl_try_wait(bar, parity)) return true;
+        if ((it & 63) == 0) {
+            if (*abort_flag) return false;
+            if (clock64() - t0 > PYRE_WAIT_CYCLES) break;
+        }
+    }
+    *abort_flag = 1;
+    if (err_flag) atomicExch(err_flag, GL_ERR_TIMEOUT);
+    return false;
+}
+// K-major operand of 128-byte rows with the 128-byte swizzle: stride byte offset 1024 (eight rows), version 1, layout type 2
+__device__ __forceinline__ uint64_t gl_desc(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+__global__ void __launch_bounds__(GL_THREADS, 2) grouped_linear_tc_kernel(GroupedArgs a, int* err_flag) {
+    extern __shared__ uint8_t gl_raw[];
     __shared__ int src_row[GL_M], dst_row[GL_M];
-    pdl_trigger();
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_word;
+    const uint32_t base = ((uint32_t)__cvta_generic_to_shared(gl_raw) + 1023u) & ~1023u;
+    const uint32_t bar_full = base + GL_BARS, bar_empty = bar_full + 8 * GL_STAGES, bar_acc = bar_empty + 8 * GL_STAGES;
+    volatile int* abort_flag = &abort_word;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     pdl_wait();
     int g, first, count;
-    if (!grouped_tile<GL_M>(a, g, first, count)) return;
+    if (!grouped_tile<GL_M>(a, g, first, count)) return;      // the whole CTA, before anything is set up
     const int n0 = blockIdx.y * GL_N;
     if (threadIdx.x < GL_M) {
         const int p = first + threadIdx.x;
@@ -250,97 +354,157 @@ __global__ void __launch_bounds__(256) grouped_linear_mma_large_kernel(GroupedAr
         src_row[threadIdx.x] = live ? (a.src ? a.src[p] : p) : -1;
         dst_row[threadIdx.x] = live ? (a.dst ? a.dst[p] : p) : -1;
     }
-    __syncthreads();
-    const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + (size_t)g * a.x_group_stride;
-    const __nv_bfloat16* w = (const __nv_bfloat16*)a.w + (size_t)g * a.w_group_stride;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wm = (warp >> 2) * 64, wn = (warp & 3) * 32;
-    float acc[4][4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-
-    // a stage: 128 rows x 32 k of each operand = 512 pieces of 16 bytes per operand, two per thread and operand
-    auto load_stage = [&](int st, int k0) {
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int idx = threadIdx.x + u * 256;
-            const int r = idx >> 2, k = (idx & 3) * 8;
-            const int sr = src_row[r];
-            __nv_bfloat16* xd = &xs[st][r][k];
-            __nv_bfloat16* wd = &ws[st][r][k];
-            if (sr >= 0 && k0 + k < a.K) {
-                const uint32_t d = (uint32_t)__cvta_generic_to_shared(xd);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(x + (size_t)sr * a.x_row_stride + k0 + k));
-            } else {
-                *reinterpret_cast<uint4*>(xd) = make_uint4(0, 0, 0, 0);
-            }
-            if (n0 + r < a.N && k0 + k < a.K) {
-                const uint32_t d = (uint32_t)__cvta_generic_to_shared(wd);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(w + (size_t)(n0 + r) * a.K + k0 + k));
-            } else {
-                *reinterpret_cast<uint4*>(wd) = make_uint4(0, 0, 0, 0);
-            }
+    if (threadIdx.x == 0) {
+        abort_word = 0;
+        for (int s = 0; s < GL_STAGES; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_full + 8 * s), "r"(128) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_empty + 8 * s), "r"(1) : "memory");
         }
-        asm volatile("cp.async.commit_group;" ::);
-    };
-    const int n_steps = (a.K + GT_K - 1) / GT_K;
-    load_stage(0, 0);
-    for (int s = 0; s < n_steps; ++s) {
-        const int st = s & 1;
-        if (s + 1 < n_steps) {
-            load_stage(st ^ 1, (s + 1) * GT_K);
-            asm volatile("cp.async.wait_group 1;" ::);
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GT_K; kk += 16) {
-            uint32_t af[4][4], bf[2][4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                ldmatrix_x4(af[i], &xs[st][wm + i * 16 + (lane & 15)][kk + (lane >> 4) * 8]);
-#pragma unroll
-            for (int j = 0; j < 2; ++j)
-                ldmatrix_x4(bf[j], &ws[st][wn + j * 16 + (lane & 7) + ((lane >> 4) << 3)][kk + ((lane >> 3) & 1) * 8]);
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) mma_bf16(acc[i][j], af[i], bf[j >> 1][(j & 1) * 2], bf[j >> 1][(j & 1) * 2 + 1]);
-        }
-        __syncthreads();      // the buffer is filled again two steps on
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar_acc), "r"(1) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 4) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(&tmem_slot)), "r"(GL_N) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *(volatile uint32_t*)&tmem_slot;
+    pdl_trigger();      // only now: a later kernel's CTA must not find tensor memory that this one has yet to take
+    const int n_steps = (a.K + GL_K - 1) / GL_K;
+
+    if (warp < 4) {
+        const __nv_bfloat16* x = (const __nv_bfloat16*)a.x + (size_t)g * a.x_group_stride;
+        const __nv_bfloat16* w = (const __nv_bfloat16*)a.w + (size_t)g * a.w_group_stride;
+        const int lr = threadIdx.x >> 3, piece = threadIdx.x & 7;       // rows lr, lr + 16, ..., eight threads to a row
+        // where this thread's pieces come from: worked out once, the issue of copies is what bounds the loaders
+        constexpr int PER = GL_M / 16;
+        const __nv_bfloat16* xp[PER];
+        const __nv_bfloat16* wp[PER];
+        uint32_t x_live = 0, w_live = 0;      // rows and features past the end are not stored: whatever their sums are
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < PER; ++i) {
+            const int r = lr + 16 * i;
+            x_live |= (uint32_t)(r < count) << i;
+            w_live |= (uint32_t)(n0 + r < a.N) << i;
+            xp[i] = x + (size_t)max(src_row[r], 0) * a.x_row_stride + piece * 8;
+            wp[i] = w + (size_t)min(n0 + r, a.N - 1) * a.K + piece * 8;
+        }
+        const uint32_t at0 = lr * 128 + ((piece ^ (lr & 7)) << 4);      // rows 16 apart lie 2048 bytes apart, swizzled alike
+        bool alive = true;
+        for (int s = 0; s < n_steps + GL_AHEAD && alive; ++s) {
+            if (s < n_steps) {
+                const int st = s % GL_STAGES;
+                if (s >= GL_STAGES) alive = gl_wait(bar_empty + 8 * st, (s / GL_STAGES - 1) & 1, abort_flag, err_flag);
+                if (!alive) break;
+                const uint32_t xs = base + st * GL_STAGE, ws = xs + GL_M * GL_K * 2;
+                const int k = s * GL_K;
+                const bool in_k = k + piece * 8 < a.K;
+                const int from = in_k ? k : 0;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int dr = dst_row[wm + i * 16 + (lane >> 2) + half * 8];
-            if (dr < 0) continue;
+                for (int i = 0; i < PER; ++i) {
+                    if (x_live >> i & 1) copy16(xs + at0 + i * 2048, xp[i] + from, in_k);
+                    if (w_live >> i & 1) copy16(ws + at0 + i * 2048, wp[i] + from, in_k);
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (s >= GL_AHEAD) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(GL_AHEAD) : "memory");
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // what this thread brought, for the tensor core
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar_full + 8 * ((s - GL_AHEAD) % GL_STAGES)) : "memory");
+            }
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        // ---- epilogue: the thread's row
+        alive = alive && gl_wait(bar_acc, 0, abort_flag, err_flag) && !*abort_flag;
+        alive = __all_sync(0xffffffffu, alive);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int dr = dst_row[threadIdx.x];
+        const size_t at = (size_t)(dr < 0 ? 0 : dr) * a.out_row_stride + (size_t)g * a.out_group_stride + n0;
+        const int esize = a.out_f32 ? 4 : 2;
+        const bool wide = (((uintptr_t)a.out + at * esize) & 31) == 0;
+        if (alive) {
+#pragma unroll 1
+            for (int c = 0; c < GL_N; c += 16) {
+                uint32_t r[16];
+                __syncwarp();
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                    : "r"(tmem + c + ((uint32_t)(warp * 32) << 16)) : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (dr < 0 || n0 + c >= a.N) continue;
+                if (wide && n0 + c + 16 <= a.N) {      // 32 bytes per request: whole sectors
+                    if (a.out_f32) {
+                        float* o = (float*)a.out + at + c;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int n = n0 + wn + j * 8 + (lane & 3) * 2;
-                const size_t at = (size_t)dr * a.out_row_stride + (size_t)g * a.out_group_stride + n;
-                const float v0 = acc[i][j][half * 2], v1 = acc[i][j][half * 2 + 1];
-                if (a.out_f32) {
-                    if (n < a.N) ((float*)a.out)[at] = v0;
-                    if (n + 1 < a.N) ((float*)a.out)[at + 1] = v1;
+                        for (int h = 0; h < 16; h += 8)
+                            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + h), "r"(r[h]), "r"(r[h + 1]), "r"(r[h + 2]),
+                                         "r"(r[h + 3]), "r"(r[h + 4]), "r"(r[h + 5]), "r"(r[h + 6]), "r"(r[h + 7]) : "memory");
+                    } else {
+                        uint32_t p[8];
+#pragma unroll
+                        for (int h = 0; h < 8; ++h) {
+                            const __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(r[2 * h]), __uint_as_float(r[2 * h + 1]));
+                            p[h] = *reinterpret_cast<const uint32_t*>(&v);
+                        }
+                        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"((__nv_bfloat16*)a.out + at + c), "r"(p[0]), "r"(p[1]),
+                                     "r"(p[2]), "r"(p[3]), "r"(p[4]), "r"(p[5]), "r"(p[6]), "r"(p[7]) : "memory");
+                    }
                 } else {
-                    if (n < a.N) ((__nv_bfloat16*)a.out)[at] = __float2bfloat16_rn(v0);
-                    if (n + 1 < a.N) ((__nv_bfloat16*)a.out)[at + 1] = __float2bfloat16_rn(v1);
+#pragma unroll
+                    for (int h = 0; h < 16; ++h) {
+                        if (n0 + c + h >= a.N) continue;
+                        if (a.out_f32) ((float*)a.out)[at + c + h] = __uint_as_float(r[h]);
+                        else ((__nv_bfloat16*)a.out)[at + c + h] = __float2bfloat16_rn(__uint_as_float(r[h]));
+                    }
                 }
             }
         }
+    } else if (lane == 0) {
+        // D fp32 (bit 4), A and B bf16 (bits 7, 10), both K-major, N >> 3 at bit 17, M >> 4 at bit 24
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GL_N >> 3) << 17) | ((uint32_t)(GL_M >> 4) << 24);
+        for (int s = 0; s < n_steps; ++s) {
+            const int st = s % GL_STAGES;
+            if (!gl_wait(bar_full + 8 * st, (s / GL_STAGES) & 1, abort_flag, err_flag)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint64_t da = gl_desc(base + st * GL_STAGE), db = gl_desc(base + st * GL_STAGE + GL_M * GL_K * 2);
+#pragma unroll
+            for (int k = 0; k < GL_K / 16; ++k)      // 16 bf16 = 32 bytes = 2 descriptor units along K
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\t"
+                    "setp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                    ::"r"(tmem), "l"(da + 2 * k), "l"(db + 2 * k), "r"(idesc), "r"((s > 0 || k > 0) ? 1u : 0u) : "memory");
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_empty + 8 * st) : "memory");
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_acc) : "memory");      // also when it gave up
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 4) {
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(GL_N) : "memory");
+    }
+}
+
+// A kernel with more dynamic shared memory than the default allows (the attribute is per device).
+template <typename K>
+static int allow_smem(K kernel, int bytes, bool (&done)[PYRE_MAX_DEVICES]) {
+    bool& configured = done[pyre_current_device()];
+    if (configured) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) configured = true;
+    return (int)e;
 }
 
 // places: an upper bound of the sorted places (the host does not know the groups' sizes); with offsets == null it is unused
 PYRE_API int pyre_grouped_linear(const void* x, long long x_row_stride, long long x_group_stride, const void* w,
                                  long long w_group_stride, void* out, long long out_row_stride, long long out_group_stride,
                                  const int* offsets, const int* src, const int* dst, int M, int N, int K, int G, int places,
-                                 int out_f32, int dtype, int use_mma, cudaStream_t stream) {
+                                 int out_f32, int dtype, int use_mma, int* err_flag, cudaStream_t stream) {
     if (N <= 0 || K <= 0 || G <= 0) return PYRE_ERR_BAD_ARG;
     GroupedArgs a{x, x_row_stride, x_group_stride, w, w_group_stride, out, out_row_stride, out_group_stride,
                   offsets, src, dst, M, N, K, G, out_f32};
@@ -359,9 +523,13 @@ PYRE_API int pyre_grouped_linear(const void* x, long long x_row_stride, long lon
         const long long rows_per_group = offsets ? (long long)places / G : M;
         if (rows_per_group >= 96) {
             const dim3 big = offsets ? dim3(ceil_div(places, GL_M) + G, ceil_div(N, GL_N), 1) : dim3(ceil_div(M, GL_M), ceil_div(N, GL_N), G);
-            pyre_launch(grouped_linear_mma_large_kernel, big, dim3(256), 0, stream, a);
+            static bool done[PYRE_MAX_DEVICES] = {};
+            if (const int rc = allow_smem(grouped_linear_tc_kernel, GL_SMEM, done)) return rc;
+            pyre_launch(grouped_linear_tc_kernel, big, dim3(GL_THREADS), (size_t)GL_SMEM, stream, a, err_flag);
         } else {
-            pyre_launch(grouped_linear_mma_kernel, grid, dim3(128), 0, stream, a);
+            static bool done[PYRE_MAX_DEVICES] = {};
+            if (const int rc = allow_smem(grouped_linear_mma_kernel, GT_SMEM, done)) return rc;
+            pyre_launch(grouped_linear_mma_kernel, grid, dim3(128), (size_t)GT_SMEM, stream, a);
         }
     } else if (dtype == PYRE_BF16) pyre_launch(grouped_linear_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, a);
     else if (dtype == PYRE_F32) pyre_launch(grouped_linear_kernel<float>, grid, dim3(256), 0, stream, a);

@@ -71,7 +71,7 @@ SIGNATURES: dict[str, tuple[str, list]] = {
     "pyre_latent_rotate_q": ("latent_attention", [P, P, P, P, I, I, I, I, I, I, I, I, I, P]),
     "pyre_latent_attention_exact": ("latent_attention", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, F, P, P, LL, I, LL, P, P]),
     "pyre_latent_attention_mma": ("latent_attention", [P, P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, P, P, LL, I, I, LL, P, P]),
-    "pyre_grouped_linear": ("grouped", [P, LL, LL, P, LL, P, LL, LL, P, P, P, I, I, I, I, I, I, I, I, P]),
+    "pyre_grouped_linear": ("grouped", [P, LL, LL, P, LL, P, LL, LL, P, P, P, I, I, I, I, I, I, I, I, P, P]),
     "pyre_route": ("grouped", [P, P, P, P, P, P, I, I, I, I, F, I, I, F, I, I, I, P]),
     "pyre_scale_to_places": ("grouped", [P, P, P, P, I, I, I, I, P]),
     "pyre_group_pairs": ("grouped", [P, I, I, I, P, P, P, P]),

@@ -1834,7 +1834,8 @@ def headwise_linear(x: torch.Tensor, w: torch.Tensor, out: "torch.Tensor | None"
         if tuple(out.shape[:2]) != (T, H) or out.shape[2] < N:
             raise ValueError("out does not match the heads")
     lib.call("pyre_grouped_linear", x.data_ptr(), row_stride, head_stride, w.data_ptr(), N * K, out.data_ptr(), H * out.shape[2], out.shape[2],
-             None, None, None, T, N, K, H, 0, 0, _dt(x.dtype), _grouped_mma_ok(x, w, row_stride, head_stride, K), _stream())
+             None, None, None, T, N, K, H, 0, 0, _dt(x.dtype), _grouped_mma_ok(x, w, row_stride, head_stride, K),
+             device_error_flag(x.device).data_ptr(), _stream())
     return out
 
 
@@ -1856,7 +1857,8 @@ def expert_linear(x: torch.Tensor, w: torch.Tensor, offsets: torch.Tensor, src: 
         raise ValueError("the result is in the activation dtype or float32")
     out = torch.empty((n_places, N), dtype=out_dtype, device=x.device)
     lib.call("pyre_grouped_linear", x.data_ptr(), K, 0, w.data_ptr(), N * K, out.data_ptr(), N, 0, offsets.data_ptr(), _ptr(src),
-             None, 0, N, K, E, int(n_places), int(out_dtype == torch.float32), _dt(x.dtype), _grouped_mma_ok(x, w, K, 0, K), _stream())
+             None, 0, N, K, E, int(n_places), int(out_dtype == torch.float32), _dt(x.dtype), _grouped_mma_ok(x, w, K, 0, K),
+             device_error_flag(x.device).data_ptr(), _stream())
     return out
 
 
