@@ -14,6 +14,7 @@ pyre/model.py:84-87,133-135,172).  See ``linear``.
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -689,11 +690,10 @@ def attention_prefill_tc(q: torch.Tensor, cache_layer: torch.Tensor, block_table
     return out
 
 
-def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_table: torch.Tensor, n_heads: int,
-                         n_kv_heads: int, head_dim: int, scale: float, window: "int | None",
-                         sink: "float | None" = None, keep_first: int = 0) -> torch.Tensor:
-    """Attention of a whole step in bfloat16: entries with many tokens go to the
-    prompt-portion kernel, the others (decoded tokens, short portions) to the split-KV kernel."""
+def _attention_plan(ctx, use_tc: bool, min_len: int, n_heads: int, n_kv_heads: int, head_dim: int,
+                    window: "int | None", keep_first: int) -> tuple:
+    """How a step's attention is cut: (tokens of the long entries, their key splits, short entries, splits, the length
+    all entries share or 0, row groups of the short entries).  From host-side facts of the step and the mixer's sizes alone."""
     lens = ctx.cu_seqlens_host[1:] - ctx.cu_seqlens_host[:-1]
     page_size = cache_layer.shape[3]
     use_tc = USE_TC_ATTENTION and head_dim in PREFILL_HEAD_DIMS and page_size & (page_size - 1) == 0 and page_size >= 4
@@ -701,7 +701,8 @@ def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_
     long_mask = lens >= min_len if head_dim in PREFILL_HEAD_DIMS else lens < 0
     n_long = int(lens[long_mask].sum())
     n_short_seqs = int((~long_mask).sum())
-    out = torch.empty_like(q)
+    key_splits = splits = 1
+    uniform = groups = 0
     if n_long and use_tc:
         long_lens, long_starts = lens[long_mask], ctx.start_pos_host[long_mask]
         q_tiles = -(-long_lens // 128)
@@ -711,19 +712,38 @@ def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_
         if window:
             keys = keys.clip(max=window + keep_first + 192.0)
         mean_tiles = float((keys / 64.0 * q_tiles).sum() / q_tiles.sum())
-        key_splits = prefill_key_splits(int(q_tiles.sum()) * n_heads, mean_tiles, q.shape[0], n_heads, head_dim)
+        key_splits = prefill_key_splits(int(q_tiles.sum()) * n_heads, mean_tiles, ctx.num_tokens, n_heads, head_dim)
+    if n_short_seqs:
+        short_ctx = int((ctx.start_pos_host + lens)[~long_mask].max())
+        tpg = max(1, 16 // min(n_heads // n_kv_heads, 16))
+        groups = int((-(-lens[~long_mask] // tpg)).sum())
+        splits = attention_splits(ctx.num_tokens - n_long, n_short_seqs, n_heads, n_kv_heads, short_ctx, window and window + keep_first, groups)
+        uniform = int(lens[0]) if not n_long and bool((lens == lens[0]).all()) else 0
+    return n_long, key_splits, n_short_seqs, splits, uniform, groups
+
+
+def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_table: torch.Tensor, n_heads: int,
+                         n_kv_heads: int, head_dim: int, scale: float, window: "int | None",
+                         sink: "float | None" = None, keep_first: int = 0) -> torch.Tensor:
+    """Attention of a whole step in bfloat16: entries with many tokens go to the
+    prompt-portion kernel, the others (decoded tokens, short portions) to the split-KV kernel."""
+    page_size = cache_layer.shape[3]
+    use_tc = USE_TC_ATTENTION and head_dim in PREFILL_HEAD_DIMS and page_size & (page_size - 1) == 0 and page_size >= 4
+    min_len = TC_ATTENTION_MIN_LEN if use_tc else PREFILL_MIN_LEN
+    # the layers of a step share their plan (some 80 us of host work)
+    key = ("attention_plan", use_tc, min_len, n_heads, n_kv_heads, head_dim, window, keep_first)
+    plan = ctx.scratch.get(key)
+    if plan is None:
+        plan = ctx.scratch[key] = _attention_plan(ctx, use_tc, min_len, n_heads, n_kv_heads, head_dim, window, keep_first)
+    n_long, key_splits, n_short_seqs, splits, uniform, groups = plan
+    out = torch.empty_like(q)
+    if n_long and use_tc:
         attention_prefill_tc(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_long, n_heads,
                              n_kv_heads, head_dim, scale, window, out, min_len, key_splits, sink=sink, keep_first=keep_first)
     elif n_long:
         attention_prefill(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_long, n_heads,
                           n_kv_heads, head_dim, scale, window, out, sink=sink, keep_first=keep_first)
     if n_short_seqs:
-        n_short = ctx.num_tokens - n_long
-        short_ctx = int((ctx.start_pos_host + lens)[~long_mask].max())
-        tpg = max(1, 16 // min(n_heads // n_kv_heads, 16))
-        groups = int((-(-lens[~long_mask] // tpg)).sum())
-        splits = attention_splits(n_short, n_short_seqs, n_heads, n_kv_heads, short_ctx, window and window + keep_first, groups)
-        uniform = int(lens[0]) if not n_long and bool((lens == lens[0]).all()) else 0
         paged_attention_mma(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_heads,
                             n_kv_heads, head_dim, scale, window, splits, out=out,
                             max_len=min_len - 1 if n_long else 0, uniform_len=uniform, sink=sink, keep_first=keep_first)
@@ -807,7 +827,11 @@ def tc_gemm_plan(M: int, N: int, K: int) -> tuple[bool, int, int]:
     CTA lands on every SM, each split keeping at least four 64-wide K blocks.  Beyond
     that the tokens take the rows and 128 to 256 output features form a tile, whichever
     width fills the rounds of the persistent CTAs best."""
-    _SM_COUNT = sm_count()
+    return _tc_gemm_plan(M, N, K, sm_count(), CTA_PAIRS)
+
+
+@functools.lru_cache(maxsize=4096)      # a step asks for the same few plans in every layer; working one out takes some 20 us
+def _tc_gemm_plan(M: int, N: int, K: int, _SM_COUNT: int, pair: bool) -> tuple[bool, int, int]:
     kb = -(-K // 64)
     if M <= 128 or N % 8:
         bn = 16 if M <= 16 else 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
@@ -831,7 +855,6 @@ def tc_gemm_plan(M: int, N: int, K: int) -> tuple[bool, int, int]:
     # 224 wide with K in two takes 63 us, 112 tiles of 128 take 88 us).
     # With CTA pairs (two CTAs of a cluster on a 256-row tile, each loading half of the tile's weight rows) an SM
     # loads 128 (128 + bn / 2) bytes per K block, its ring is deeper, and the workers are the 74 pairs.
-    pair = CTA_PAIRS
     workers = _SM_COUNT // 2 if pair else _SM_COUNT
     rows = -(-M // (256 if pair else 128))
     latency = 1.7 - 0.035 * min(-(-M // 128), 16)
