@@ -558,9 +558,10 @@ def paged_attention_mma(q: torch.Tensor, cache_layer: torch.Tensor, block_table:
                         n_kv_heads: int, head_dim: int, scale: float, window: "int | None" = None,
                         n_splits: int = 1, out: "torch.Tensor | None" = None,
                         scratch: "torch.Tensor | None" = None, max_len: int = 0, uniform_len: int = 0,
-                        sink: "float | None" = None, keep_first: int = 0) -> torch.Tensor:
+                        sink: "float | None" = None, keep_first: int = 0, n_groups: int = 0) -> torch.Tensor:
     """bfloat16 attention on the tensor cores over the block table (decode tokens and
-    prompt portions alike); ``n_splits`` > 1 splits each sequence's keys over CTAs and needs
+    prompt portions alike); ``n_groups``: how many row groups the entries taken have in all, where the caller has counted
+    them (0: the kernel's launch takes a bound); ``n_splits`` > 1 splits each sequence's keys over CTAs and needs
     ``T * nh * n_splits * (hd + 2)`` floats of scratch (allocated here if not given)."""
     _check(q, "q", torch.bfloat16, 2)
     _check(cache_layer, "cache_layer", torch.bfloat16, 5)
@@ -591,7 +592,7 @@ def paged_attention_mma(q: torch.Tensor, cache_layer: torch.Tensor, block_table:
     lib.call("pyre_paged_attention_mma", q.data_ptr(), cache_layer.data_ptr(), out.data_ptr(), _ptr(scratch),
              block_table.data_ptr(), block_table.stride(0), cu_seqlens.data_ptr(), positions.data_ptr(), T, n_seqs,
              n_heads, n_kv_heads, head_dim, page_size, int(window or 0), int(keep_first), float(scale), _sink_args(sink, n_heads)[0], _sink_args(sink, n_heads)[1], n_splits, int(max_len),
-             cache_layer.shape[0], int(uniform_len), device_error_flag(q.device).data_ptr(), _stream())
+             cache_layer.shape[0], int(uniform_len), int(n_groups), device_error_flag(q.device).data_ptr(), _stream())
     return out
 
 
@@ -746,7 +747,7 @@ def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_
     if n_short_seqs:
         paged_attention_mma(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_heads,
                             n_kv_heads, head_dim, scale, window, splits, out=out,
-                            max_len=min_len - 1 if n_long else 0, uniform_len=uniform, sink=sink, keep_first=keep_first)
+                            max_len=min_len - 1 if n_long else 0, uniform_len=uniform, sink=sink, keep_first=keep_first, n_groups=groups)
     return out
 
 
