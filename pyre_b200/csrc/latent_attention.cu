@@ -52,10 +52,36 @@ __device__ __forceinline__ float head_gate_of(const T* gates, long long gate_str
 //   cache[slot[t]] = [ rmsnorm(latent) * wc | rotate(key part) ]          rows of `row` >= rank + rope entries
 //   qa[t, h, rank ..] = [ rotate(rotated part of head h's query) | 0 ]    (qa null: the queries are handled elsewhere);
 //                       head h's query lies at column qh_col + h (dq + rope), its rotated part last
-// One block per token.
+// What bounds it is a chain of memory latencies on little data (a decoded token's projection may be sixteen partial sums of a few
+// thousand columns), so a token's three independent pieces (blockIdx.y: the query latent, the cached row, the rotated queries)
+// go to blocks of their own, a thread reads four neighbouring columns of all partial sums at once and keeps the values between the sum of
+// squares and the result.  Four tokens, 768 + 320 columns in partial sums: 18.5 -> 6.9 us (one block of 128
+// threads per token read a column at a time, twice).
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void latent_prepare_kernel(const T* proj, const float* parts, int n_parts, long long part_stride, int W,
+constexpr int LP_THREADS = 256, LP_KEEP = 4;
+
+// V neighbouring columns from `at` on, the partial sums added in their order
+template <typename T, int V>
+__device__ __forceinline__ void proj_vec(const T* proj, const float* parts, int n_parts, long long part_stride, size_t at, float (&v)[V]) {
+    if (parts) {
+        Vec<float, V> acc = load_vec<float, V>(parts + at);
+#pragma unroll 8
+        for (int s = 1; s < n_parts; ++s) {
+            const Vec<float, V> q = load_vec<float, V>(parts + (size_t)s * part_stride + at);
+#pragma unroll
+            for (int e = 0; e < V; ++e) acc.v[e] += q.v[e];
+        }
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = acc.v[e];
+    } else {
+        const Vec<T, V> q = load_vec<T, V>(proj + at);
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] = to_f32<T>(q.v[e]);
+    }
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(LP_THREADS) latent_prepare_kernel(const T* proj, const float* parts, int n_parts, long long part_stride, int W,
                                       int q_col, int q_rank, int c_col, int rank, int rope, int rot, const float* wq,
                                       const float* wc, float eps, const float* cos_t, const float* sin_t, T* cq_out,
                                       T* cache, const int* slot_mapping, int row, long long n_pages, int page_size,
@@ -65,23 +91,61 @@ __global__ void latent_prepare_kernel(const T* proj, const float* parts, int n_p
     pdl_wait();
     const int t = blockIdx.x;
     const size_t base = (size_t)t * W;
-    if (q_rank > 0) {
-        float ss = 0.f;
-        for (int i = threadIdx.x; i < q_rank; i += blockDim.x) {
-            const float v = proj_at<T>(proj, parts, n_parts, part_stride, base + q_col + i);
-            ss = fmaf(v, v, ss);
+    // dst[i] = rmsnorm(columns col .. col + width)[i] * w[i]
+    auto normed = [&](int col, int width, const float* w, T* dst) {
+        float keep[LP_KEEP][V], ss = 0.f;
+        auto add = [&](const float (&v)[V]) {
+#pragma unroll
+            for (int e = 0; e < V; ++e) ss = fmaf(v[e], v[e], ss);
+        };
+#pragma unroll
+        for (int n = 0; n < LP_KEEP; ++n) {
+            const int i = (n * LP_THREADS + threadIdx.x) * V;
+            if (i < width) {
+                proj_vec<T, V>(proj, parts, n_parts, part_stride, base + col + i, keep[n]);
+                add(keep[n]);
+            }
         }
-        const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)q_rank + eps);
-        for (int i = threadIdx.x; i < q_rank; i += blockDim.x) {
-            const float v = proj_at<T>(proj, parts, n_parts, part_stride, base + q_col + i);
-            cq_out[(size_t)t * q_rank + i] = from_f32<T>(__fmul_rn(__fmul_rn(v, rstd), wq[i]));
+        for (int i = (LP_KEEP * LP_THREADS + threadIdx.x) * V; i < width; i += LP_THREADS * V) {
+            float v[V];
+            proj_vec<T, V>(proj, parts, n_parts, part_stride, base + col + i, v);
+            add(v);
         }
-    }
+        const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
+        auto put = [&](int i, const float (&v)[V]) {
+            Vec<T, V> o;
+#pragma unroll
+            for (int e = 0; e < V; ++e) o.v[e] = from_f32<T>(__fmul_rn(__fmul_rn(v[e], rstd), w[i + e]));
+            store_vec<T, V>(dst + i, o);
+        };
+#pragma unroll
+        for (int n = 0; n < LP_KEEP; ++n) {
+            const int i = (n * LP_THREADS + threadIdx.x) * V;
+            if (i < width) put(i, keep[n]);
+        }
+        for (int i = (LP_KEEP * LP_THREADS + threadIdx.x) * V; i < width; i += LP_THREADS * V) {
+            float v[V];
+            proj_vec<T, V>(proj, parts, n_parts, part_stride, base + col + i, v);
+            put(i, v);
+        }
+    };
     const float* ct = cos_t + (size_t)t * (rot / 2);
     const float* st = sin_t + (size_t)t * (rot / 2);
-    if (qa) {
+    if (blockIdx.y == 0) {
+        const int slot = cache ? pyre_checked_slot(slot_mapping[t], n_pages, page_size, err_flag) : -1;
+        if (slot < 0) return;   // the whole block
+        T* dst = cache + (size_t)slot * row;
+        normed(c_col, rank, wc, dst);
+        for (int i = threadIdx.x; i < rope; i += LP_THREADS) {
+            const size_t at0 = base + c_col + rank;
+            dst[rank + i] = from_f32<T>(turned([&](int j) { return proj_at<T>(proj, parts, n_parts, part_stride, at0 + j); }, i, rot, halves, ct, st));
+        }
+        for (int i = rank + rope + threadIdx.x; i < row; i += LP_THREADS) dst[i] = from_f32<T>(0.f);
+    } else if (blockIdx.y == 1 && q_rank > 0) {
+        normed(q_col, q_rank, wq, cq_out + (size_t)t * q_rank);
+    } else if (qa) {
         const int tail = row - rank;
-        for (int idx = threadIdx.x; idx < nh * tail; idx += blockDim.x) {
+        for (int idx = threadIdx.x; idx < nh * tail; idx += LP_THREADS) {
             const int h = idx / tail, i = idx - h * tail;
             float o = 0.f;
             if (i < rope) {
@@ -91,24 +155,6 @@ __global__ void latent_prepare_kernel(const T* proj, const float* parts, int n_p
             qa[((size_t)t * nh + h) * row + rank + i] = from_f32<T>(o);
         }
     }
-    const int slot = cache ? pyre_checked_slot(slot_mapping[t], n_pages, page_size, err_flag) : -1;
-    if (slot < 0) return;   // the whole block
-    T* dst = cache + (size_t)slot * row;
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < rank; i += blockDim.x) {
-        const float v = proj_at<T>(proj, parts, n_parts, part_stride, base + c_col + i);
-        ss = fmaf(v, v, ss);
-    }
-    const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)rank + eps);
-    for (int i = threadIdx.x; i < rank; i += blockDim.x) {
-        const float v = proj_at<T>(proj, parts, n_parts, part_stride, base + c_col + i);
-        dst[i] = from_f32<T>(__fmul_rn(__fmul_rn(v, rstd), wc[i]));
-    }
-    for (int i = threadIdx.x; i < rope; i += blockDim.x) {
-        const size_t at0 = base + c_col + rank;
-        dst[rank + i] = from_f32<T>(turned([&](int j) { return proj_at<T>(proj, parts, n_parts, part_stride, at0 + j); }, i, rot, halves, ct, st));
-    }
-    for (int i = rank + rope + threadIdx.x; i < row; i += blockDim.x) dst[i] = from_f32<T>(0.f);
 }
 
 PYRE_API int pyre_latent_prepare(const void* proj, const float* parts, int n_parts, long long part_stride, int W, int q_col,
@@ -121,16 +167,17 @@ PYRE_API int pyre_latent_prepare(const void* proj, const float* parts, int n_par
         row < rank + rope || (q_rank > 0 && (!wq || !cq_out)) || !wc || (cache && !slot_mapping) ||
         (rot > 0 && (!cos_t || !sin_t)) || (qa && (nh <= 0 || dq <= 0 || qh_col < 0 || (long long)qh_col + (long long)nh * (dq + rope) > W)))
         return PYRE_ERR_BAD_ARG;
-    const int threads = qa && nh * (row - rank) >= 1024 ? 256 : 128;
-    if (dtype == PYRE_BF16)
-        pyre_launch(latent_prepare_kernel<__nv_bfloat16>, dim3(n_tokens), dim3(threads), 0, stream, (const __nv_bfloat16*)proj, parts,
-                    n_parts, part_stride, W, q_col, q_rank, c_col, rank, rope, rot, wq, wc, eps, cos_t, sin_t,
-                    (__nv_bfloat16*)cq_out, (__nv_bfloat16*)cache, slot_mapping, row, n_pages, page_size, halves, (__nv_bfloat16*)qa, qh_col, nh, dq, err_flag);
-    else if (dtype == PYRE_F32)
-        pyre_launch(latent_prepare_kernel<float>, dim3(n_tokens), dim3(threads), 0, stream, (const float*)proj, parts, n_parts,
-                    part_stride, W, q_col, q_rank, c_col, rank, rope, rot, wq, wc, eps, cos_t, sin_t, (float*)cq_out,
-                    (float*)cache, slot_mapping, row, n_pages, page_size, halves, (float*)qa, qh_col, nh, dq, err_flag);
+    const dim3 grid(n_tokens, 1 + (q_rank > 0 ? 1 : 0) + (qa ? 1 : 0));
+    // four columns at a time where columns, row lengths and addresses allow it (never depending on the batch)
+    const int esize = dtype == PYRE_F32 ? 4 : 2, in_esize = parts ? 4 : esize;
+    const bool vec = W % 4 == 0 && part_stride % 4 == 0 && q_col % 4 == 0 && q_rank % 4 == 0 && c_col % 4 == 0 && rank % 4 == 0 && row % 4 == 0 &&
+                     ((uintptr_t)(parts ? (const void*)parts : proj)) % (4 * in_esize) == 0 && (uintptr_t)cache % (4 * esize) == 0 && (uintptr_t)cq_out % (4 * esize) == 0;
+#define GO(T, V) pyre_launch(latent_prepare_kernel<T, V>, grid, dim3(LP_THREADS), 0, stream, (const T*)proj, parts, n_parts, part_stride, W, q_col, q_rank, c_col, \
+                             rank, rope, rot, wq, wc, eps, cos_t, sin_t, (T*)cq_out, (T*)cache, slot_mapping, row, n_pages, page_size, halves, (T*)qa, qh_col, nh, dq, err_flag)
+    if (dtype == PYRE_BF16) vec ? GO(__nv_bfloat16, 4) : GO(__nv_bfloat16, 1);
+    else if (dtype == PYRE_F32) vec ? GO(float, 4) : GO(float, 1);
     else return PYRE_ERR_BAD_ARG;
+#undef GO
     PYRE_LAUNCH_CHECK();
     return 0;
 }
@@ -591,25 +638,54 @@ __global__ void __launch_bounds__(512) latent_attention_mma_kernel(
     }
 }
 
-// out[t, h] = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m): the shares of one (token, head); maxima are base-2 exponents
-__global__ void latent_combine_kernel(const float* part_o, const float* part_ml, __nv_bfloat16* out, int n_splits, int rank,
+// out[t, h] = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m): the shares of one (token, head); maxima are base-2 exponents.
+// A share that saw no key has left nothing in part_o: what lies there is read (it costs no wait of its own) but not used.  All
+// maxima, sums and the first LM_ONCE shares are asked for at once.
+constexpr int LM_ONCE = 16;
+
+__global__ void __launch_bounds__(128) latent_combine_kernel(const float* part_o, const float* part_ml, __nv_bfloat16* out, int n_splits, int rank,
                                       int nh, const float* head_sinks, const __nv_bfloat16* gates, long long gate_stride) {
+    extern __shared__ float weight_s[];      // [n_splits]
     pdl_trigger();
     pdl_wait();
     const size_t th = blockIdx.x;
-    const float* ml = part_ml + th * n_splits * 2;
-    float mx = -INFINITY;
-    for (int s = 0; s < n_splits; ++s) mx = fmaxf(mx, ml[2 * s]);
-    float denom = 0.f;
-    for (int s = 0; s < n_splits; ++s) denom += ml[2 * s] == -INFINITY ? 0.f : ml[2 * s + 1] * exp2f(ml[2 * s] - mx);
+    const int lane = threadIdx.x & 31;
     const int t = (int)(th / nh), head = (int)(th - (size_t)t * nh);
-    if (head_sinks) denom += exp2f(head_sinks[head] * 1.4426950408889634f - mx);
-    const float inv = head_gate_of<__nv_bfloat16>(gates, gate_stride, t, head) / denom;
+    const float* po = part_o + th * n_splits * rank;
+    float part[LM_ONCE];      // this thread's first column
+    const int c0 = min((int)threadIdx.x, rank - 1);
+#pragma unroll
+    for (int s = 0; s < LM_ONCE; ++s) part[s] = s < n_splits ? po[(size_t)s * rank + c0] : 0.f;
+    if (threadIdx.x < 32) {
+        const float2* ml = reinterpret_cast<const float2*>(part_ml) + th * n_splits;
+        float mx = -INFINITY, denom = 0.f;
+        for (int s = lane; s < n_splits; s += 32) mx = fmaxf(mx, ml[s].x);
+        mx = warp_max(mx);
+        for (int s = lane; s < n_splits; s += 32) {
+            const float2 v = ml[s];
+            const float w = exp2f(v.x - mx);
+            if (v.x != -INFINITY) denom = fmaf(v.y, w, denom);
+            weight_s[s] = v.x == -INFINITY ? -1.f : w;      // -1: nothing there
+        }
+        denom = warp_sum(denom);
+        if (head_sinks) denom += exp2f(head_sinks[head] * 1.4426950408889634f - mx);
+        const float inv = head_gate_of<__nv_bfloat16>(gates, gate_stride, t, head) / denom;
+        for (int s = lane; s < n_splits; s += 32)
+            if (weight_s[s] != -1.f) weight_s[s] *= inv;
+    }
+    __syncthreads();
     for (int c = threadIdx.x; c < rank; c += blockDim.x) {
+        if (c != c0) {
+#pragma unroll
+            for (int s = 0; s < LM_ONCE; ++s) part[s] = s < n_splits ? po[(size_t)s * rank + c] : 0.f;
+        }
         float acc = 0.f;
-        for (int s = 0; s < n_splits; ++s)
-            if (ml[2 * s] != -INFINITY) acc = fmaf(part_o[(th * n_splits + s) * rank + c], exp2f(ml[2 * s] - mx), acc);
-        out[th * rank + c] = __float2bfloat16_rn(acc * inv);
+#pragma unroll
+        for (int s = 0; s < LM_ONCE; ++s)
+            if (s < n_splits && !(weight_s[s] == -1.f)) acc = fmaf(part[s], weight_s[s], acc);
+        for (int s = LM_ONCE; s < n_splits; ++s)
+            if (!(weight_s[s] == -1.f)) acc = fmaf(po[(size_t)s * rank + c], weight_s[s], acc);
+        out[th * rank + c] = __float2bfloat16_rn(acc);
     }
 }
 
@@ -642,7 +718,7 @@ PYRE_API int pyre_latent_attention_mma(const void* qa, const void* cache, void* 
                 gate_stride, n_splits, max_len, n_pages, err_flag);
     PYRE_LAUNCH_CHECK();
     if (n_splits > 1) {
-        pyre_launch(latent_combine_kernel, dim3(n_tokens * nh), dim3(128), 0, stream, (const float*)part_o, (const float*)part_ml,
+        pyre_launch(latent_combine_kernel, dim3(n_tokens * nh), dim3(128), (size_t)n_splits * sizeof(float), stream, (const float*)part_o, (const float*)part_ml,
                     (__nv_bfloat16*)out, n_splits, rank, nh, head_sinks, (const __nv_bfloat16*)gates, gate_stride);
         PYRE_LAUNCH_CHECK();
     }

@@ -696,9 +696,6 @@ def _attention_plan(ctx, use_tc: bool, min_len: int, n_heads: int, n_kv_heads: i
     """How a step's attention is cut: (tokens of the long entries, their key splits, short entries, splits, the length
     all entries share or 0, row groups of the short entries).  From host-side facts of the step and the mixer's sizes alone."""
     lens = ctx.cu_seqlens_host[1:] - ctx.cu_seqlens_host[:-1]
-    page_size = cache_layer.shape[3]
-    use_tc = USE_TC_ATTENTION and head_dim in PREFILL_HEAD_DIMS and page_size & (page_size - 1) == 0 and page_size >= 4
-    min_len = TC_ATTENTION_MIN_LEN if use_tc else PREFILL_MIN_LEN
     long_mask = lens >= min_len if head_dim in PREFILL_HEAD_DIMS else lens < 0
     n_long = int(lens[long_mask].sum())
     n_short_seqs = int((~long_mask).sum())
@@ -2049,7 +2046,9 @@ def latent_mma_ok(dtype: torch.dtype, row: int) -> bool:
 def latent_attention_splits(n_tiles: int, n_heads: int, rank: int, span: int, row: "int | None" = None) -> int:
     """Into how many shares the tensor-core latent attention cuts the keys of every row tile: as many as fill the CTAs
     that are resident at once (its shared memory and threads allow one to a few per SM: whole rounds, since a second
-    round of CTAs costs as much as the first), at least four key tiles per share, at most 16.  ``span``: the most keys
+    round of CTAs costs as much as the first) with at least four key tiles per share, or as many as have an SM each with at least
+    two (a share is a chain of memory latencies, and SMs idle: four tokens of 16 heads after 700 rows, combining included, 24.5 us
+    with five shares, 18.5 with eleven); at most 16.  ``span``: the most keys
     a tile walks; ``row``: entries of a cached row (default: the latent and a rotated part of a quarter of it)."""
     ctas = max(1, n_tiles * -(-n_heads // LATENT_MMA_ROWS))      # the column groups of a wide latent are warps of one CTA
     groups = -(-rank // LATENT_MMA_COLS)
@@ -2057,7 +2056,7 @@ def latent_attention_splits(n_tiles: int, n_heads: int, rank: int, span: int, ro
     smem = (LATENT_MMA_ROWS + 2 * LATENT_MMA_KEYS) * (row + 8) * 2 + (4 * groups * 16 * 32 * 4 if groups > 1 else 0)
     resident = sm_count() * max(1, min(227 * 1024 // smem, 2048 // (128 * groups), 4))
     tiles = -(-span // LATENT_MMA_KEYS) + 1
-    return int(max(1, min(resident // ctas, tiles // 4, 16)))
+    return int(max(1, min(resident // ctas, tiles // 4, 16), min(sm_count() // ctas, tiles // 2, 16)))
 
 
 def latent_attention_mma(qa: torch.Tensor, cache_layer: torch.Tensor, block_table: torch.Tensor, cu_seqlens: torch.Tensor,
