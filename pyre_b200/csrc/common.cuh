@@ -121,6 +121,13 @@ __device__ __forceinline__ unsigned long long pyre_now_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
+// Large constants (a router's rows) asked for before pdl_wait(): a decode step streams hundreds of megabytes of weights between two
+// uses, so they come from memory.  n floats from p on; `who` of `count` threads.  (Not for norm weights and biases: asked
+// for ahead in the norm and rotary kernels they made decode steps of 8 and 64 requests 1 % slower.)
+__device__ __forceinline__ void prefetch_floats(const float* p, int n, int who, int count) {
+    if (!p) return;
+    for (int i = who * 32; i < n; i += count * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + i));
+}
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 #include <cstdlib>

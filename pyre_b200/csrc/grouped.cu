@@ -557,6 +557,12 @@ __global__ void route_kernel(const T* h, const float* w, const float* correction
                              int groups, int keep) {
     extern __shared__ float z_smem[];   // [n_out] logits, then scores; [n_out] choice scores; [groups] group scores
     pdl_trigger();
+    // four blocks ask for the router's rows (a few hundred KB) while they wait; with the loads of a row unrolled by eight:
+    // 18.8 -> 15.6 us a launch on average (34 outputs of 2,048 columns, steps of 4 tokens and one prompt)
+    if (blockIdx.x < 4) {
+        prefetch_floats(w, n_out * H, blockIdx.x * blockDim.x + threadIdx.x, 4 * blockDim.x);
+        if (blockIdx.x == 0) prefetch_floats(correction, n_out, threadIdx.x, blockDim.x);
+    }
     pdl_wait();
     const int t = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
@@ -569,6 +575,7 @@ __global__ void route_kernel(const T* h, const float* w, const float* correction
         const float* wr = w + (size_t)e * H;
         float acc[4] = {0.f, 0.f, 0.f, 0.f};
         if (vec) {
+#pragma unroll 8
             for (int i = lane * 4; i < H; i += 128) {
                 const Vec<T, 4> hv = load_vec<T, 4>(hr + i);
                 const Vec<float, 4> wv = load_vec<float, 4>(wr + i);
