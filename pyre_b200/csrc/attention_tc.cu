@@ -15,11 +15,17 @@
 //                        copy costs about a hundred cycles, so the two rings have a warp each.
 //   warp 1, one thread : issues the MMAs.  S (128 x 64, fp32, one of two TMEM buffers) = Q K^T with
 //                        both operands K-major; then, once the softmax threads have put P
-//                        (bf16, 128 x 64) into shared memory, O (128 x hd, TMEM columns
-//                        128..) += P V with V as an MN-major operand straight from the page rows.
+//                        (bf16, 128 x 64) over the S it came from, O (128 x hd, TMEM columns
+//                        128..) += P V with P read from tensor memory and V as an MN-major operand
+//                        straight from the page rows.
 //   warps 2..5         : one thread per query row.  Reads its row of S with tcgen05.ld, masks
 //                        by position (causal limit, window), keeps the running maximum and sum
 //                        in fp32, writes P.  No shuffles: a row lives in one thread.
+// P stays in tensor memory, over the scores it came from: through shared memory (16 KB written and read per tile) 1,024 tokens after
+// 3,072 (40 / 8 heads of 128) took 115 us instead of 104, 500 after 30,720 (28 / 4) 226 instead of 222.  Cycles of a row
+// thread per tile there: 1,030 softmax (two such warps share a scheduler), 330 waiting for scores, 215 for the P V before, 250
+// handing over, 210 tensor memory.  What did not help: two threads per row (265 us), a third K stage (230), every
+// fourth to second exponential on the FMA pipe (243 to 257).
 // The accumulator O is rescaled only when a row's maximum grows by more than 2^8 beyond the
 // value it was scaled with (probabilities then stay below 256, exact in the final O / l);
 // the rescale is a tcgen05.ld / multiply / tcgen05.st pass over the row.
@@ -114,6 +120,14 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
+// A (here P, 16 keys = 8 columns of packed pairs) from tensor memory
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
@@ -197,12 +211,10 @@ struct Smem {
     static constexpr int HALVES = HD / 64;                 // 128-byte column boxes per row
     static constexpr int Q_BYTES = HALVES * BM * 128;
     static constexpr int KV_TILE = HALVES * BN * 128;      // one K (or V) tile
-    static constexpr int P_BYTES = BM * 128;               // 128 rows x 64 bf16
     static constexpr int OFF_Q = 0;
     static constexpr int OFF_K = Q_BYTES;                  // [2 stages]
     static constexpr int OFF_V = OFF_K + 2 * KV_TILE;      // [2 stages]
-    static constexpr int OFF_P = OFF_V + 2 * KV_TILE;
-    static constexpr int OFF_BAR = OFF_P + P_BYTES;        // q_full, k_full[2], v_full[2], s_full[2], o_ready[2], p_full
+    static constexpr int OFF_BAR = OFF_V + 2 * KV_TILE;    // q_full, k_full[2], v_full[2], s_full[2], o_ready[2], p_full
     static constexpr int N_BARS = 10;
     static constexpr int TOTAL = OFF_BAR + N_BARS * 8 + 16;   // the dynamic window must start 1024-byte aligned (checked)
 };
@@ -375,10 +387,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int i = 0; i < n_tiles && ok; ++i) {
                 const int st = i & 1;
                 if (i + 1 < n_tiles) {
-                    ok = issue_s(i + 1);
+                    // the scores of tile i + 1 go where P of tile i - 1 lies: its P V has to be over (nothing orders two MMAs on
+                    // different accumulators); the row threads are busy with tile i meanwhile
+                    if (i > 0) ok = mbar_wait(bar_o + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1, abort_flag, p.err_flag);
+                    if (ok) ok = issue_s(i + 1);
                     if (!ok) break;
                 }
-                ok = mbar_wait(bar_p, i & 1, abort_flag, p.err_flag);   // P is in shared memory, O has been rescaled
+                ok = mbar_wait(bar_p, i & 1, abort_flag, p.err_flag);   // P is in tensor memory, O has been rescaled
                 if (ok) ok = mbar_wait(bar_v_full + 8 * st, (i >> 1) & 1, abort_flag, p.err_flag);
                 if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -386,9 +401,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 // O += P V: 4 steps of 16 keys; V rows are 128 B per column box, the second box lies BN * 128 B further
 #pragma unroll
                 for (int j = 0; j < BN / 16; ++j)
-                    umma_bf16(tmem_base + O_COL, desc_k_major(base + L::OFF_P) + 2 * j,
-                              desc_mn_major(vd + j * (16 * 128), BN * 128), idesc_pv, (i > 0 || j > 0) ? 1u : 0u);
-                umma_commit(bar_o + 8 * st);   // O holds this tile; P may be overwritten, the V stage refilled
+                    umma_bf16_ts(tmem_base + O_COL, tmem_base + S_COL + st * BN + 8 * j,
+                                 desc_mn_major(vd + j * (16 * 128), BN * 128), idesc_pv, (i > 0 || j > 0) ? 1u : 0u);
+                umma_commit(bar_o + 8 * st);   // O holds this tile; the V stage may be refilled (and P's columns be written again)
             }
         }
     } else {
@@ -474,7 +489,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             unpack2(sum2[1], sum[2], sum[3]);
             l_sum = l_sum * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
 
-            // the previous tile's P V must be complete before P is overwritten or O is touched
+            // P (bf16 pairs, a column of 32 bits each) over the scores it came from
+#pragma unroll
+            for (int c = 0; c < BN / 2; c += 16) {
+                uint32_t w[16];
+#pragma unroll
+                for (int q = 0; q < 16; ++q) w[q] = pack_bf16(sc[2 * (c + q)], sc[2 * (c + q) + 1]);
+                tmem_st16(lane_addr + S_COL + s * BN + c, w);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            // the previous tile's P V must be complete before O is touched (its barrier also bounds how far this thread runs ahead)
             if (i > 0) {
                 ok = mbar_wait(bar_o + 8 * ((i - 1) & 1), ((i - 1) >> 1) & 1, abort_flag, p.err_flag);
                 alive = __all_sync(0xffffffffu, ok);
@@ -505,18 +529,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (key > pos_last || (key < lo_cta && key >= keep))
                         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(vd + (rem >> 3) * (BN * 128) + k * 128 + (rem & 7) * 16), "r"(0u) : "memory");
                 }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes before the tensor core reads them
             }
-            // P (bf16) into shared memory, K-major with the 128-byte swizzle: chunk c of row r at c ^ (r & 7)
-            {
-                const uint32_t prow = base + L::OFF_P + row * 128;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const uint32_t w0 = pack_bf16(sc[8 * c], sc[8 * c + 1]), w1 = pack_bf16(sc[8 * c + 2], sc[8 * c + 3]);
-                    const uint32_t w2 = pack_bf16(sc[8 * c + 4], sc[8 * c + 5]), w3 = pack_bf16(sc[8 * c + 6], sc[8 * c + 7]);
-                    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(prow + ((c ^ (row & 7)) * 16)), "r"(w0), "r"(w1), "r"(w2), "r"(w3) : "memory");
-                }
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes before the tensor core reads them
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_p);
