@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(256) grouped_linear_kernel(GroupedArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// bfloat16, groups of few rows: a 64 x 64 tile by mma.sync, bound by reading the weights (a decoded token's experts have a row
+// bfloat16, groups of few rows: tiles of 64 features by mma.sync, bound by reading the weights (a decoded token's experts have a row
 // or two each).  K in steps of 64 through a ring of four stages filled by cp.async, so that a CTA has 24 KB of weights in
 // flight and three CTAs fit on an SM; each of the four warps owns 16 output features and as many 16-row pieces as the
 // tile has rows, so that two rows do not cost the multiplications of 64.  Measured inside a decode step of 4 tokens (16
@@ -150,8 +150,15 @@ __global__ void __launch_bounds__(256) grouped_linear_kernel(GroupedArgs a) {
 // tiles whatever the rows, one step ahead through registers); 64 tokens: 111 -> 70 us.
 // Needs K % 8 == 0 and 16-byte aligned rows of x and w.
 // ---------------------------------------------------------------------------
-constexpr int GT_K = 64, GT_LD = GT_K + 8, GT_STAGES = 4;   // padded rows: 144 bytes, conflict-free for ldmatrix
-constexpr int GT_STAGE = (GB_M + GB_N) * GT_LD, GT_SMEM = GT_STAGES * GT_STAGE * 2;
+//
+// ROWS: the height of a tile.  Groups of few rows take tiles of 16 rows, whose ring holds little but weights; a group with more rows
+// takes more tiles, whose weights then come out of the L2 cache.  32 experts of 2048 x 2048, top 4, captured launches one after the
+// other, 64 rows of four stages / 16 rows of six / of four: 4 tokens 27.4 / 21.6 / 23.5 us, 8: 49.7 / 39.5 / 45.6, 32: 72.3 / 57.2 /
+// 50.5, 128: 76.4 / 70.6 / 64.6.
+constexpr int GT_K = 64, GT_LD = GT_K + 8;   // padded rows: 144 bytes, conflict-free for ldmatrix
+template <int ROWS, int STAGES> struct GtRing {
+    static constexpr int STAGE = (ROWS + GB_N) * GT_LD, SMEM = STAGES * STAGE * 2;
+};
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], const void* p) {
     const uint32_t addr = (uint32_t)__cvta_generic_to_shared(p);
@@ -189,9 +196,11 @@ __device__ __forceinline__ void store_pair(const GroupedArgs& a, size_t at, int 
     }
 }
 
+template <int ROWS, int GT_STAGES>
 __global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs a) {
-    extern __shared__ __align__(16) __nv_bfloat16 g_ring[];      // [stages][64 rows of x, 64 rows of w][GT_LD]
-    __shared__ int src_row[GB_M], dst_row[GB_M];
+    constexpr int GT_STAGE = GtRing<ROWS, GT_STAGES>::STAGE;
+    extern __shared__ __align__(16) __nv_bfloat16 g_ring[];      // [stages][ROWS rows of x, 64 rows of w][GT_LD]
+    __shared__ int src_row[ROWS], dst_row[ROWS];
     pdl_trigger();
     const int n0 = blockIdx.y * GB_N;
     const int n_steps = (a.K + GT_K - 1) / GT_K;
@@ -199,7 +208,7 @@ __global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs 
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(g_ring);
     auto load_w = [&](const __nv_bfloat16* w, int s) {
         if (s >= n_steps) return;
-        const uint32_t to = ring + ((s % GT_STAGES) * GT_STAGE + GB_M * GT_LD) * 2;
+        const uint32_t to = ring + ((s % GT_STAGES) * GT_STAGE + ROWS * GT_LD) * 2;
         const int k = s * GT_K + lk;
         const bool in_k = k < a.K;
 #pragma unroll
@@ -213,11 +222,11 @@ __global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs 
         for (int s = 0; s < GT_STAGES - 1; ++s) load_w(w, s);
     }
     pdl_wait();
-    if (!grouped_tile(a, g, first, count)) {
+    if (!grouped_tile<ROWS>(a, g, first, count)) {
         asm volatile("cp.async.wait_all;" ::: "memory");
         return;
     }
-    if (threadIdx.x < GB_M) {
+    if (threadIdx.x < ROWS) {
         const int p = first + threadIdx.x;
         const bool live = (int)threadIdx.x < count;
         src_row[threadIdx.x] = live ? (a.src ? a.src[p] : p) : -1;
@@ -241,9 +250,9 @@ __global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs 
         load_x(s);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
-    float acc[4][2][4];
+    float acc[ROWS / 16][2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < ROWS / 16; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -255,13 +264,13 @@ __global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs 
         load_x(s + GT_STAGES - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const __nv_bfloat16* xs = g_ring + (s % GT_STAGES) * GT_STAGE;
-        const __nv_bfloat16* ws = xs + (GB_M + warp * 16) * GT_LD;
+        const __nv_bfloat16* ws = xs + (ROWS + warp * 16) * GT_LD;
 #pragma unroll
         for (int kk = 0; kk < GT_K; kk += 16) {
             uint32_t bf[4];      // 16 n-rows: two 8-wide n tiles, both k halves
             ldmatrix_x4(bf, ws + ((lane & 7) + ((lane >> 4) << 3)) * GT_LD + kk + ((lane >> 3) & 1) * 8);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < ROWS / 16; ++i) {
                 if (i < m_tiles) {
                     uint32_t af[4];
                     ldmatrix_x4(af, xs + (i * 16 + (lane & 15)) * GT_LD + kk + (lane >> 4) * 8);
@@ -273,7 +282,7 @@ __global__ void __launch_bounds__(128, 3) grouped_linear_mma_kernel(GroupedArgs 
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < ROWS / 16; ++i)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int dr = dst_row[i * 16 + (lane >> 2) + half * 8];
@@ -508,29 +517,31 @@ PYRE_API int pyre_grouped_linear(const void* x, long long x_row_stride, long lon
     if (N <= 0 || K <= 0 || G <= 0) return PYRE_ERR_BAD_ARG;
     GroupedArgs a{x, x_row_stride, x_group_stride, w, w_group_stride, out, out_row_stride, out_group_stride,
                   offsets, src, dst, M, N, K, G, out_f32};
-    dim3 grid;
-    if (offsets) {
-        if (places <= 0) return 0;
-        grid = dim3(ceil_div(places, GB_M) + G, ceil_div(N, GB_N), 1);
-    } else {
-        if (M <= 0) return 0;
-        grid = dim3(ceil_div(M, GB_M), ceil_div(N, GB_N), G);
-    }
+    if ((offsets ? places : M) <= 0) return 0;
+    auto tiles_of = [&](int rows, int features) {
+        return offsets ? dim3(ceil_div(places, rows) + G, ceil_div(N, features), 1) : dim3(ceil_div(M, rows), ceil_div(N, features), G);
+    };
+    const dim3 grid = tiles_of(GB_M, GB_N);
     if (dtype == PYRE_BF16 && use_mma) {
         if (K % 8 || x_row_stride % 8 || x_group_stride % 8 || w_group_stride % 8 || (((uintptr_t)x | (uintptr_t)w) & 15))
             return PYRE_ERR_UNSUPPORTED;
-        // groups of about a hundred rows or more (a prompt portion's heads or experts): the large tiles
+        // by the rows per group on average: about a hundred or more (a prompt portion's heads or experts), tcgen05 on tiles of 128;
+        // up to 16, tiles of 16 rows, with the deeper ring where nearly every group has one tile of a row or two (the figures
+        // stand with the kernels)
         const long long rows_per_group = offsets ? (long long)places / G : M;
+        auto small = [&](auto kernel, int rows, int smem, bool (&done)[PYRE_MAX_DEVICES]) {
+            if (const int rc = allow_smem(kernel, smem, done)) return rc;
+            return (int)pyre_launch(kernel, tiles_of(rows, GB_N), dim3(128), (size_t)smem, stream, a);
+        };
+        static bool done_tc[PYRE_MAX_DEVICES] = {}, done_64[PYRE_MAX_DEVICES] = {}, done_16[PYRE_MAX_DEVICES] = {}, done_16d[PYRE_MAX_DEVICES] = {};
+        int rc;
         if (rows_per_group >= 96) {
-            const dim3 big = offsets ? dim3(ceil_div(places, GL_M) + G, ceil_div(N, GL_N), 1) : dim3(ceil_div(M, GL_M), ceil_div(N, GL_N), G);
-            static bool done[PYRE_MAX_DEVICES] = {};
-            if (const int rc = allow_smem(grouped_linear_tc_kernel, GL_SMEM, done)) return rc;
-            pyre_launch(grouped_linear_tc_kernel, big, dim3(GL_THREADS), (size_t)GL_SMEM, stream, a, err_flag);
-        } else {
-            static bool done[PYRE_MAX_DEVICES] = {};
-            if (const int rc = allow_smem(grouped_linear_mma_kernel, GT_SMEM, done)) return rc;
-            pyre_launch(grouped_linear_mma_kernel, grid, dim3(128), (size_t)GT_SMEM, stream, a);
-        }
+            rc = allow_smem(grouped_linear_tc_kernel, GL_SMEM, done_tc);
+            if (!rc) rc = (int)pyre_launch(grouped_linear_tc_kernel, tiles_of(GL_M, GL_N), dim3(GL_THREADS), (size_t)GL_SMEM, stream, a, err_flag);
+        } else if (rows_per_group > 16) rc = small(grouped_linear_mma_kernel<64, 4>, 64, GtRing<64, 4>::SMEM, done_64);
+        else if (rows_per_group > 2) rc = small(grouped_linear_mma_kernel<16, 4>, 16, GtRing<16, 4>::SMEM, done_16);
+        else rc = small(grouped_linear_mma_kernel<16, 6>, 16, GtRing<16, 6>::SMEM, done_16d);
+        if (rc) return rc;
     } else if (dtype == PYRE_BF16) pyre_launch(grouped_linear_kernel<__nv_bfloat16>, grid, dim3(256), 0, stream, a);
     else if (dtype == PYRE_F32) pyre_launch(grouped_linear_kernel<float>, grid, dim3(256), 0, stream, a);
     else return PYRE_ERR_BAD_ARG;

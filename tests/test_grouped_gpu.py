@@ -65,3 +65,16 @@ def test_product_per_head(ops, T, H, N, K):
     assert torch.isnan(out[:, :, N:]).all(), "columns beyond a head's result stay"
     for h in range(H):
         agree(out[:, h, :N], x[:, h].double(), w[h].double(), f"head {h}")
+
+
+@pytest.mark.parametrize("G,per", [(4, 2), (4, 3), (5, 16), (5, 17), (3, 95), (3, 96)])
+def test_where_the_kernels_take_over(ops, G, per):
+    """The rows per group at which another kernel takes a product, all of them in one group, so that it takes many tiles."""
+    g = torch.Generator(device="cuda").manual_seed(G * per)
+    places, N, K = G * per, 70, 136
+    offsets = torch.tensor([0] + [0] * (G - 1) + [places], dtype=torch.int32, device="cuda")
+    x = torch.randn(places, K, device="cuda", generator=g).to(torch.bfloat16)
+    w = torch.randn(G, N, K, device="cuda", generator=g).to(torch.bfloat16)
+    got = ops.expert_linear(x, w, offsets, None, places, torch.float32)
+    ops.check_device_errors()
+    agree(got, x.double(), w[G - 1].double(), "the last group")
