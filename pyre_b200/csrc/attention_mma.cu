@@ -770,7 +770,7 @@ PYRE_API int pyre_paged_attention_mma(const void* q, const void* cache, void* ou
                                       const int* block_table, int bt_stride, const int* cu_seqlens,
                                       const int* positions, int n_tokens, int n_seqs, int nh, int nkv, int hd,
                                       int page_size, int window, int keep_first, float scale, float sink, const float* head_sinks, int n_splits,
-                                      int max_len, long long n_pages, int uniform_len, int n_groups, int* err_flag, cudaStream_t stream) {
+                                      int max_len, long long n_pages, int uniform_len, int* err_flag, cudaStream_t stream) {
     if (n_tokens <= 0) return 0;
     if (hd % 16 || hd < 16 || hd > 128 || nkv <= 0 || nh % nkv || page_size <= 0 || n_splits < 1 || keep_first < 0) return PYRE_ERR_UNSUPPORTED;
     // without scratch the splits merge through a thread-block cluster (at most 16 CTAs)
@@ -810,11 +810,7 @@ PYRE_API int pyre_paged_attention_mma(const void* q, const void* cache, void* ou
     p.hpg = n_rep < 16 ? n_rep : 16;
     p.tpg = 16 / p.hpg;
     p.head_blocks = (n_rep + p.hpg - 1) / p.hpg;
-    // the sum over the entries taken of ceil(len / tpg): the caller's number, or else a bound.  Beside a prompt portion of
-    // thousands of tokens, which another kernel takes, the bound would launch hundreds of CTAs for each one with work
-    // (16 decoded tokens of 40 heads
-    // after up to 8,000 keys beside a portion of 1,024: 120 -> 76 us)
-    const int groups_bound = n_groups > 0 ? n_groups : n_tokens / p.tpg + n_seqs;
+    const int groups_bound = n_tokens / p.tpg + n_seqs;  // sum over entries of ceil(len / tpg) is at most this
     int rc;
 #define GO(HD_) rc = p.keep_first > 0 ? launch<HD_, true>(map, p, groups_bound, use_cluster, stream) : launch<HD_, false>(map, p, groups_bound, use_cluster, stream); break;
     switch (hd) {

@@ -40,7 +40,7 @@ SIGNATURES: dict[str, tuple[str, list]] = {
     "pyre_sample_slices": ("sampling", [I]),
     "pyre_paged_attention_generic": ("attention_generic", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, F, F, P, I, LL, P, I, P]),
     "pyre_sgemm_nt": ("gemm_f32", [P, LL, P, LL, P, LL, P, I, I, I, P]),
-    "pyre_paged_attention_mma": ("attention_mma", [P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, LL, I, I, P, P]),
+    "pyre_paged_attention_mma": ("attention_mma", [P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, LL, I, P, P]),
     "pyre_attention_prefill_tc": ("attention_tc", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, LL, I, I, F, F, P, I, I, P, P, P, P]),
     "pyre_attention_prefill": ("attention_prefill", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, LL, P, P]),
     "pyre_cast_rows": ("blockops", [P, P, LL, I, P]),

@@ -558,10 +558,9 @@ def paged_attention_mma(q: torch.Tensor, cache_layer: torch.Tensor, block_table:
                         n_kv_heads: int, head_dim: int, scale: float, window: "int | None" = None,
                         n_splits: int = 1, out: "torch.Tensor | None" = None,
                         scratch: "torch.Tensor | None" = None, max_len: int = 0, uniform_len: int = 0,
-                        sink: "float | None" = None, keep_first: int = 0, n_groups: int = 0) -> torch.Tensor:
+                        sink: "float | None" = None, keep_first: int = 0) -> torch.Tensor:
     """bfloat16 attention on the tensor cores over the block table (decode tokens and
-    prompt portions alike); ``n_groups``: how many row groups the entries taken have in all, where the caller has counted
-    them (0: the kernel's launch takes a bound); ``n_splits`` > 1 splits each sequence's keys over CTAs and needs
+    prompt portions alike); ``n_splits`` > 1 splits each sequence's keys over CTAs and needs
     ``T * nh * n_splits * (hd + 2)`` floats of scratch (allocated here if not given)."""
     _check(q, "q", torch.bfloat16, 2)
     _check(cache_layer, "cache_layer", torch.bfloat16, 5)
@@ -592,7 +591,7 @@ def paged_attention_mma(q: torch.Tensor, cache_layer: torch.Tensor, block_table:
     lib.call("pyre_paged_attention_mma", q.data_ptr(), cache_layer.data_ptr(), out.data_ptr(), _ptr(scratch),
              block_table.data_ptr(), block_table.stride(0), cu_seqlens.data_ptr(), positions.data_ptr(), T, n_seqs,
              n_heads, n_kv_heads, head_dim, page_size, int(window or 0), int(keep_first), float(scale), _sink_args(sink, n_heads)[0], _sink_args(sink, n_heads)[1], n_splits, int(max_len),
-             cache_layer.shape[0], int(uniform_len), int(n_groups), device_error_flag(q.device).data_ptr(), _stream())
+             cache_layer.shape[0], int(uniform_len), device_error_flag(q.device).data_ptr(), _stream())
     return out
 
 
@@ -694,13 +693,13 @@ def attention_prefill_tc(q: torch.Tensor, cache_layer: torch.Tensor, block_table
 def _attention_plan(ctx, use_tc: bool, min_len: int, n_heads: int, n_kv_heads: int, head_dim: int,
                     window: "int | None", keep_first: int) -> tuple:
     """How a step's attention is cut: (tokens of the long entries, their key splits, short entries, splits, the length
-    all entries share or 0, row groups of the short entries).  From host-side facts of the step and the mixer's sizes alone."""
+    the short entries' kernel may take for granted or 0, tokens of the short entries if they come first, else 0).  From host-side facts of the step and the mixer's sizes alone."""
     lens = ctx.cu_seqlens_host[1:] - ctx.cu_seqlens_host[:-1]
     long_mask = lens >= min_len if head_dim in PREFILL_HEAD_DIMS else lens < 0
     n_long = int(lens[long_mask].sum())
     n_short_seqs = int((~long_mask).sum())
     key_splits = splits = 1
-    uniform = groups = 0
+    uniform = head = 0
     if n_long and use_tc:
         long_lens, long_starts = lens[long_mask], ctx.start_pos_host[long_mask]
         q_tiles = -(-long_lens // 128)
@@ -716,8 +715,11 @@ def _attention_plan(ctx, use_tc: bool, min_len: int, n_heads: int, n_kv_heads: i
         tpg = max(1, 16 // min(n_heads // n_kv_heads, 16))
         groups = int((-(-lens[~long_mask] // tpg)).sum())
         splits = attention_splits(ctx.num_tokens - n_long, n_short_seqs, n_heads, n_kv_heads, short_ctx, window and window + keep_first, groups)
-        uniform = int(lens[0]) if not n_long and bool((lens == lens[0]).all()) else 0
-    return n_long, key_splits, n_short_seqs, splits, uniform, groups
+        if n_long and not long_mask[:n_short_seqs].any():
+            head = int(ctx.cu_seqlens_host[n_short_seqs])
+        taken = lens[:n_short_seqs]
+        uniform = int(lens[0]) if (head or not n_long) and bool((taken == lens[0]).all()) else 0
+    return n_long, key_splits, n_short_seqs, splits, uniform, head
 
 
 def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_table: torch.Tensor, n_heads: int,
@@ -733,7 +735,7 @@ def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_
     plan = ctx.scratch.get(key)
     if plan is None:
         plan = ctx.scratch[key] = _attention_plan(ctx, use_tc, min_len, n_heads, n_kv_heads, head_dim, window, keep_first)
-    n_long, key_splits, n_short_seqs, splits, uniform, groups = plan
+    n_long, key_splits, n_short_seqs, splits, uniform, head = plan
     out = torch.empty_like(q)
     if n_long and use_tc:
         attention_prefill_tc(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_long, n_heads,
@@ -741,12 +743,17 @@ def paged_attention_bf16(ctx, q: torch.Tensor, cache_layer: torch.Tensor, block_
     elif n_long:
         attention_prefill(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_long, n_heads,
                           n_kv_heads, head_dim, scale, window, out, sink=sink, keep_first=keep_first)
-    if n_short_seqs:
-        # beside a portion the groups are counted; a step of decoded tokens alone keeps the bound, whose few spare CTAs cost
-        # nothing (eight requests of the 7B shape: 501 us a step so, 504 counted)
+    if n_short_seqs and head:
+        # The scheduler puts decoded tokens first: their kernel gets that head of the batch alone.  Its grid is bounded by the tokens
+        # it is given, and a portion of 1,024 tokens behind 16 decoded ones made it 5,800 CTAs for 256 with work (40 heads, up
+        # to 8,000 keys: 120 -> 76 us).
+        paged_attention_mma(q[:head], cache_layer, block_table[:n_short_seqs], ctx.cu_seqlens[:n_short_seqs + 1], ctx.positions[:head],
+                            n_short_seqs, n_heads, n_kv_heads, head_dim, scale, window, splits, out=out[:head], uniform_len=uniform,
+                            sink=sink, keep_first=keep_first)
+    elif n_short_seqs:
         paged_attention_mma(q, cache_layer, block_table, ctx.cu_seqlens, ctx.positions, ctx.num_seqs, n_heads,
                             n_kv_heads, head_dim, scale, window, splits, out=out,
-                            max_len=min_len - 1 if n_long else 0, uniform_len=uniform, sink=sink, keep_first=keep_first, n_groups=groups if n_long else 0)
+                            max_len=min_len - 1 if n_long else 0, uniform_len=uniform, sink=sink, keep_first=keep_first)
     return out
 
 
