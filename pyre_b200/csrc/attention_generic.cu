@@ -77,8 +77,8 @@ __global__ void __launch_bounds__(AG_WARPS * 32, DEEP ? 1 : 2) paged_attention_g
         const bool live = r < rows && r % hpg < heads;
         const int pos = live ? positions[row_token(r)] : -1;
         row_seq[r] = r < rows ? seq_of_token[row_token(r)] : -1;
-        row_pos[r] = pos;                                                      // -1: a row that sees nothing and is not stored
-        row_lo[r] = (window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
+        row_pos[r] = pos;                                                      // negative: sees no key
+        row_lo[r] = !live ? -1 : (pos >= 0 && window > 0 && pos - window + 1 > 0) ? pos - window + 1 : 0;
     }
     for (int e = threadIdx.x; e < R * hd; e += AG_WARPS * 32) {
         const int r = e / hd, d = e - r * hd;
@@ -105,6 +105,10 @@ __global__ void __launch_bounds__(AG_WARPS * 32, DEEP ? 1 : 2) paged_attention_g
         for (; r1 < rows && row_seq[r1] == seq; ++r1) {
             pos = max(pos, row_pos[r1]);
             if (row_pos[r1] >= 0) lo = min(lo, row_lo[r1]);
+        }
+        if (pos < 0) {      // no row of this piece sees a key
+            r0 = r1;
+            continue;
         }
         const int* table = block_table + (size_t)seq * bt_stride;
         const int lo_chunk = (lo / 32) * 32;
@@ -148,7 +152,7 @@ __global__ void __launch_bounds__(AG_WARPS * 32, DEEP ? 1 : 2) paged_attention_g
             if (alike && tpg > 1) {
 #pragma unroll
                 for (int r = 0; r < R; ++r)
-                    alike = alike && (row_pos[r] < 0 || (c + 31 <= row_pos[r] && (c >= row_lo[r] || c + 32 <= keep)));
+                    alike = alike && (row_lo[r] < 0 || (c + 31 <= row_pos[r] && (c >= row_lo[r] || c + 32 <= keep)));
             }
             float alpha[R];
             __syncwarp();      // every lane has read the probabilities of the chunk before
@@ -235,14 +239,14 @@ __global__ void __launch_bounds__(AG_WARPS * 32, DEEP ? 1 : 2) paged_attention_g
     __syncthreads();
     for (int e = threadIdx.x; e < R * hd; e += AG_WARPS * 32) {
         const int r = e / hd;
-        if (row_pos[r] < 0) continue;
+        if (row_lo[r] < 0) continue;      // a row that is not there
         float top = m_s[0][r];
 #pragma unroll
         for (int w = 1; w < AG_WARPS; ++w) top = fmaxf(top, m_s[w][r]);
         float sum = 0.f, den = 0.f;
 #pragma unroll
         for (int w = 0; w < AG_WARPS; ++w) {
-            const float f = expf(m_s[w][r] - top);      // a warp without a chunk: exp(-inf) = 0
+            const float f = m_s[w][r] == -INFINITY ? 0.f : expf(m_s[w][r] - top);      // a warp without a chunk: nothing
             sum = fmaf(merged[w * R * hd + e], f, sum);
             den = fmaf(l_s[w][r], f, den);
         }

@@ -103,3 +103,28 @@ def test_attention_however_rows_share_a_cta(ops, dtype, nh, nkv, hd, page, windo
         later[int(table[s, j // page]), 1, :, j % page] = float("inf")
     got = ops.paged_attention_generic(q, later, table, seq, pos, nh, nkv, hd, scale, window, sink=sink, keep_first=keep)
     assert torch.equal(got[150:150 + p + 1], whole[150:150 + p + 1])
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(2, 2, 32), (6, 2, 64), (7, 1, 16)])
+@pytest.mark.parametrize("window,keep", [(None, 0), (40, 5)])
+def test_attention_of_tokens_without_a_position(ops, nh, nkv, hd, window, keep):
+    """A token at a negative position sees no key: nothing is read for it, with a sink its result is zero (the sink takes all of the
+    weight), and the tokens that share its CTA have the bits that they have without it."""
+    g = torch.Generator(device="cuda").manual_seed(nh)
+    T, page = 300, 16
+    table = torch.arange(-(-T // page), dtype=torch.int32, device="cuda").view(1, -1).repeat(2, 1)
+    cache = torch.randn(table.shape[1], 2, nkv, page, hd, device="cuda", generator=g)
+    cache[0, 1, :, 3] = float("inf")                # a value that a row without keys must not touch
+    pos = torch.arange(T, dtype=torch.int32, device="cuda")
+    pos[[0, 5, 6, 40]] = torch.tensor([-1, -1, -7, -2147483648], dtype=torch.int32, device="cuda")
+    pos[64:96] = -1                                 # whole CTAs of them
+    seq = (torch.arange(T, device="cuda") >= 200).to(torch.int32)
+    q, sink = torch.randn(T, nh * hd, device="cuda", generator=g), torch.randn(nh, device="cuda", generator=g)
+
+    def run(rows):
+        return ops.paged_attention_generic(q[rows].contiguous(), cache, table, seq[rows], pos[rows], nh, nkv, hd, hd ** -0.5, window, sink=sink, keep_first=keep)
+    got, none = run(slice(0, T)), pos < 0
+    assert torch.equal(got[none], torch.zeros_like(got[none]))
+    keep_rows = (~none).nonzero()[:, 0]
+    # bytes, since the infinite value makes some results infinite or not a number
+    assert torch.equal(got[keep_rows].view(torch.int32), run(keep_rows).view(torch.int32))
