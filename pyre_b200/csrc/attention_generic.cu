@@ -165,8 +165,9 @@ __global__ void __launch_bounds__(AG_WARPS * 32, DEEP ? 1 : 2) paged_attention_g
                     const bool valid = (j >= rl || j < keep) && j <= rp;
                     const float score = valid ? ((lo2(dot[r][0]) + hi2(dot[r][0])) + (lo2(dot[r][1]) + hi2(dot[r][1]))) * scale : -INFINITY;
                     const float m_new = fmaxf(m[r], warp_max(score));
-                    const float e = valid ? expf(score - m_new) : 0.f;
-                    alpha[r] = expf(m[r] - m_new);      // m = -inf at the start: exp(-inf) = 0
+                    const float ref = m_new == -INFINITY ? 0.f : m_new;      // no score above minus infinity so far: every term is zero
+                    const float e = valid ? expf(score - ref) : 0.f;
+                    alpha[r] = expf(m[r] - ref);      // m = -inf at the start: exp(-inf) = 0
                     l[r] = l[r] * alpha[r] + warp_sum(e);
                     m[r] = m_new;
                     if (valid) p = e;

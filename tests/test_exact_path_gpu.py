@@ -128,3 +128,28 @@ def test_attention_of_tokens_without_a_position(ops, nh, nkv, hd, window, keep):
     keep_rows = (~none).nonzero()[:, 0]
     # bytes, since the infinite value makes some results infinite or not a number
     assert torch.equal(got[keep_rows].view(torch.int32), run(keep_rows).view(torch.int32))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(2, 2, 32), (4, 1, 144), (7, 1, 16)])
+@pytest.mark.parametrize("low", [[32], [33, 34, 35], list(range(64, 96)), list(range(32)), list(range(96, 101)), list(range(40))])
+def test_attention_with_scores_of_minus_infinity(ops, dtype, nh, nkv, hd, low):
+    """Keys whose score overflows to minus infinity have no weight, also where they are all that a chunk of 32 keys holds; without any
+    other key a row is not a number, or zero where a sink takes all of the weight."""
+    g = torch.Generator(device="cuda").manual_seed(hd + len(low))
+    page, T = 16, 101
+    table = torch.randperm(-(-T // page), generator=torch.Generator().manual_seed(1)).to(torch.int32).cuda()[None]
+    cache = torch.randn(table.shape[1], 2, nkv, page, hd, device="cuda", generator=g).to(dtype)
+    cache[:, 0, :, :, 0] = 0
+    for j in low:
+        cache[int(table[0, j // page]), 0, :, j % page, 0] = -1e30
+    q = torch.randn(T, nh * hd, device="cuda", generator=g).to(dtype)
+    q[:, ::hd] = 1e30
+    pos, seq = torch.arange(T, dtype=torch.int32, device="cuda"), torch.zeros(T, dtype=torch.int32, device="cuda")
+    none = torch.tensor([all(j in low for j in range(p + 1)) for p in range(T)], device="cuda")
+    for sink in (torch.full((nh,), float("-inf"), device="cuda"), torch.zeros(nh, device="cuda")):
+        got = ops.paged_attention_generic(q, cache, table, seq, pos, nh, nkv, hd, hd ** -0.5, sink=sink)
+        assert torch.isnan(got[none]).all() if sink[0] < 0 else (got[none] == 0).all()
+        want = reference(q, cache, table, seq, pos, nh, nkv, hd, hd ** -0.5, None, 0, sink)
+        err = (got.double() - want).abs()[~none]
+        assert (err <= (2e-6 if dtype == torch.float32 else 2.0 ** -8 * want.abs()[~none] + 1e-5)).all(), float(err.max())
