@@ -471,7 +471,7 @@ def paged_attention_generic(q: torch.Tensor, cache_layer: torch.Tensor, block_ta
     lib.call("pyre_paged_attention_generic", q.data_ptr(), cache_layer.data_ptr(), out.data_ptr(),
              block_table.data_ptr(), block_table.stride(0), seq_of_token.data_ptr(), positions.data_ptr(), T,
              n_heads, n_kv_heads, head_dim, page_size, int(window or 0), int(keep_first), float(scale), _sink_args(sink, n_heads)[0], _sink_args(sink, n_heads)[1], _dt(q.dtype), cache_layer.shape[0],
-             device_error_flag(q.device).data_ptr(), block_table.shape[0], _stream())
+             device_error_flag(q.device).data_ptr(), block_table.shape[0], max(block_table.shape[1], block_table.stride(0)), _stream())
     return out
 
 

@@ -153,3 +153,33 @@ def test_attention_with_scores_of_minus_infinity(ops, dtype, nh, nkv, hd, low):
         want = reference(q, cache, table, seq, pos, nh, nkv, hd, hd ** -0.5, None, 0, sink)
         err = (got.double() - want).abs()[~none]
         assert (err <= (2e-6 if dtype == torch.float32 else 2.0 ** -8 * want.abs()[~none] + 1e-5)).all(), float(err.max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nh,nkv,hd", [(2, 2, 16), (6, 2, 48), (7, 1, 128), (5, 5, 128), (3, 1, 144), (8, 4, 256)])
+@pytest.mark.parametrize("most", [16, 32, 33, 64, 65, 128, 129, 256])
+@pytest.mark.parametrize("tokens", ["decoded", "few", "many"])
+def test_attention_of_short_tables(ops, dtype, nh, nkv, hd, most, tokens):
+    """A table that holds one to eight chunks of keys lets fewer warps share a row; one token, or hundreds of short sequences: the bits are
+    those that a wide table gives, and near an evaluation in 64 bits."""
+    g = torch.Generator(device="cuda").manual_seed(nh + hd + most)
+    page, n_seqs = 16, 1 if tokens == "decoded" else 3 if tokens == "few" else 300
+    width = -(-most // page)
+    table = torch.randint(0, 40, (n_seqs, width), generator=torch.Generator().manual_seed(most)).to(torch.int32).cuda()
+    wide = torch.cat([table, torch.full((n_seqs, 30), -1, dtype=torch.int32, device="cuda")], 1)
+    cache = torch.randn(40, 2, nkv, page, hd, device="cuda", generator=g).to(dtype)
+    seq = torch.arange(n_seqs, dtype=torch.int32, device="cuda")
+    pos = torch.randint(0, most, (n_seqs,), device="cuda", generator=g).to(torch.int32)
+    pos[0] = most - 1
+    if tokens == "few":      # a portion beside decoded tokens
+        seq = torch.cat([seq, torch.full((min(most, 50),), 2, dtype=torch.int32, device="cuda")])
+        pos = torch.cat([pos, torch.arange(min(most, 50), dtype=torch.int32, device="cuda")])
+    q = torch.randn(len(seq), nh * hd, device="cuda", generator=g).to(dtype)
+    sink = torch.randn(nh, device="cuda", generator=g)
+    for window, keep in ((None, 0), (20, 3)):
+        got = ops.paged_attention_generic(q, cache, table, seq, pos, nh, nkv, hd, hd ** -0.5, window, sink=sink, keep_first=keep)
+        assert torch.equal(got, ops.paged_attention_generic(q, cache, wide, seq, pos, nh, nkv, hd, hd ** -0.5, window, sink=sink, keep_first=keep))
+        some = slice(0, 60)
+        want = reference(q[some], cache, table, seq[some], pos[some], nh, nkv, hd, hd ** -0.5, window, keep, sink)
+        err = (got[some].double() - want).abs()
+        assert (err <= (2e-6 if dtype == torch.float32 else 2.0 ** -8 * want.abs() + 1e-5)).all(), float(err.max())
