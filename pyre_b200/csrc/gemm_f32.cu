@@ -11,11 +11,13 @@
 // or tile shape computes it: a row's result is bit-identical for any M and any batch composition.  The chains are
 // what the kernels divide among threads (few rows) or CTAs (few tiles) without changing a bit.
 //
-// Three kernels, the same arithmetic in each:
-//   * many rows, rows of both operands 16-byte aligned and K a multiple of 4: 64 x 64 tiles, one CTA per tile or a
-//     cluster of eight, one per chain;
-//   * up to 32 rows (decode), same alignment: a weight stream, 16 output features per CTA, the chains in different threads;
-//   * anything else: the plain tile kernel with scalar loads.
+// Two kernels, the same arithmetic in each:
+//   * many rows: 64 x 64 tiles, one CTA per tile or a cluster of eight, one per chain;
+//   * up to 32 rows (decode): a weight stream, 16 output features per CTA, the chains in different threads.
+// Both bring their operands to shared memory by cp.async, 16 bytes at a time (VEC) where the rows of both operands are 16-byte
+// aligned and K is a multiple of 4, else 4 bytes at a time.  Measured with rows of 3,585 floats (M x N; a plain tile kernel
+// with scalar loads through registers, 128 x 128 or 64 x 128 outputs / 4-byte copies): 4 x 18944: 631 and 1417 / 87 us, 32 x 18944: 716
+// and 1494 / 253 us, 509 x 18944: 8598 and 13395 / 2294 us; with rows of a multiple of four: 3385 us for 509 x 37888 x 3584.
 #include "common.cuh"
 
 namespace {
@@ -35,90 +37,13 @@ __device__ __forceinline__ void copy16(float* dst, const float* src, bool live) 
     const int bytes = live ? 16 : 0;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
-}  // namespace
-
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN))
-sgemm_nt_kernel(const float* A, long long lda, const float* W, long long ldw,
-                float* C, long long ldc, const float* bias, int M, int N, int K) {
-    constexpr int THREADS = (BM / TM) * (BN / TN), BK = 8;
-    static_assert(RUN % BK == 0 && BK % 2 == 0, "a run ends at a tile's end, a tile holds whole even-odd pairs");
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Ws[BK][BN + 4];
-    pdl_trigger();
-    pdl_wait();
-    const int tid = threadIdx.x;
-    const int tx = tid % (BN / TN);  // column group
-    const int ty = tid / (BN / TN);  // row group
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const int n_runs = (K + RUN - 1) / RUN;
-
-    float total[TM][TN];
-#pragma unroll
-    for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) total[i][j] = 0.f;
-
-    for (int c = 0; c < CHAINS && c < n_runs; ++c) {
-        float acc[TM][TN];
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
-        for (int run = c; run < n_runs; run += CHAINS) {
-            float part[2][TM][TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) part[0][i][j] = part[1][i][j] = 0.f;
-            for (int k0 = run * RUN; k0 < run * RUN + RUN; k0 += BK) {
-                // tile loads: consecutive threads read consecutive k of one row
-                for (int e = tid; e < BM * BK; e += THREADS) {
-                    const int r = e / BK, kk = e % BK;
-                    const int gm = m0 + r, gk = k0 + kk;
-                    As[kk][r] = (gm < M && gk < K) ? A[(size_t)gm * lda + gk] : 0.f;
-                }
-                for (int e = tid; e < BN * BK; e += THREADS) {
-                    const int r = e / BK, kk = e % BK;
-                    const int gn = n0 + r, gk = k0 + kk;
-                    Ws[kk][r] = (gn < N && gk < K) ? W[(size_t)gn * ldw + gk] : 0.f;
-                }
-                __syncthreads();
-#pragma unroll
-                for (int kk = 0; kk < BK; ++kk) {
-                    float a[TM], w[TN];
-#pragma unroll
-                    for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
-#pragma unroll
-                    for (int j = 0; j < TN; ++j) w[j] = Ws[kk][tx * TN + j];
-#pragma unroll
-                    for (int i = 0; i < TM; ++i)
-#pragma unroll
-                        for (int j = 0; j < TN; ++j) part[kk & 1][i][j] = fmaf(a[i], w[j], part[kk & 1][i][j]);
-                }
-                __syncthreads();
-            }
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] += part[0][i][j] + part[1][i][j];
-        }
-#pragma unroll
-        for (int i = 0; i < TM; ++i)
-#pragma unroll
-            for (int j = 0; j < TN; ++j) total[i][j] += acc[i][j];
-    }
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        const int gm = m0 + ty * TM + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            const int gn = n0 + tx * TN + j;
-            if (gn < N) C[(size_t)gm * ldc + gn] = bias ? total[i][j] + bias[gn] : total[i][j];
-        }
-    }
+// a 4-byte copy, or 4 bytes of zeros
+__device__ __forceinline__ void copy4(float* dst, const float* src, bool live) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int bytes = live ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
 }
+}  // namespace
 
 // ---------------------------------------------------------------------------
 // Many rows.  Bound by the FMA pipe: fma.rn.f32x2 alone, out of registers, reaches 49 TFLOP/s on this chip; a thread owns 8 x 4
@@ -134,7 +59,7 @@ sgemm_nt_kernel(const float* A, long long lda, const float* W, long long ldw,
 // ---------------------------------------------------------------------------
 constexpr int TILE = 64, TILE_STAGES = 3;
 
-template <int PARTS>
+template <int PARTS, bool VEC>
 __global__ void __launch_bounds__(128, 3)
 sgemm_nt_tiles_kernel(const float* A, long long lda, const float* W, long long ldw,
                       float* C, long long ldc, const float* bias, int M, int N, int K, int tiles_m) {
@@ -148,24 +73,29 @@ sgemm_nt_tiles_kernel(const float* A, long long lda, const float* W, long long l
     // the tiles of one block of weight rows follow one another: their weights come out of the L2 cache
     const int m0 = (tile % tiles_m) * BM, n0 = (tile / tiles_m) * BN;
     const int n_runs = (K + RUN - 1) / RUN;
-    // copies: per step 128 rows of 4 quads; a thread fetches quad lq of the rows lr, lr + 32 of both operands
-    const int lr = tid >> 2, lq = tid & 3;
+    // copies: per step 128 rows of 16 k; a thread fetches pieces of P floats, piece lq of the rows lr, lr + STEP, ... of both operands
+    constexpr int P = VEC ? 4 : 1, PIECES = BK / P, STEP = 128 / PIECES;
+    const int lr = tid / PIECES, lq = tid % PIECES;
     int f_chain = rank, f_run = rank, f_half = 0, f_stage = 0;      // where the next fetch stands
+    auto copy = [](float* dst, const float* src, bool live) {
+        if constexpr (VEC) copy16(dst, src, live);
+        else copy4(dst, src, live);
+    };
     auto fetch = [&]() {
         if (f_run < n_runs) {
-            const int gk = f_run * RUN + f_half * BK + 4 * lq;
+            const int gk = f_run * RUN + f_half * BK + P * lq;
             const bool in_k = gk < K;
-            float* dst = tiles + f_stage * STAGE + lr * PITCH + 4 * lq;
+            float* dst = tiles + f_stage * STAGE + lr * PITCH + P * lq;
             // rows outside the matrices are not stored: whatever their sums are
 #pragma unroll
-            for (int h = 0; h < BM / 32; ++h) {
-                const int gm = m0 + lr + 32 * h;
-                if (gm < M) copy16(dst + 32 * h * PITCH, in_k ? A + (size_t)gm * lda + gk : A, in_k);
+            for (int h = 0; h < BM; h += STEP) {
+                const int gm = m0 + lr + h;
+                if (gm < M) copy(dst + h * PITCH, in_k ? A + (size_t)gm * lda + gk : A, in_k);
             }
 #pragma unroll
-            for (int h = 0; h < BN / 32; ++h) {
-                const int gn = n0 + lr + 32 * h;
-                if (gn < N) copy16(dst + (BM + 32 * h) * PITCH, in_k ? W + (size_t)gn * ldw + gk : W, in_k);
+            for (int h = 0; h < BN; h += STEP) {
+                const int gn = n0 + lr + h;
+                if (gn < N) copy(dst + (BM + h) * PITCH, in_k ? W + (size_t)gn * ldw + gk : W, in_k);
             }
             f_half ^= 1;
             if (f_half == 0) {
@@ -289,37 +219,54 @@ sgemm_nt_tiles_kernel(const float* A, long long lda, const float* W, long long l
 // read at): 4 x 37888 x 3584: 226 -> 119 us (4.6 TB/s); 4 x 3584 x 18944: 185 -> 70 us (3.9 TB/s); 8 x 3584 x 18944: 184 -> 97 us;
 // 12 x 3584 x 18944: 723 -> 138 us; 32 x 3584 x 18944: 441 -> 213 us (a stage was one run of 32 k, a CTA's threads all walked it).
 // ---------------------------------------------------------------------------
-template <int MR, int F, int GROUPS, int STAGES>
+template <int MR, int F, int GROUPS, int STAGES, bool VEC>
 __global__ void __launch_bounds__(CHAINS * 16 / F * GROUPS)
 sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long ldw,
                        float* C, long long ldc, const float* bias, int M, int N, int K) {
     constexpr int FN = 16, FT = FN / F, MT = MR * GROUPS, THREADS = CHAINS * FT * GROUPS;
     constexpr int RUN_PITCH = RUN + 4, ROW = CHAINS * RUN_PITCH + 4, KS = RUN * CHAINS;
     constexpr int STAGE = (FN + MT) * ROW, STEP = THREADS / 64;
-    static_assert(CHAINS * MT * FN <= STAGE * STAGES && THREADS % 64 == 0 && FN % STEP == 0, "copies and the last sum fit");
+    static_assert(CHAINS * MT * FN <= STAGE * STAGES && THREADS % 64 == 0 && FN % STEP == 0 && KS % THREADS == 0, "copies and the last sum fit");
     extern __shared__ __align__(16) float ring[];
     pdl_trigger();
     const int tid = threadIdx.x;
     const int ft = tid % FT, chain = tid / FT % CHAINS, group = tid / (FT * CHAINS);
     const int n0 = blockIdx.x * FN;
     const int n_steps = (K + KS - 1) / KS;
-    // copies: a thread fetches quad cq of the rows cr, cr + STEP, ...
+    // copies: VEC: a thread fetches quad cq of the rows cr, cr + STEP, ...; else a warp 32 neighbouring floats of a row
     const int cq = tid & 63, cr = tid >> 6;
     float* const to = ring + (cq >> 3) * RUN_PITCH + (cq & 7) * 4;
+    // row r of `live` ones, on row `at` of the stage; rows outside the matrices are not stored: whatever their sums are
+    auto load_scalars = [&](const float* from, long long ld, int rows, int live, int at, int t, int st) {
+#pragma unroll 1
+        for (int r = 0; r < min(rows, live); ++r) {
+            float* dst = ring + st * STAGE + (at + r) * ROW;
+            const float* src = from + (size_t)r * ld;
+#pragma unroll
+            for (int k = tid; k < KS; k += THREADS) {
+                const int gk = t * KS + k;
+                copy4(dst + (k / RUN) * RUN_PITCH + k % RUN, gk < K ? src + gk : src, gk < K);
+            }
+        }
+    };
     auto load_w = [&](int t, int st) {
         const int gk = t * KS + 4 * cq;
         const bool live = gk < K;
         if (t >= n_steps) return;
+        if constexpr (VEC) {
 #pragma unroll
-        for (int r = cr; r < FN; r += STEP)      // rows outside the matrices are not stored: whatever their sums are
-            if (n0 + r < N) copy16(to + st * STAGE + r * ROW, live ? W + (size_t)(n0 + r) * ldw + gk : W, live);
+            for (int r = cr; r < FN; r += STEP)
+                if (n0 + r < N) copy16(to + st * STAGE + r * ROW, live ? W + (size_t)(n0 + r) * ldw + gk : W, live);
+        } else load_scalars(W + (size_t)n0 * ldw, ldw, FN, N - n0, 0, t, st);
     };
     auto load_a = [&](int t, int st) {
         const int gk = t * KS + 4 * cq;
         const bool live = gk < K;
         if (t >= n_steps) return;
-        for (int r = cr; r < MT; r += STEP)
-            if (r < M) copy16(to + st * STAGE + (FN + r) * ROW, live ? A + (size_t)r * lda + gk : A, live);
+        if constexpr (VEC) {
+            for (int r = cr; r < MT; r += STEP)
+                if (r < M) copy16(to + st * STAGE + (FN + r) * ROW, live ? A + (size_t)r * lda + gk : A, live);
+        } else load_scalars(A, lda, MT, M, FN, t, st);
     };
     // the weights depend on no earlier kernel: their first stages are on their way before the wait
     for (int s = 0; s < STAGES - 1; ++s) load_w(s, s);
@@ -387,14 +334,14 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
     }
 }
 
-template <int MR, int F, int GROUPS, int STAGES>
+template <int MR, int F, int GROUPS, int STAGES, bool VEC>
 static int launch_stream(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
                          const float* bias, int M, int N, int K, cudaStream_t stream) {
     constexpr int BYTES = STAGES * (16 + MR * GROUPS) * (CHAINS * (RUN + 4) + 4) * 4;
     static_assert(BYTES <= 232448, "the ring does not fit into shared memory");
     static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attribute is per device
     bool& configured = configured_on[pyre_current_device()];
-    auto kernel = sgemm_nt_stream_kernel<MR, F, GROUPS, STAGES>;
+    auto kernel = sgemm_nt_stream_kernel<MR, F, GROUPS, STAGES, VEC>;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
         if (e != cudaSuccess) return (int)e;
@@ -404,13 +351,13 @@ static int launch_stream(const float* A, long long lda, const float* W, long lon
                             A, lda, W, ldw, C, ldc, bias, M, N, K);
 }
 
-template <int PARTS>
+template <int PARTS, bool VEC>
 static int launch_tiles_as(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
                            const float* bias, int M, int N, int K, cudaStream_t stream) {
     constexpr int BYTES = (TILE_STAGES * 2 * TILE * 20 + TILE * TILE) * 4;
     static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attribute is per device
     bool& configured = configured_on[pyre_current_device()];
-    auto kernel = sgemm_nt_tiles_kernel<PARTS>;
+    auto kernel = sgemm_nt_tiles_kernel<PARTS, VEC>;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
         if (e != cudaSuccess) return (int)e;
@@ -434,6 +381,7 @@ static int launch_tiles_as(const float* A, long long lda, const float* W, long l
     return (int)cudaLaunchKernelEx(&cfg, kernel, A, lda, W, ldw, C, ldc, bias, M, N, K, tiles_m);
 }
 
+template <bool VEC>
 static int launch_tiles(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
                         const float* bias, int M, int N, int K, cudaStream_t stream) {
     const long long tiles = (long long)ceil_div(M, TILE) * ceil_div(N, TILE);
@@ -442,26 +390,28 @@ static int launch_tiles(const float* A, long long lda, const float* W, long long
     // a chain is long enough (four runs) to pay for the cluster's meeting
     const long long busiest = (tiles + sms - 1) / sms;
     if (K >= 4 * RUN * CHAINS && busiest * sms * 10 > tiles * 11)
-        return launch_tiles_as<CHAINS>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
-    return launch_tiles_as<1>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+        return launch_tiles_as<CHAINS, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    return launch_tiles_as<1, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+}
+
+template <bool VEC>
+static int launch_product(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
+                          const float* bias, int M, int N, int K, cudaStream_t stream) {
+    if (M <= 4) return launch_stream<4, 1, 1, 4, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    if (M <= 8) return launch_stream<8, 1, 1, 4, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    if (M <= 16) return launch_stream<8, 2, 2, 3, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    if (M <= 32) return launch_stream<8, 2, 4, 2, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    return launch_tiles<VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
 }
 
 PYRE_API int pyre_sgemm_nt(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
                            const float* bias, int M, int N, int K, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K < 0) return PYRE_ERR_BAD_ARG;
-    // float4 loads and 16-byte copies need aligned rows in both operands
+    // 16-byte copies need aligned rows in both operands
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && !((uintptr_t)A & 15) && !((uintptr_t)W & 15);
-    int rc = 0;
-    if (vec && M <= 4) rc = launch_stream<4, 1, 1, 4>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
-    else if (vec && M <= 8) rc = launch_stream<8, 1, 1, 4>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
-    else if (vec && M <= 16) rc = launch_stream<8, 2, 2, 3>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
-    else if (vec && M <= 32) rc = launch_stream<8, 2, 4, 2>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
-    else if (vec) rc = launch_tiles(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
-    else if (M > 32) rc = (int)pyre_launch(sgemm_nt_kernel<64, 128, 4, 8>, dim3(ceil_div(N, 128), ceil_div(M, 64)), dim3(256), 0, stream,
-                                           A, lda, W, ldw, C, ldc, bias, M, N, K);
-    else rc = (int)pyre_launch(sgemm_nt_kernel<32, 128, 2, 8>, dim3(ceil_div(N, 128), ceil_div(M, 32)), dim3(256), 0, stream,
-                               A, lda, W, ldw, C, ldc, bias, M, N, K);
+    const int rc = vec ? launch_product<true>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream)
+                       : launch_product<false>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
     if (rc) return rc;
     PYRE_LAUNCH_CHECK();
     return 0;

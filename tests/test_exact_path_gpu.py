@@ -183,3 +183,14 @@ def test_attention_of_short_tables(ops, dtype, nh, nkv, hd, most, tokens):
         want = reference(q[some], cache, table, seq[some], pos[some], nh, nkv, hd, hd ** -0.5, window, keep, sink)
         err = (got[some].double() - want).abs()
         assert (err <= (2e-6 if dtype == torch.float32 else 2.0 ** -8 * want.abs() + 1e-5)).all(), float(err.max())
+
+
+@pytest.mark.parametrize("K", [3, 4])
+def test_product_of_very_many_rows(ops, K):
+    """More tiles of rows than the second dimension of a grid holds, from rows on and off 16-byte boundaries."""
+    M, N = 64 * 65535 + 70, 3
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, w = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    got = ops.sgemm_nt(a, w)
+    want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
+    assert ((got.double() - want).abs() <= 4 * EPS * size).all()      # two additions of each of two chains, one of the chains
