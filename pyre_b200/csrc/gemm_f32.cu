@@ -219,10 +219,12 @@ sgemm_nt_tiles_kernel(const float* A, long long lda, const float* W, long long l
 // read at): 4 x 37888 x 3584: 226 -> 119 us (4.6 TB/s); 4 x 3584 x 18944: 185 -> 70 us (3.9 TB/s); 8 x 3584 x 18944: 184 -> 97 us;
 // 12 x 3584 x 18944: 723 -> 138 us; 32 x 3584 x 18944: 441 -> 213 us (a stage was one run of 32 k, a CTA's threads all walked it).
 // ---------------------------------------------------------------------------
-template <int MR, int F, int GROUPS, int STAGES, bool VEC>
+// SHORT: K fits into one stage.  A CTA then takes one of `row_tiles` tiles of MT rows (their weights are read once more from the L2
+// cache, which is less than what a CTA loses on rows it walks one after another), and runs past K are neither copied nor multiplied.
+template <int MR, int F, int GROUPS, int STAGES, bool VEC, bool SHORT>
 __global__ void __launch_bounds__(CHAINS * 16 / F * GROUPS)
 sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long ldw,
-                       float* C, long long ldc, const float* bias, int M, int N, int K) {
+                       float* C, long long ldc, const float* bias, int M, int N, int K, int row_tiles) {
     constexpr int FN = 16, FT = FN / F, MT = MR * GROUPS, THREADS = CHAINS * FT * GROUPS;
     constexpr int RUN_PITCH = RUN + 4, ROW = CHAINS * RUN_PITCH + 4, KS = RUN * CHAINS;
     constexpr int STAGE = (FN + MT) * ROW, STEP = THREADS / 64;
@@ -231,7 +233,13 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
     pdl_trigger();
     const int tid = threadIdx.x;
     const int ft = tid % FT, chain = tid / FT % CHAINS, group = tid / (FT * CHAINS);
-    const int n0 = blockIdx.x * FN;
+    const int n0 = (SHORT ? blockIdx.x / row_tiles : blockIdx.x) * FN;
+    if (SHORT) {
+        const int m0 = blockIdx.x % row_tiles * MT;
+        A += (size_t)m0 * lda;
+        C += (size_t)m0 * ldc;
+        M -= m0;
+    }
     const int n_steps = (K + KS - 1) / KS;
     // copies: VEC: a thread fetches quad cq of the rows cr, cr + STEP, ...; else a warp 32 neighbouring floats of a row
     const int cq = tid & 63, cr = tid >> 6;
@@ -245,6 +253,7 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
 #pragma unroll
             for (int k = tid; k < KS; k += THREADS) {
                 const int gk = t * KS + k;
+                if (SHORT && gk - k % RUN >= K) continue;      // a run past the end
                 copy4(dst + (k / RUN) * RUN_PITCH + k % RUN, gk < K ? src + gk : src, gk < K);
             }
         }
@@ -254,6 +263,7 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
         const bool live = gk < K;
         if (t >= n_steps) return;
         if constexpr (VEC) {
+            if (SHORT && gk - 4 * (cq & 7) >= K) return;      // a run past the end
 #pragma unroll
             for (int r = cr; r < FN; r += STEP)
                 if (n0 + r < N) copy16(to + st * STAGE + r * ROW, live ? W + (size_t)(n0 + r) * ldw + gk : W, live);
@@ -264,6 +274,7 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
         const bool live = gk < K;
         if (t >= n_steps) return;
         if constexpr (VEC) {
+            if (SHORT && gk - 4 * (cq & 7) >= K) return;
             for (int r = cr; r < MT; r += STEP)
                 if (r < M) copy16(to + st * STAGE + (FN + r) * ROW, live ? A + (size_t)r * lda + gk : A, live);
         } else load_scalars(A, lda, MT, M, FN, t, st);
@@ -291,6 +302,7 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
         const float* ws = ring + st * STAGE + ft * ROW + chain * RUN_PITCH;
         const float* as = ring + st * STAGE + (FN + group * MR) * ROW + chain * RUN_PITCH;
         st = st == STAGES - 1 ? 0 : st + 1;
+        if (SHORT && chain * RUN >= K) continue;
         f32x2 part[MR][F];
 #pragma unroll
         for (int i = 0; i < MR; ++i)
@@ -334,21 +346,22 @@ sgemm_nt_stream_kernel(const float* A, long long lda, const float* W, long long 
     }
 }
 
-template <int MR, int F, int GROUPS, int STAGES, bool VEC>
+template <int MR, int F, int GROUPS, int STAGES, bool VEC, bool SHORT = false>
 static int launch_stream(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
                          const float* bias, int M, int N, int K, cudaStream_t stream) {
     constexpr int BYTES = STAGES * (16 + MR * GROUPS) * (CHAINS * (RUN + 4) + 4) * 4;
     static_assert(BYTES <= 232448, "the ring does not fit into shared memory");
     static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attribute is per device
     bool& configured = configured_on[pyre_current_device()];
-    auto kernel = sgemm_nt_stream_kernel<MR, F, GROUPS, STAGES, VEC>;
+    auto kernel = sgemm_nt_stream_kernel<MR, F, GROUPS, STAGES, VEC, SHORT>;
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
         if (e != cudaSuccess) return (int)e;
         configured = true;
     }
-    return (int)pyre_launch(kernel, dim3(ceil_div(N, 16)), dim3(CHAINS * 16 / F * GROUPS), (size_t)BYTES, stream,
-                            A, lda, W, ldw, C, ldc, bias, M, N, K);
+    const int row_tiles = SHORT ? ceil_div(M, MR * GROUPS) : 1;
+    return (int)pyre_launch(kernel, dim3(ceil_div(N, 16) * row_tiles), dim3(CHAINS * 16 / F * GROUPS), (size_t)BYTES, stream,
+                            A, lda, W, ldw, C, ldc, bias, M, N, K, row_tiles);
 }
 
 template <int PARTS, bool VEC>
@@ -397,6 +410,10 @@ static int launch_tiles(const float* A, long long lda, const float* W, long long
 template <bool VEC>
 static int launch_product(const float* A, long long lda, const float* W, long long ldw, float* C, long long ldc,
                           const float* bias, int M, int N, int K, cudaStream_t stream) {
+    // up to a stage's K: tiles of 4 or 8 rows (M x N x K, tiles of 16 or 32 rows and four times the shared memory /
+    // so: 8 x 64 x 64: 1.89 / 1.72 us, 16 x 512 x 64: 2.57 / 1.89, 32 x 512 x 64: 3.26 / 1.89, 32 x 64 x 176: 3.05 / 1.89)
+    if (K <= RUN * CHAINS && M <= 4) return launch_stream<4, 1, 1, 2, VEC, true>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
+    if (K <= RUN * CHAINS && M <= 32) return launch_stream<8, 1, 1, 2, VEC, true>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
     if (M <= 4) return launch_stream<4, 1, 1, 4, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
     if (M <= 8) return launch_stream<8, 1, 1, 4, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
     if (M <= 16) return launch_stream<8, 2, 2, 3, VEC>(A, lda, W, ldw, C, ldc, bias, M, N, K, stream);
