@@ -639,58 +639,64 @@ __global__ void __launch_bounds__(512) latent_attention_mma_kernel(
 }
 
 // out[t, h] = sum_s O_s 2^(m_s - m) / sum_s l_s 2^(m_s - m): the shares of one (token, head); maxima are base-2 exponents.
-// A share that saw no key has left nothing in part_o: what lies there is read (it costs no wait of its own) but not used.  All
-// maxima, sums and the first LM_ONCE shares are asked for at once.
+// A share that saw no key has left nothing in part_o: what lies there is read (it costs no wait of its own) but not used.
+// A warp per (token, head) and 32 V columns, which asks for the first LM_ONCE shares' columns before it knows their weights: a
+// chain of memory latencies where a few tokens are decoded, bound by reading the shares where there are many rows.  With the attention
+// before it, 64 tokens of 64 heads of 256 after 200 rows in two shares: 34.4 us with a block per row whose threads read the maxima and
+// shares one after the other, 41.5 with one that asked for all at once from a single warp, 37 so; four tokens of 16 heads after 700 in eleven: 14.6 and 13.0.
 constexpr int LM_ONCE = 16;
 
+template <int V>
 __global__ void __launch_bounds__(128) latent_combine_kernel(const float* part_o, const float* part_ml, __nv_bfloat16* out, int n_splits, int rank,
-                                      int nh, const float* head_sinks, const __nv_bfloat16* gates, long long gate_stride) {
-    extern __shared__ float weight_s[];      // [n_splits]
+                                      int nh, long long items, int slices, const float* head_sinks, const __nv_bfloat16* gates, long long gate_stride) {
     pdl_trigger();
     pdl_wait();
-    const size_t th = blockIdx.x;
     const int lane = threadIdx.x & 31;
-    const int t = (int)(th / nh), head = (int)(th - (size_t)t * nh);
-    const float* po = part_o + th * n_splits * rank;
-    float part[LM_ONCE];      // this thread's first column
-    const int c0 = min((int)threadIdx.x, rank - 1);
+    const long long item = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (item >= items) return;      // the whole warp
+    const long long th = item / slices;
+    const int c = ((int)(item - th * slices) * 32 + lane) * V;
+    const bool has = c < rank;
+    const float* po = part_o + (size_t)th * n_splits * rank + (has ? c : 0);
+    const float2* ml = reinterpret_cast<const float2*>(part_ml) + (size_t)th * n_splits;
+    Vec<float, V> part[LM_ONCE];
 #pragma unroll
-    for (int s = 0; s < LM_ONCE; ++s) part[s] = s < n_splits ? po[(size_t)s * rank + c0] : 0.f;
-    if (threadIdx.x < 32) {
-        const float2* ml = reinterpret_cast<const float2*>(part_ml) + th * n_splits;
-        float mx = -INFINITY, denom = 0.f;
-        for (int s = lane; s < n_splits; s += 32) mx = fmaxf(mx, ml[s].x);
-        mx = warp_max(mx);
-        for (int s = lane; s < n_splits; s += 32) {
-            const float2 v = ml[s];
-            const float w = exp2f(v.x - mx);
-            if (v.x != -INFINITY) denom = fmaf(v.y, w, denom);
-            weight_s[s] = v.x == -INFINITY ? -1.f : w;      // -1: nothing there
+    for (int s = 0; s < LM_ONCE; ++s)
+        if (s < n_splits) part[s] = load_vec<float, V>(po + (size_t)s * rank);
+    float mx = -INFINITY;
+    for (int s = lane; s < n_splits; s += 32) mx = fmaxf(mx, ml[s].x);
+    mx = warp_max(mx);
+    float denom = 0.f, acc[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = 0.f;
+    auto add = [&](const Vec<float, V>& p, float w, float lw) {
+        if (w < 0.f) return;      // nothing there
+        denom += lw;
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[e] = fmaf(p.v[e], w, acc[e]);
+    };
+    for (int s0 = 0; s0 < n_splits; s0 += 32) {      // lane s: share s0 + s
+        const float2 mine = s0 + lane < n_splits ? ml[s0 + lane] : make_float2(-INFINITY, 0.f);
+        const float w = mine.x == -INFINITY ? -1.f : exp2f(mine.x - mx), lw = mine.y * w;
+        const int here = min(32, n_splits - s0);
+        if (s0 == 0) {
+#pragma unroll
+            for (int s = 0; s < LM_ONCE; ++s)
+                if (s < here) add(part[s], __shfl_sync(0xffffffffu, w, s), __shfl_sync(0xffffffffu, lw, s));
         }
-        denom = warp_sum(denom);
-        if (head_sinks) denom += exp2f(head_sinks[head] * 1.4426950408889634f - mx);
-        const float inv = head_gate_of<__nv_bfloat16>(gates, gate_stride, t, head) / denom;
-        for (int s = lane; s < n_splits; s += 32)
-            if (weight_s[s] != -1.f) weight_s[s] *= inv;
+        for (int s = s0 == 0 ? LM_ONCE : 0; s < here; ++s)
+            add(load_vec<float, V>(po + (size_t)(s0 + s) * rank), __shfl_sync(0xffffffffu, w, s), __shfl_sync(0xffffffffu, lw, s));
     }
-    __syncthreads();
-    for (int c = threadIdx.x; c < rank; c += blockDim.x) {
-        if (c != c0) {
+    const int t = (int)(th / nh), head = (int)(th - (long long)t * nh);
+    if (head_sinks) denom += exp2f(head_sinks[head] * 1.4426950408889634f - mx);
+    const float inv = head_gate_of<__nv_bfloat16>(gates, gate_stride, t, head) / denom;      // no share with a key: not a number, as without shares
+    if (!has) return;
+    Vec<__nv_bfloat16, V> o;
 #pragma unroll
-            for (int s = 0; s < LM_ONCE; ++s) part[s] = s < n_splits ? po[(size_t)s * rank + c] : 0.f;
-        }
-        float acc = 0.f;
-#pragma unroll
-        for (int s = 0; s < LM_ONCE; ++s)
-            if (s < n_splits && !(weight_s[s] == -1.f)) acc = fmaf(part[s], weight_s[s], acc);
-        for (int s = LM_ONCE; s < n_splits; ++s)
-            if (!(weight_s[s] == -1.f)) acc = fmaf(po[(size_t)s * rank + c], weight_s[s], acc);
-        out[th * rank + c] = __float2bfloat16_rn(acc);
-    }
+    for (int e = 0; e < V; ++e) o.v[e] = __float2bfloat16_rn(acc[e] * inv);
+    store_vec<__nv_bfloat16, V>(out + (size_t)th * rank + c, o);
 }
 
-// n_tiles: an upper bound of the row tiles over the entries this launch takes (sum of ceil(len / (64 / hg)));
-// max_len > 0: only entries of at most that many tokens.  part_o [T, nh, n_splits, rank], part_ml [T, nh, n_splits, 2].
 PYRE_API int pyre_latent_attention_mma(const void* qa, const void* cache, void* out, float* part_o, float* part_ml,
                                        const int* block_table, int bt_stride, const int* cu_seqlens, const int* positions,
                                        int n_tokens, int n_seqs, int n_tiles, int nh, int rank, int row, int page_size, int window,
@@ -718,8 +724,12 @@ PYRE_API int pyre_latent_attention_mma(const void* qa, const void* cache, void* 
                 gate_stride, n_splits, max_len, n_pages, err_flag);
     PYRE_LAUNCH_CHECK();
     if (n_splits > 1) {
-        pyre_launch(latent_combine_kernel, dim3(n_tokens * nh), dim3(128), (size_t)n_splits * sizeof(float), stream, (const float*)part_o, (const float*)part_ml,
-                    (__nv_bfloat16*)out, n_splits, rank, nh, head_sinks, (const __nv_bfloat16*)gates, gate_stride);
+        const bool vec = rank % 4 == 0 && !((uintptr_t)part_o & 15) && !((uintptr_t)out & 7);
+        const int slices = ceil_div(rank, vec ? 128 : 32);
+        const long long items = (long long)n_tokens * nh * slices;
+        const auto kernel = vec ? latent_combine_kernel<4> : latent_combine_kernel<1>;
+        pyre_launch(kernel, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, stream, (const float*)part_o, (const float*)part_ml, (__nv_bfloat16*)out, n_splits, rank,
+                    nh, items, slices, head_sinks, (const __nv_bfloat16*)gates, gate_stride);
         PYRE_LAUNCH_CHECK();
     }
     return 0;
