@@ -61,9 +61,9 @@ __device__ __forceinline__ float head_gate_of(const T* gates, long long gate_str
 constexpr int LP_THREADS = 256, LP_KEEP = 4;
 
 // V neighbouring columns from `at` on, the partial sums added in their order
-template <typename T, int V>
+template <typename T, int V, bool PARTS>
 __device__ __forceinline__ void proj_vec(const T* proj, const float* parts, int n_parts, long long part_stride, size_t at, float (&v)[V]) {
-    if (parts) {
+    if (PARTS) {
         Vec<float, V> acc = load_vec<float, V>(parts + at);
 #pragma unroll 8
         for (int s = 1; s < n_parts; ++s) {
@@ -80,7 +80,7 @@ __device__ __forceinline__ void proj_vec(const T* proj, const float* parts, int 
     }
 }
 
-template <typename T, int V>
+template <typename T, int V, bool PARTS>
 __global__ void __launch_bounds__(LP_THREADS) latent_prepare_kernel(const T* proj, const float* parts, int n_parts, long long part_stride, int W,
                                       int q_col, int q_rank, int c_col, int rank, int rope, int rot, const float* wq,
                                       const float* wc, float eps, const float* cos_t, const float* sin_t, T* cq_out,
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prepare_kernel(const T* pro
     __shared__ float scratch[33];
     pdl_trigger();
     pdl_wait();
-    const int t = blockIdx.x;
+    const int t = blockIdx.x, threads = blockDim.x;
     const size_t base = (size_t)t * W;
     // dst[i] = rmsnorm(columns col .. col + width)[i] * w[i]
     auto normed = [&](int col, int width, const float* w, T* dst) {
@@ -100,15 +100,15 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prepare_kernel(const T* pro
         };
 #pragma unroll
         for (int n = 0; n < LP_KEEP; ++n) {
-            const int i = (n * LP_THREADS + threadIdx.x) * V;
+            const int i = (n * threads + threadIdx.x) * V;
             if (i < width) {
-                proj_vec<T, V>(proj, parts, n_parts, part_stride, base + col + i, keep[n]);
+                proj_vec<T, V, PARTS>(proj, parts, n_parts, part_stride, base + col + i, keep[n]);
                 add(keep[n]);
             }
         }
-        for (int i = (LP_KEEP * LP_THREADS + threadIdx.x) * V; i < width; i += LP_THREADS * V) {
+        for (int i = (LP_KEEP * threads + threadIdx.x) * V; i < width; i += threads * V) {
             float v[V];
-            proj_vec<T, V>(proj, parts, n_parts, part_stride, base + col + i, v);
+            proj_vec<T, V, PARTS>(proj, parts, n_parts, part_stride, base + col + i, v);
             add(v);
         }
         const float rstd = 1.0f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
@@ -120,12 +120,12 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prepare_kernel(const T* pro
         };
 #pragma unroll
         for (int n = 0; n < LP_KEEP; ++n) {
-            const int i = (n * LP_THREADS + threadIdx.x) * V;
+            const int i = (n * threads + threadIdx.x) * V;
             if (i < width) put(i, keep[n]);
         }
-        for (int i = (LP_KEEP * LP_THREADS + threadIdx.x) * V; i < width; i += LP_THREADS * V) {
+        for (int i = (LP_KEEP * threads + threadIdx.x) * V; i < width; i += threads * V) {
             float v[V];
-            proj_vec<T, V>(proj, parts, n_parts, part_stride, base + col + i, v);
+            proj_vec<T, V, PARTS>(proj, parts, n_parts, part_stride, base + col + i, v);
             put(i, v);
         }
     };
@@ -136,16 +136,16 @@ __global__ void __launch_bounds__(LP_THREADS) latent_prepare_kernel(const T* pro
         if (slot < 0) return;   // the whole block
         T* dst = cache + (size_t)slot * row;
         normed(c_col, rank, wc, dst);
-        for (int i = threadIdx.x; i < rope; i += LP_THREADS) {
+        for (int i = threadIdx.x; i < rope; i += threads) {
             const size_t at0 = base + c_col + rank;
             dst[rank + i] = from_f32<T>(turned([&](int j) { return proj_at<T>(proj, parts, n_parts, part_stride, at0 + j); }, i, rot, halves, ct, st));
         }
-        for (int i = rank + rope + threadIdx.x; i < row; i += LP_THREADS) dst[i] = from_f32<T>(0.f);
+        for (int i = rank + rope + threadIdx.x; i < row; i += threads) dst[i] = from_f32<T>(0.f);
     } else if (blockIdx.y == 1 && q_rank > 0) {
         normed(q_col, q_rank, wq, cq_out + (size_t)t * q_rank);
     } else if (qa) {
         const int tail = row - rank;
-        for (int idx = threadIdx.x; idx < nh * tail; idx += LP_THREADS) {
+        for (int idx = threadIdx.x; idx < nh * tail; idx += threads) {
             const int h = idx / tail, i = idx - h * tail;
             float o = 0.f;
             if (i < rope) {
@@ -172,10 +172,14 @@ PYRE_API int pyre_latent_prepare(const void* proj, const float* parts, int n_par
     const int esize = dtype == PYRE_F32 ? 4 : 2, in_esize = parts ? 4 : esize;
     const bool vec = W % 4 == 0 && part_stride % 4 == 0 && q_col % 4 == 0 && q_rank % 4 == 0 && c_col % 4 == 0 && rank % 4 == 0 && row % 4 == 0 &&
                      ((uintptr_t)(parts ? (const void*)parts : proj)) % (4 * in_esize) == 0 && (uintptr_t)cache % (4 * esize) == 0 && (uintptr_t)cq_out % (4 * esize) == 0;
-#define GO(T, V) pyre_launch(latent_prepare_kernel<T, V>, grid, dim3(LP_THREADS), 0, stream, (const T*)proj, parts, n_parts, part_stride, W, q_col, q_rank, c_col, \
-                             rank, rope, rot, wq, wc, eps, cos_t, sin_t, (T*)cq_out, (T*)cache, slot_mapping, row, n_pages, page_size, halves, (T*)qa, qh_col, nh, dq, err_flag)
-    if (dtype == PYRE_BF16) vec ? GO(__nv_bfloat16, 4) : GO(__nv_bfloat16, 1);
-    else if (dtype == PYRE_F32) vec ? GO(float, 4) : GO(float, 1);
+    // as many threads as the widest piece has vectors, up to LP_THREADS: a thread without a vector adds a zero, so their number does not
+    // change a bit
+    const int vectors = max(ceil_div(max(q_rank, rank), vec ? 4 : 1), qa ? nh * (row - rank) : rope);
+    const int threads = 32 * min(LP_THREADS / 32, ceil_div(vectors, 32));
+#define GO(T, V, PARTS) pyre_launch(latent_prepare_kernel<T, V, PARTS>, grid, dim3(threads), 0, stream, (const T*)proj, parts, n_parts, part_stride, W, q_col, q_rank, c_col, \
+                                    rank, rope, rot, wq, wc, eps, cos_t, sin_t, (T*)cq_out, (T*)cache, slot_mapping, row, n_pages, page_size, halves, (T*)qa, qh_col, nh, dq, err_flag)
+    if (dtype == PYRE_BF16) parts ? (vec ? GO(__nv_bfloat16, 4, true) : GO(__nv_bfloat16, 1, true)) : vec ? GO(__nv_bfloat16, 4, false) : GO(__nv_bfloat16, 1, false);
+    else if (dtype == PYRE_F32) parts ? (vec ? GO(float, 4, true) : GO(float, 1, true)) : vec ? GO(float, 4, false) : GO(float, 1, false);
     else return PYRE_ERR_BAD_ARG;
 #undef GO
     PYRE_LAUNCH_CHECK();
