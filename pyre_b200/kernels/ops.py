@@ -2055,9 +2055,10 @@ def latent_mma_ok(dtype: torch.dtype, row: int) -> bool:
 def latent_attention_splits(n_tiles: int, n_heads: int, rank: int, span: int, row: "int | None" = None) -> int:
     """Into how many shares the tensor-core latent attention cuts the keys of every row tile: as many as fill the CTAs
     that are resident at once (its shared memory and threads allow one to a few per SM: whole rounds, since a second
-    round of CTAs costs as much as the first) with at least four key tiles per share, or as many as have an SM each with at least
-    two (a share is a chain of memory latencies, and SMs idle: four tokens of 16 heads after 700 rows, combining included, 24.5 us
-    with five shares, 18.5 with eleven); at most 16.  ``span``: the most keys
+    round of CTAs costs as much as the first) with at least four key tiles per share, or, where the estimate says that it pays,
+    as many as have an SM each with at least two (a share is a chain of memory latencies, and SMs idle: four tokens of 16 heads after
+    700 rows, combining included, 20.5 us with five shares, 13.0 with eleven; but what a share leaves goes through memory: 64
+    tokens of 64 heads after 100 rows 27.2 us with one, 30.1 with two); at most 16.  ``span``: the most keys
     a tile walks; ``row``: entries of a cached row (default: the latent and a rotated part of a quarter of it)."""
     ctas = max(1, n_tiles * -(-n_heads // LATENT_MMA_ROWS))      # the column groups of a wide latent are warps of one CTA
     groups = -(-rank // LATENT_MMA_COLS)
@@ -2065,7 +2066,11 @@ def latent_attention_splits(n_tiles: int, n_heads: int, rank: int, span: int, ro
     smem = (LATENT_MMA_ROWS + 2 * LATENT_MMA_KEYS) * (row + 8) * 2 + (4 * groups * 16 * 32 * 4 if groups > 1 else 0)
     resident = sm_count() * max(1, min(227 * 1024 // smem, 2048 // (128 * groups), 4))
     tiles = -(-span // LATENT_MMA_KEYS) + 1
-    return int(max(1, min(resident // ctas, tiles // 4, 16), min(sm_count() // ctas, tiles // 2, 16)))
+    few, many = int(max(1, min(resident // ctas, tiles // 4, 16))), int(min(sm_count() // ctas, tiles // 2, 16))
+
+    def estimate(n):      # microseconds, fitted to decoded tokens of 8 to 128 heads and latents of 64 to 512
+        return -(-(tiles - 1) // n) * (1.0 + 0.0063 * rank) + (2.4 + 0.0006 * n * n_tiles * n_heads if n > 1 else 0.0)
+    return many if many > few and estimate(many) < estimate(few) else few
 
 
 def latent_attention_mma(qa: torch.Tensor, cache_layer: torch.Tensor, block_table: torch.Tensor, cu_seqlens: torch.Tensor,

@@ -111,3 +111,18 @@ def test_shares_of_the_keys_in_the_prompt_attention(monkeypatch):
     assert ops.prefill_key_splits(1 * 28, 481.0, 128, 28, 128) == 8             # one query tile per head
     assert ops.prefill_key_splits(1 * 28, 40.0, 128, 28, 128) == 2              # shares of at least 16 tiles
     assert ops.prefill_key_splits(2 * 28, 484.0, 1 << 18, 28, 128) == 1         # the scratch would not fit
+
+
+def test_latent_attention_shares():
+    """Shares of a latent attention's keys: in range, and where they were measured as measured (one share or few against as many as have an SM)."""
+    for tiles in [1, 2, 8, 24, 48, 64, 128, 500]:
+        for heads, rank, row in [(2, 24, 32), (16, 256, 320), (28, 512, 576), (72, 128, 160), (128, 512, 576)]:
+            for span in [1, 33, 70, 200, 1500, 30000]:
+                n = ops.latent_attention_splits(tiles, heads, rank, span, row)
+                assert 1 <= n <= 16 and (n == 1 or n <= span // 32 + 2), (tiles, heads, rank, span, n)
+    assert ops.latent_attention_splits(4, 16, 256, 700, 320) == 11       # 20.5 us with five, 13.0 so
+    assert ops.latent_attention_splits(1, 16, 256, 100, 320) == 2        # 15.5 with one, 12.0 so
+    assert ops.latent_attention_splits(4, 28, 512, 100, 576) == 2        # 25.3 with one, 17.7 so
+    assert ops.latent_attention_splits(64, 64, 256, 100, 320) == 1       # 27.2 so, 30.1 with two: 4,096 rows make the trip through memory
+    assert ops.latent_attention_splits(24, 72, 128, 100, 160) == 1       # 17.4 so, 18.6 with two
+    assert ops.latent_attention_splits(32, 128, 512, 70, 576) == 1       # 31.3 so, 34.0 with two
