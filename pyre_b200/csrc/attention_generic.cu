@@ -41,7 +41,7 @@ __device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((uint32_t
 __device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
 
 // R rows of NI * 128 dims at most (a lane holds the dims 4 lane + 128 i .. + 3).  Rows are (token of the group, head of
-// the group), token first: `tpg` tokens of `hpg` heads, hpg * tpg <= R; blockIdx.y is the head group: kv head, and which
+// the group), token first: `tpg` tokens of `hpg` heads, hpg * tpg <= R; blockIdx.y (and .z) is the head group: kv head, and which
 // of its `hgroups` groups of query heads.  Warp w takes chain w of the rows' chunks.
 // SHORT: tables of at most 256 keys, so that a chain is one chunk and most chains of short rows are empty.  A CTA then owns `per_cta` groups
 // of rows; as many warps share a group as its longest row has chunks, and the groups that do not fit follow in passes.
@@ -67,8 +67,10 @@ __global__ void __launch_bounds__(AG_WARPS * 32, DEEP ? 1 : R * NI <= 2 ? 3 : 2)
     __shared__ int seq_all[AG_WARPS * R], pos_all[AG_WARPS * R], lo_all[AG_WARPS * R], last_pos;
     pdl_trigger();
     pdl_wait();
-    const int n_rep = nh / nkv, kvh = blockIdx.y / hgroups;
-    const int first_head = (blockIdx.y - kvh * hgroups) * hpg;                 // within the kv head's query heads
+    const int head_group = blockIdx.y + gridDim.y * blockIdx.z;                // a grid's second dimension ends at 65,535
+    if (head_group >= nkv * hgroups) return;                                   // the whole CTA
+    const int n_rep = nh / nkv, kvh = head_group / hgroups;
+    const int first_head = (head_group - kvh * hgroups) * hpg;                 // within the kv head's query heads
     const int heads = min(hpg, n_rep - first_head);
     const int t_cta = blockIdx.x * groups * tpg;
     // row r of group g: its token, or -1 where there is no such row
@@ -319,7 +321,8 @@ template <typename T, int R, int NI, bool DEEP, bool SHORT>
 static int launch_generic_as(const GenericArgs& a, const GenericPlan& p) {
     const size_t smem = ((size_t)p.per_cta * R * a.hd + AG_WARPS * 32 * R + (size_t)AG_WARPS * R * a.hd) * sizeof(float);
     static_assert(((SHORT ? AG_WARPS + most_per_cta(R, NI) : AG_WARPS + 1) * R * NI * 128 + AG_WARPS * 32 * R) * 4 <= 46 * 1024, "fits without an attribute");
-    const dim3 grid(ceil_div(ceil_div(a.n_tokens, p.tpg), p.per_cta), a.nkv * p.hgroups);
+    const int head_groups = a.nkv * p.hgroups, across = min(head_groups, 32768);
+    const dim3 grid(ceil_div(ceil_div(a.n_tokens, p.tpg), p.per_cta), across, ceil_div(head_groups, across));
     return (int)pyre_launch(paged_attention_generic_kernel<T, R, NI, DEEP, SHORT>, grid, dim3(AG_WARPS * 32), smem, a.stream,
                             (const T*)a.q, (const T*)a.cache, (T*)a.out, a.block_table, a.bt_stride, a.seq_of_token, a.positions,
                             a.n_tokens, a.nh, a.nkv, a.hd, a.page_size, a.window, a.keep_first, a.scale, a.sink, a.head_sinks, a.n_pages, a.err_flag,

@@ -194,3 +194,17 @@ def test_product_of_very_many_rows(ops, K):
     got = ops.sgemm_nt(a, w)
     want, size = a.double() @ w.double().t(), a.double().abs() @ w.double().abs().t()
     assert ((got.double() - want).abs() <= 4 * EPS * size).all()      # two additions of each of two chains, one of the chains
+
+
+@pytest.mark.parametrize("nh,nkv", [(65541, 65541), (65537 * 3, 1)])
+def test_attention_of_very_many_heads(ops, nh, nkv):
+    """More groups of heads than the second dimension of a grid holds."""
+    g = torch.Generator(device="cuda").manual_seed(nkv)
+    hd, page = 16, 4
+    cache = torch.randn(2, 2, nkv, page, hd, device="cuda", generator=g)
+    table = torch.tensor([[1, 0], [0, 1]], dtype=torch.int32, device="cuda")
+    seq, pos = (torch.tensor(v, dtype=torch.int32, device="cuda") for v in ([0, 1], [6, 2]))
+    q, sink = torch.randn(2, nh * hd, device="cuda", generator=g), torch.randn(nh, device="cuda", generator=g)
+    got = ops.paged_attention_generic(q, cache, table, seq, pos, nh, nkv, hd, 0.25, sink=sink)
+    want = reference(q, cache, table, seq, pos, nh, nkv, hd, 0.25, None, 0, sink)
+    assert ((got.double() - want).abs() <= 2e-6).all()
