@@ -342,7 +342,7 @@ static int launch_generic(const GenericArgs& a, GenericPlan p, bool is_short) {
 }
 
 // The most rows whose groups still fill the SMs: 1.5 groups of eight per SM, 0.6 of four or two (few groups are bound by the
-// chain of a warp's latencies, which more rows make longer); at least half of a group's rows have to be live.  Tables of a chunk or two: at most two
+// chain of a warp's latencies, which more rows make longer); more than half of a group's rows have to be live.  Tables of a chunk or two: at most two
 // rows, of up to eight chunks: at most four.  Tokens share a group only where the sequences (at most `n_seqs`) bring four groups each on
 // average: rows of different sequences are walked one after the other.  Measured with float32 storage (us: a warp per row / eight warps
 // and always eight rows / by this rule): 32 query heads on 32 of 128, 64 decoded tokens after some 1,600 keys 1040 / 1253 / 597, after 20 keys 15 / 106 /

@@ -30,7 +30,7 @@
 // value it was scaled with (probabilities then stay below 256, exact in the final O / l);
 // the rescale is a tcgen05.ld / multiply / tcgen05.st pass over the row.
 // S is double-buffered in tensor memory: the scores of tile i + 1 are computed while the row
-// threads work on tile i.  Two CTAs fit on an SM (112 KB of shared memory, 256 TMEM columns
+// threads work on tile i.  Two CTAs fit on an SM (96 KB of shared memory, 256 TMEM columns
 // each), so the tensor core also alternates between two CTAs.  The grid runs the heads fastest
 // and the tiles of a portion from its end, so the tiles with the most keys start first.
 // The softmax arithmetic uses the packed fp32 pairs of sm_100 (fma.rn.f32x2, add.rn.f32x2), the

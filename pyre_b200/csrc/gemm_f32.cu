@@ -46,7 +46,8 @@ __device__ __forceinline__ void copy4(float* dst, const float* src, bool live) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Many rows.  Bound by the FMA pipe: fma.rn.f32x2 alone, out of registers, reaches 49 TFLOP/s on this chip; a thread owns 8 x 4
+// Many rows.  Bound by the FMA pipe's operands: out of registers alone, fma.rn.f32x2 reaches 49 TFLOP/s on this chip where no
+// operand stays from one instruction to the next and 58 to 63 where one does (the register file's ports; scalar fmaf 61).  A thread owns 8 x 4
 // outputs as even-odd pairs, four k cost it 12 reads of 16 bytes from shared memory and 64 fma.rn.f32x2.  128 threads on a
 // 64 x 64 tile and 168 registers put three CTAs on an SM, whose barriers and first loads hide behind one another; operands
 // arrive by cp.async, 16 k at a time and two steps ahead, in rows of 20 floats (reads of 16 bytes by eight neighbouring

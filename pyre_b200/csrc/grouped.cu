@@ -8,10 +8,12 @@
 //   * the rows are sorted by group, group g owning the sorted places offsets[g] .. offsets[g + 1] (a product per
 //     EXPERT of a routed feed-forward: `src` gathers a place's input row, `dst` says where its result goes).
 //
-// One CTA computes a 64 x 64 tile of a group's result (128 x 128 for bfloat16 groups of many rows).  float32: FFMA, one chain per output element over k in
+// One CTA computes a tile of a group's result.  float32: 64 x 64, FFMA, one chain per output element over k in
 // ascending order, so a row's result does not depend on which other rows share its tile or its launch.
-// bfloat16 operands: on the tensor cores with fp32 accumulators, groups of few rows by mma.sync m16n8k16 (a weight stream:
-// its tiles grow with the rows in steps of 16), groups of many rows by tcgen05.mma.
+// bfloat16 operands: on the tensor cores with fp32 accumulators, by the rows per group on average: up to 16 of them tiles of
+// 16 rows x 64 features, below 96 (or with K below 64) tiles of 64 x 64, both by mma.sync m16n8k16 (a weight stream), else 128 x 128 by
+// tcgen05.mma.  The two instructions add the products of a k step in different orders: a bfloat16 row's last bits depend on which
+// kernel takes its launch.
 // `dtype`: type of x and w (0 = float32, 1 = bfloat16); `out_f32`: the result stays fp32, else it is rounded to dtype.
 #include "common.cuh"
 
@@ -143,18 +145,17 @@ __global__ void __launch_bounds__(256) grouped_linear_kernel(GroupedArgs a) {
 
 // ---------------------------------------------------------------------------
 // bfloat16, groups of few rows: tiles of 64 features by mma.sync, bound by reading the weights (a decoded token's experts have a row
-// or two each).  K in steps of 64 through a ring of four stages filled by cp.async, so that a CTA has 24 KB of weights in
-// flight and three CTAs fit on an SM; each of the four warps owns 16 output features and as many 16-row pieces as the
-// tile has rows, so that two rows do not cost the multiplications of 64.  Measured inside a decode step of 4 tokens (16
-// places of 32 experts, 2048 x 2048 and 2048 x 1024 weights): 95 -> 28 us and 50 -> 16 us (64-row
-// tiles whatever the rows, one step ahead through registers); 64 tokens: 111 -> 70 us.
-// Needs K % 8 == 0 and 16-byte aligned rows of x and w.
-// ---------------------------------------------------------------------------
-//
+// or two each).  K in steps of 64 through a ring filled by cp.async, so that a CTA has up to 40 KB of weights in
+// flight; each of the four warps owns 16 output features and as many 16-row pieces as the
+// tile has rows, so that two rows do not cost the multiplications of 64.  Needs K % 8 == 0 and 16-byte aligned rows of x and w.
+// Measured inside a decode step of 4 tokens (16 places of 32 experts, 2048 x 2048 and 2048 x 1024 weights), 64-row tiles one step
+// ahead through registers / the ring with 64 rows: 95 / 28 us and 50 / 16 us; 64 tokens: 111 / 70 us.
 // ROWS: the height of a tile.  Groups of few rows take tiles of 16 rows, whose ring holds little but weights; a group with more rows
 // takes more tiles, whose weights then come out of the L2 cache.  32 experts of 2048 x 2048, top 4, captured launches one after the
 // other, 64 rows of four stages / 16 rows of six / of four: 4 tokens 27.4 / 21.6 / 23.5 us, 8: 49.7 / 39.5 / 45.6, 32: 72.3 / 57.2 /
-// 50.5, 128: 76.4 / 70.6 / 64.6.
+// 50.5, 128: 76.4 / 70.6 / 64.6.  The lines were drawn there; against the kernels with registers in 300 other cases (8 to 256 experts of
+// 64 x 64 to 14336 x 4096, 1 to 2,240 tokens, top 2 and 4, also with all rows in four of the experts) no one got slower.
+// ---------------------------------------------------------------------------
 constexpr int GT_K = 64, GT_LD = GT_K + 8;   // padded rows: 144 bytes, conflict-free for ldmatrix
 template <int ROWS, int STAGES> struct GtRing {
     static constexpr int STAGE = (ROWS + GB_N) * GT_LD, SMEM = STAGES * STAGE * 2;
