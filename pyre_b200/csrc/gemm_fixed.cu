@@ -1,0 +1,615 @@
+// 32-bit matrix product in fixed point on the 5th-generation tensor cores:  C[M, N] = A[M, K] * W[N, K]^T, all float32.
+//
+// A row of either operand is taken as 31-bit integers on a power-of-two scale of its own, x = X 2^(E - 29) with E the
+// exponent of the row's largest element (|X| <= 2^30), and X as four signed bytes, X = sum_p d_p 2^(8 (3 - p)).  Products of
+// byte planes are summed by tcgen05.mma kind::i8 in 32-bit integers, exactly, planes i and j into the sum i + j; the sums
+// 0 .. 4 (13 of the 16 products) make a 64-bit integer that is scaled and rounded to float once.  An output is therefore
+// off by one rounding to float, 2^-30 of the rows' largest elements per factor, and the products left out (some 2^-35 of the product of
+// the two largest elements per term), where a chain of fused multiply-adds rounds with every term.  Against 64 bits (2-norm of the
+// error over 2-norm of the result, this / the sums of gemm_f32.cu): normal operands, K = 512 .. 3,584 2.5e-8 / 0.9-1.2e-7; rows with one
+// element 3,000 times the others 3.4e-8 / 1.5e-7; log-normal operands 4.0e-8 / 4.1e-8; where one column of A is a thousand times the others
+// and that column of W a thousandth, so that the result does not see it, 3.0e-7 / 1.2e-7.
+//
+// Integers add up in any order: a row's result has the same bits for any M, tile, split of K or order of arrival.
+//
+// A row with an infinity or a NaN has no scale.  Its outputs are worked out from the float operands: NaN if the row holds
+// one, else the sum over the infinite elements, which is what an IEEE sum over all of them gives.
+//
+// Two kernels: the activations' exponents and byte planes (they are few), then the product.  The product's CTA (640 threads)
+// owns 128 output features (the weights on the MMA's rows) and TN tokens, K in steps of 32:
+//   warp 0, one thread  : TMA.  Weights as they are, 128 x 32 floats a step (128-byte swizzle), into one ring; the tokens' four
+//                         byte planes, 128 k at a time, into another.
+//   warps 4..19         : a thread owns a feature.  Groups of four warps take the steps in turn: 32 floats from shared memory,
+//                         scaled, converted, transposed into byte planes (six instructions each) and stored to tensor
+//                         memory, which is where the MMAs take their A operand from.  After the K loop the same threads
+//                         put the five sums of their features together.
+//   warp 1, one thread  : four MMAs a step, one per weight plane i, with the tokens' planes 0 .. 4 - i side by side as the N
+//                         dimension: they add to the sums i .. 4, which lie side by side in the same order.
+// Weights stay float32 in memory and are converted on the way, once per tile of tokens: with few tokens that hides behind the
+// stream from memory, with many behind the MMAs.
+#include <cuda.h>
+
+#include "common.cuh"
+
+namespace {
+constexpr int ERR_TIMEOUT = 2;
+constexpr int E_NAN = 2000, E_INF = 1000;      // exponents of rows without a scale: a NaN, an infinity
+constexpr int E_MIN = -98;                     // of a row of zeros (its scale is a normal float)
+constexpr int FEATURES = 128, STEP = 32, BLOCK_K = 128;
+constexpr int CONV_WARP0 = 4, GROUPS = 4, CONV_THREADS = GROUPS * 128, THREADS = CONV_WARP0 * 32 + CONV_THREADS;
+constexpr int W_BYTES = FEATURES * STEP * 4;   // a step's weights
+constexpr int A_STAGES = 6, A_COLS = 32;       // converted steps in tensor memory: 8 columns per plane
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Bounded wait: false if the limit ran out or another thread already gave up.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err_flag) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const long long t0 = clock64();
+    for (uint32_t it = 1;; ++it) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((it & 63) == 0) {
+            if (*abort_flag) return false;
+            if (clock64() - t0 > PYRE_WAIT_CYCLES) break;
+        }
+    }
+    *abort_flag = 1;
+    if (err_flag) atomicExch(err_flag, ERR_TIMEOUT);
+    return false;
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1) : "memory");
+}
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+// K-major tile of 128-byte rows, 128-byte swizzle (eight rows 1024 bytes apart)
+__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
+           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+// D (tensor memory, 32-bit integers) += A (tensor memory, signed bytes) * B (shared memory, signed bytes)
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
+                 ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr) : "memory");
+}
+
+// 2^e for e in [-126, 127]
+__device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+// The exponent of a row from the largest |x| of its elements as bits (NaN above infinity above all numbers).
+__device__ __forceinline__ int row_exponent(uint32_t abs_bits) {
+    if (abs_bits >= 0x7f800000u) return abs_bits > 0x7f800000u ? E_NAN : E_INF;
+    if (abs_bits == 0) return E_MIN;
+    const int e = (int)(abs_bits >> 23);
+    return e ? e - 127 : 31 - __clz(abs_bits) - 149;
+}
+// x 2^(29 - E) as two factors: 29 - E reaches 178 for rows of the smallest numbers
+struct RowScale {
+    float s1, s2;
+};
+__device__ __forceinline__ RowScale row_scale(int E) {
+    if (E >= E_INF) return {0.f, 1.f};
+    const int t = 29 - E;
+    return {pow2f(min(t, 127)), t > 127 ? pow2f(t - 127) : 1.f};
+}
+// Four numbers already on their row's scale -> a word of four bytes for each plane.  Signed digits: adding 0x80 to the three lower bytes
+// carries what they exceed 127 by, taking it off again byte by byte leaves digits in [-128, 127].
+__device__ __forceinline__ void bytes_of(float x0, float x1, float x2, float x3, uint32_t& p0, uint32_t& p1, uint32_t& p2, uint32_t& p3) {
+    const uint32_t y0 = (uint32_t)__float2int_rn(x0) + 0x808080u, y1 = (uint32_t)__float2int_rn(x1) + 0x808080u;
+    const uint32_t y2 = (uint32_t)__float2int_rn(x2) + 0x808080u, y3 = (uint32_t)__float2int_rn(x3) + 0x808080u;
+    const uint32_t a = __byte_perm(y0, y1, 0x5140), b = __byte_perm(y2, y3, 0x5140);      // bytes 0 and 1
+    const uint32_t c = __byte_perm(y0, y1, 0x7362), d = __byte_perm(y2, y3, 0x7362);      // bytes 2 and 3
+    p3 = __byte_perm(a, b, 0x5410) ^ 0x80808080u;
+    p2 = __byte_perm(a, b, 0x7632) ^ 0x80808080u;
+    p1 = __byte_perm(c, d, 0x5410) ^ 0x80808080u;
+    p0 = __byte_perm(c, d, 0x7632);
+}
+
+// One output of rows of which at least one has no scale (rare: no attempt at speed).
+__device__ __noinline__ float unscaled_output(const float* a, const float* w, int K, int Ea, int Ew) {
+    if (Ea == E_NAN || Ew == E_NAN) return __uint_as_float(0x7fffffffu);
+    float sum = 0.f;
+    for (int k = 0; k < K; ++k) {
+        const float x = a[k], y = w[k];
+        if (isinf(x) || isinf(y)) {
+            sum += x * y;
+            if (isnan(sum)) break;
+        }
+    }
+    return sum;
+}
+
+struct FixedParams {
+    const float* A;
+    const float* W;
+    const int* w_exp;             // [N]
+    const int* a_exp;             // [M]
+    float* C;
+    long long lda, ldw, ldc;
+    int M, N, K;
+    int tiles_m, tiles;           // tiles of tokens; of everything (tokens fastest: the tiles of a block of weights run together)
+    int splits, steps_per_split;  // of K, in steps of 32 (a multiple of four per split)
+    long long* partial;           // [splits][tiles][TN][128] where K is split
+    int* counters;                // [tiles], zero
+    int* err_flag;
+};
+
+template <int TN> struct Layout {
+    static constexpr int W_STAGES = TN <= 16 ? 12 : TN <= 48 ? 9 : 8;
+    static constexpr int B_BYTES = 4 * TN * BLOCK_K, B_STAGES = TN <= 16 ? 4 : 3;
+    static constexpr int W_OFF = 0, B_OFF = W_STAGES * W_BYTES, BARS = B_OFF + B_STAGES * B_BYTES;
+    static constexpr int N_BARS = 2 * W_STAGES + 2 * B_STAGES + 2 * A_STAGES + 2;
+    static constexpr int TOTAL = BARS + N_BARS * 8 + 32 + 1024;
+    // an MMA of M = 128 takes N in sixteens: with eight tokens the third plane's product is one plane wider (its last sum is not read)
+    static constexpr int SUMS = TN == 8 ? 6 : 5;
+    static constexpr int A_COL0 = 512 - A_STAGES * A_COLS;
+    static_assert(TOTAL <= 232448 && SUMS * TN <= A_COL0 && (TN == 8 || TN % 16 == 0), "fits");
+};
+
+template <int TN>
+__global__ void __launch_bounds__(THREADS, 1)
+fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_b, const FixedParams p) {
+    using L = Layout<TN>;
+    static_assert(CONV_THREADS == 512, "the named barrier's count");
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* gen = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t w_full = base + L::BARS, w_empty = w_full + 8 * L::W_STAGES;
+    const uint32_t b_full = w_empty + 8 * L::W_STAGES, b_empty = b_full + 8 * L::B_STAGES;
+    const uint32_t a_full = b_empty + 8 * L::B_STAGES, a_empty = a_full + 8 * A_STAGES;
+    const uint32_t acc_full = a_empty + 8 * A_STAGES, acc_empty = acc_full + 8;
+    volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::BARS + L::N_BARS * 8);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 8);
+    volatile int* last_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 16);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int items = p.tiles * p.splits, total_steps = (p.K + STEP - 1) / STEP;
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        for (int s = 0; s < L::W_STAGES; ++s) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 4); }
+        for (int s = 0; s < L::B_STAGES; ++s) { mbar_init(b_full + 8 * s, 1); mbar_init(b_empty + 8 * s, 1); }
+        for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full + 8 * s, 4); mbar_init(a_empty + 8 * s, 1); }
+        mbar_init(acc_full, 1);
+        mbar_init(acc_empty, CONV_THREADS / 32);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    pdl_trigger();
+
+    // an item: a tile and a share of its K
+    auto range = [&](int item, int& tile, int& split, int& first, int& n) {
+        tile = item % p.tiles;
+        split = item / p.tiles;
+        first = split * p.steps_per_split;
+        n = max(0, min(p.steps_per_split, total_steps - first));
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_w)) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&map_b)) : "memory");
+            bool waited = false, ok = true;
+            int it = 0, bt = 0;      // steps and blocks of 128 k asked for so far
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+                int tile, split, first, n;
+                range(item, tile, split, first, n);
+                const int f0 = tile / p.tiles_m * FEATURES, t0 = tile % p.tiles_m * TN;
+                auto weights = [&](int i, int at) {
+                    const int s = at % L::W_STAGES;
+                    if (!mbar_wait(w_empty + 8 * s, ((at / L::W_STAGES) & 1) ^ 1, abort_flag, p.err_flag)) return false;
+                    mbar_expect_tx(w_full + 8 * s, W_BYTES);
+                    tma_load_2d(base + L::W_OFF + s * W_BYTES, &map_w, w_full + 8 * s, (first + i) * STEP, f0);
+                    return true;
+                };
+                int done = 0;
+                if (!waited) {
+                    // the weights depend on no earlier kernel
+                    done = min(n, L::W_STAGES);
+                    for (int i = 0; i < done; ++i) weights(i, i);
+                    pdl_wait();
+                    waited = true;
+                }
+                for (int i = 0; i < n && ok; ++i) {
+                    if ((i & 3) == 0) {
+                        const int s = bt % L::B_STAGES;
+                        ok = mbar_wait(b_empty + 8 * s, ((bt / L::B_STAGES) & 1) ^ 1, abort_flag, p.err_flag);
+                        if (!ok) break;
+                        mbar_expect_tx(b_full + 8 * s, L::B_BYTES);
+                        tma_load_3d(base + L::B_OFF + s * L::B_BYTES, &map_b, b_full + 8 * s, (first + i) * STEP, t0, 0);
+                        ++bt;
+                    }
+                    if (i >= done) ok = weights(i, it + i);
+                }
+                it += n;
+            }
+            if (!waited) pdl_wait();
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // D 32-bit integers (2 at bit 4), A and B signed bytes (1 at bits 7 and 10), N >> 3 at bit 17, M >> 4 at bit 24
+            constexpr uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(FEATURES >> 4) << 24);
+            constexpr uint32_t n4 = (uint32_t)(4 * TN >> 3) << 17, n3 = (uint32_t)((TN == 8 ? 32 : 3 * TN) >> 3) << 17, n2 = (uint32_t)(2 * TN >> 3) << 17;
+            int it = 0, bt = 0, j = 0;
+            bool ok = true;
+            for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++j) {
+                int tile, split, first, n;
+                range(item, tile, split, first, n);
+                ok = mbar_wait(acc_empty, j & 1, abort_flag, p.err_flag);
+                if (!ok) { umma_commit(acc_full); break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int i = 0; i < n; ++i, ++it) {
+                    const int sb = bt % L::B_STAGES, sa = it % A_STAGES;
+                    if ((i & 3) == 0) {
+                        ok = mbar_wait(b_full + 8 * sb, (bt / L::B_STAGES) & 1, abort_flag, p.err_flag);
+                        if (!ok) break;
+                    }
+                    ok = mbar_wait(a_full + 8 * sa, (it / A_STAGES) & 1, abort_flag, p.err_flag);
+                    if (!ok) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t db = umma_desc(base + L::B_OFF + sb * L::B_BYTES) + 2 * (i & 3);      // 32 bytes of k further
+                    const uint32_t a = tmem + L::A_COL0 + sa * A_COLS;
+                    umma_i8(tmem, a, db, idesc | n4, i > 0);                      // plane 0: sums 0 .. 3
+                    umma_i8(tmem + TN, a + 8, db, idesc | n4, 1);                 // plane 1: sums 1 .. 4 (4 starts as zeros)
+                    umma_i8(tmem + 2 * TN, a + 16, db, idesc | n3, 1);            // plane 2: sums 2 .. 4
+                    umma_i8(tmem + 3 * TN, a + 24, db, idesc | n2, 1);            // plane 3: sums 3, 4
+                    umma_commit(a_empty + 8 * sa);
+                    if ((i & 3) == 3 || i == n - 1) {
+                        umma_commit(b_empty + 8 * sb);
+                        ++bt;
+                    }
+                }
+                umma_commit(acc_full);      // also where a wait ran out
+            }
+        }
+    } else if (warp >= CONV_WARP0) {
+        const int group = (warp - CONV_WARP0) >> 2, quarter = warp & 3, row = quarter * 32 + lane;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        // the tile's columns that this group puts together (whole loads of eight: with few columns not every group has some)
+        constexpr int COLS = (TN + 8 * GROUPS - 1) / (8 * GROUPS) * 8;
+        const int col0 = group * COLS;
+        const bool has_cols = col0 < TN;
+        static_assert(TN % COLS == 0, "every group has all of its columns or none");
+        const uint32_t zeros[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        auto clear_last_sum = [&]() {      // no first MMA overwrites the sum 4
+            if (has_cols)
+                for (int c = 0; c < COLS; c += 8) tmem_st8(tmem + lanes + 4 * TN + col0 + c, zeros);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty);
+        };
+        clear_last_sum();
+        bool waited = false, ok = true;
+        int it = 0, j = 0;
+        for (int item = blockIdx.x; item < items; item += gridDim.x, ++j) {
+            int tile, split, first, n;
+            range(item, tile, split, first, n);
+            const int f = tile / p.tiles_m * FEATURES + row, t0 = tile % p.tiles_m * TN;
+            const int Ew = f < p.N ? p.w_exp[f] : E_MIN;
+            const RowScale sc = row_scale(Ew);
+            const bool tiny = __any_sync(0xffffffffu, sc.s2 != 1.f);
+            for (int i = (group - it) & (GROUPS - 1); i < n && ok; i += GROUPS) {
+                const int at = it + i, s = at % L::W_STAGES, sa = at % A_STAGES;
+                ok = mbar_wait(w_full + 8 * s, (at / L::W_STAGES) & 1, abort_flag, p.err_flag);
+                const uint32_t src = base + L::W_OFF + s * W_BYTES + row * 128;
+                uint32_t pl[4][8];
+                float4 v[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q].z), "=f"(v[q].w)
+                                 : "r"(src + ((q ^ (row & 7)) << 4)) : "memory");
+                if (tiny) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) { v[q].x *= sc.s2; v[q].y *= sc.s2; v[q].z *= sc.s2; v[q].w *= sc.s2; }
+                }
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    bytes_of(v[q].x * sc.s1, v[q].y * sc.s1, v[q].z * sc.s1, v[q].w * sc.s1, pl[0][q], pl[1][q], pl[2][q], pl[3][q]);
+                __syncwarp();
+                if (lane == 0) mbar_arrive(w_empty + 8 * s);
+                ok = mbar_wait(a_empty + 8 * sa, ((at / A_STAGES) & 1) ^ 1, abort_flag, p.err_flag) && ok;
+                ok = __all_sync(0xffffffffu, ok);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+                for (int q = 0; q < 4; ++q) tmem_st8(tmem + lanes + L::A_COL0 + sa * A_COLS + 8 * q, pl[q]);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(a_full + 8 * sa);
+            }
+            it += n;
+            if (!waited) { pdl_wait(); waited = true; }
+            ok = mbar_wait(acc_full, j & 1, abort_flag, p.err_flag) && ok && !*abort_flag;
+            // all warps of the groups agree: they meet at a barrier below
+            {
+                uint32_t r;
+                asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.and.pred q, 1, 512, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                             : "=r"(r) : "r"((uint32_t)ok) : "memory");
+                ok = r != 0;
+            }
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // sum s stands for 2^(8 (6 - s)); a row's scale is 2^(E - 29): C = total 2^(16 + Ea + Ew - 58)
+            auto finish = [&](int t, long long total) {
+                if (t >= p.M || f >= p.N) return;
+                const int Ea = p.a_exp[t];
+                float out;
+                if (Ea >= E_INF || Ew >= E_INF) out = unscaled_output(p.A + (size_t)t * p.lda, p.W + (size_t)f * p.ldw, p.K, Ea, Ew);
+                else out = (float)(__ll2double_rn(total) * __hiloint2double((Ea + Ew - 42 + 1023) << 20, 0));
+                p.C[(size_t)t * p.ldc + f] = out;
+            };
+            long long* const mine = p.partial + ((size_t)(split * p.tiles + tile) * TN) * FEATURES + row;
+            if (has_cols) {
+#pragma unroll 1
+                for (int c = 0; c < COLS; c += 8) {
+                    int s[5][8];
+                    __syncwarp();
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) tmem_ld8(tmem + lanes + q * TN + col0 + c, s[q]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) {
+                        const long long total = ((long long)s[0][e] << 32) + ((long long)s[1][e] << 24) + ((long long)s[2][e] << 16) +
+                                                ((long long)s[3][e] << 8) + s[4][e];
+                        if (p.splits == 1) finish(t0 + col0 + c + e, total);
+                        else if (t0 + col0 + c + e < p.M) mine[(size_t)(col0 + c + e) * FEATURES] = total;
+                    }
+                }
+            }
+            __syncwarp();
+            clear_last_sum();
+            if (p.splits > 1) {
+                // whoever arrives last adds up the tile's shares
+                __threadfence();
+                asm volatile("bar.sync 1, 512;" ::: "memory");
+                if (threadIdx.x == CONV_WARP0 * 32) *last_flag = atomicAdd(p.counters + tile, 1) == p.splits - 1;
+                asm volatile("bar.sync 1, 512;" ::: "memory");
+                if (*last_flag) {
+                    __threadfence();
+                    const int rows = min(TN, p.M - t0);
+                    for (int c = group; c < rows; c += GROUPS) {
+                        const long long* from = p.partial + ((size_t)tile * TN + c) * FEATURES + row;
+                        long long total = 0;
+                        for (int z = 0; z < p.splits; ++z) total += __ldcg(from + (size_t)z * p.tiles * TN * FEATURES);
+                        finish(t0 + c, total);
+                    }
+                }
+                asm volatile("bar.sync 1, 512;" ::: "memory");      // the flag is read before the next item writes it
+            }
+        }
+        if (!waited) pdl_wait();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+// A row's exponent, and (PLANES) its elements as four byte planes [4][rows][pitch].  A block per row, which it reads twice (the second time
+// out of the caches).
+constexpr int ROW_THREADS = 256;
+template <bool PLANES, bool VEC>
+__global__ void __launch_bounds__(ROW_THREADS)
+fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* planes, long long plane_stride, int pitch, int* counters, int n_counters) {
+    __shared__ uint32_t s_max[ROW_THREADS / 32];
+    if (PLANES) pdl_trigger();      // a weight's exponents: no product may start beside them (it reads them ahead of its own wait)
+    pdl_wait();
+    const int tid = threadIdx.x;
+    const float* a = A + (size_t)blockIdx.x * lda;
+    if (PLANES)
+        for (int i = blockIdx.x * ROW_THREADS + tid; i < n_counters; i += gridDim.x * ROW_THREADS) counters[i] = 0;
+    uint32_t most = 0;
+    if constexpr (VEC) {
+#pragma unroll 4
+        for (int k = 4 * tid; k < K; k += 4 * ROW_THREADS) {
+            const uint4 v = *reinterpret_cast<const uint4*>(a + k);
+            most = max(max(max(most, v.x & 0x7fffffffu), max(v.y & 0x7fffffffu, v.z & 0x7fffffffu)), v.w & 0x7fffffffu);
+        }
+    } else {
+#pragma unroll 4
+        for (int k = tid; k < K; k += ROW_THREADS) most = max(most, __float_as_uint(a[k]) & 0x7fffffffu);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((tid & 31) == 0) s_max[tid >> 5] = most;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ROW_THREADS / 32; ++i) most = max(most, s_max[i]);
+    const int E = row_exponent(most);
+    if (tid == 0) exps[blockIdx.x] = E;
+    if constexpr (PLANES) {
+        const RowScale sc = row_scale(E);
+        uint8_t* out = planes + (size_t)blockIdx.x * pitch;
+#pragma unroll 2
+        for (int k = 4 * tid; k < pitch; k += 4 * ROW_THREADS) {
+            float x[4];
+            if (VEC && k < K) {
+                const float4 v = *reinterpret_cast<const float4*>(a + k);
+                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = k + e < K ? a[k + e] : 0.f;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[e] = E >= E_INF ? 0.f : x[e] * sc.s2 * sc.s1;
+            uint32_t w[4];
+            bytes_of(x[0], x[1], x[2], x[3], w[0], w[1], w[2], w[3]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) *reinterpret_cast<uint32_t*>(out + q * plane_stride + k) = w[q];
+        }
+    }
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiledFn encode_tiled() {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void* ptr = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiledFn>(ptr);
+    }
+    return fn;
+}
+
+struct Plan {
+    int tn, tiles_m, tiles, splits, steps_per_split;
+    long long planes, exps, counters, partial, bytes;      // offsets into the workspace
+    int pitch;
+};
+// Tokens per tile and shares of K by estimated cycles of the busiest SM.
+Plan make_plan(int M, int N, int K, int sms, int force_tn, int force_splits) {
+    Plan best = {};
+    const int steps = (K + STEP - 1) / STEP, blocks_n = ceil_div(N, FEATURES);
+    double best_cost = 0;
+    const int widths[5] = {8, 16, 32, 48, 64};
+    for (int wi = 0; wi < 5; ++wi) {
+        const int tn = widths[wi];
+        if (force_tn ? tn != force_tn : (tn < 64 && tn < M && M <= 64)) continue;      // up to 64 tokens: one tile
+        const int tiles_m = ceil_div(M, tn);
+        const long long tiles = (long long)tiles_m * blocks_n;
+        const double step_cost = tn <= 16 ? 350 : tn <= 32 ? 360 : tn <= 48 ? 420 : 520;
+        for (int sp = 1; sp <= 16; ++sp) {
+            if (force_splits ? sp != force_splits : (sp > 1 && (steps / sp < 16 || tiles >= 2 * sms))) continue;
+            const int per = (ceil_div(steps, sp) + 3) / 4 * 4;
+            if ((sp - 1) * per >= steps || tiles * sp > 0x7fffffffll) continue;      // no empty share
+            const double rounds = (double)((tiles * sp + sms - 1) / sms);
+            const double cost = rounds * (per * step_cost + 1500 + 12.0 * tn) + (sp > 1 ? 2500 + 30.0 * tn * (1 + rounds) : 0);
+            if (!best.tn || cost < best_cost) {
+                best_cost = cost;
+                best.tn = tn; best.tiles_m = tiles_m; best.tiles = (int)tiles; best.splits = sp; best.steps_per_split = per;
+            }
+        }
+        if (!force_tn && M <= tn) break;
+    }
+    auto up = [](long long v) { return (v + 255) / 256 * 256; };
+    best.pitch = (K + 15) / 16 * 16;
+    best.planes = 0;
+    best.exps = up(4ll * M * best.pitch);
+    best.counters = best.exps + up(4ll * M);
+    best.partial = best.counters + up(best.splits > 1 ? 4ll * best.tiles : 0);
+    best.bytes = best.partial + (best.splits > 1 ? 8ll * best.splits * best.tiles * best.tn * FEATURES : 0);
+    return best;
+}
+
+template <int TN>
+int launch(const CUtensorMap& mw, const CUtensorMap& mb, const FixedParams& p, cudaStream_t stream) {
+    using L = Layout<TN>;
+    static bool configured_on[PYRE_MAX_DEVICES] = {};      // the attribute is per device
+    bool& configured = configured_on[pyre_current_device()];
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(fixed_gemm_kernel<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+        if (e != cudaSuccess) return (int)e;
+        configured = true;
+    }
+    const int items = p.tiles * p.splits, sms = pyre_sm_count();
+    return (int)pyre_launch(fixed_gemm_kernel<TN>, dim3(items < sms ? items : sms), dim3(THREADS), (size_t)L::TOTAL, stream, mw, mb, p);
+}
+}  // namespace
+
+// The sizes that `pyre_fixed_linear` takes: sums of at most 3 K 2^14 in 32 bits, TMA rows on 16-byte boundaries.
+static bool fixed_ok(const void* w, long long ldw, int K) { return K > 0 && K <= 40960 && ldw % 4 == 0 && !((uintptr_t)w & 15); }
+
+// The exponents of a weight's rows, worked out once: exps[N].
+PYRE_API int pyre_fixed_exponents(const float* w, long long ldw, int N, int K, int* exps, cudaStream_t stream) {
+    if (N <= 0) return 0;
+    if (!fixed_ok(w, ldw, K)) return PYRE_ERR_UNSUPPORTED;
+    const bool vec = K % 4 == 0;
+    const cudaError_t e = pyre_launch(vec ? fixed_rows_kernel<false, true> : fixed_rows_kernel<false, false>, dim3(N), dim3(ROW_THREADS), (size_t)0, stream,
+                                      w, ldw, K, exps, (uint8_t*)nullptr, 0ll, 0, (int*)nullptr, 0);
+    if (e != cudaSuccess) return (int)e;
+    PYRE_LAUNCH_CHECK();
+    return 0;
+}
+
+// Bytes of scratch memory that a product of these sizes needs (256-byte aligned), or -1 (tn and splits: 0 = the plan's own).
+PYRE_API long long pyre_fixed_workspace(int M, int N, int K, int tn, int splits) {
+    if (M <= 0 || N <= 0) return 0;
+    const Plan pl = make_plan(M, N, K, pyre_sm_count(), tn, splits);
+    return pl.tn ? pl.bytes : -1;
+}
+
+PYRE_API int pyre_fixed_linear(const float* A, long long lda, const float* W, long long ldw, const int* w_exp, float* C, long long ldc,
+                               int M, int N, int K, void* workspace, long long workspace_bytes, int tn, int splits, int* err_flag, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (!fixed_ok(W, ldw, K) || ((uintptr_t)workspace & 255)) return PYRE_ERR_UNSUPPORTED;
+    const Plan pl = make_plan(M, N, K, pyre_sm_count(), tn, splits);
+    if (!pl.tn || workspace_bytes < pl.bytes) return PYRE_ERR_BAD_ARG;
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return PYRE_ERR_UNSUPPORTED;
+    uint8_t* ws = (uint8_t*)workspace;
+    CUtensorMap mw, mb;
+    {
+        cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)N};
+        cuuint64_t strides[1] = {(cuuint64_t)ldw * 4};
+        cuuint32_t box[2] = {STEP, FEATURES}, elem[2] = {1, 1};
+        if (fn(&mw, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(W), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return PYRE_ERR_BAD_ARG;
+    }
+    {
+        cuuint64_t dims[3] = {(cuuint64_t)pl.pitch, (cuuint64_t)M, 4};
+        cuuint64_t strides[2] = {(cuuint64_t)pl.pitch, (cuuint64_t)pl.pitch * M};
+        cuuint32_t box[3] = {BLOCK_K, (cuuint32_t)pl.tn, 4}, elem[3] = {1, 1, 1};
+        if (fn(&mb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, ws + pl.planes, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return PYRE_ERR_BAD_ARG;
+    }
+    const bool vec = K % 4 == 0 && lda % 4 == 0 && !((uintptr_t)A & 15);
+    int* a_exp = (int*)(ws + pl.exps);
+    int* counters = (int*)(ws + pl.counters);
+    const cudaError_t e = pyre_launch(vec ? fixed_rows_kernel<true, true> : fixed_rows_kernel<true, false>, dim3(M), dim3(ROW_THREADS), (size_t)0, stream,
+                                      A, lda, K, a_exp, ws + pl.planes, (long long)pl.pitch * M, pl.pitch, counters, pl.splits > 1 ? pl.tiles : 0);
+    if (e != cudaSuccess) return (int)e;
+    FixedParams p = {A, W, w_exp, a_exp, C, lda, ldw, ldc, M, N, K, pl.tiles_m, pl.tiles, pl.splits, pl.steps_per_split,
+                     (long long*)(ws + pl.partial), counters, err_flag};
+    int rc;
+    switch (pl.tn) {
+        case 8: rc = launch<8>(mw, mb, p, stream); break;
+        case 16: rc = launch<16>(mw, mb, p, stream); break;
+        case 32: rc = launch<32>(mw, mb, p, stream); break;
+        case 48: rc = launch<48>(mw, mb, p, stream); break;
+        default: rc = launch<64>(mw, mb, p, stream); break;
+    }
+    if (rc) return rc;
+    PYRE_LAUNCH_CHECK();
+    return 0;
+}

@@ -30,6 +30,7 @@ LIBRARIES = {
     "sampling": "sampling.cu",
     "attention_generic": "attention_generic.cu",
     "gemm_f32": "gemm_f32.cu",
+    "gemm_fixed": "gemm_fixed.cu",
     "attention_mma": "attention_mma.cu",
     "gemm_tc": "gemm_tc.cu",
     "attention_prefill": "attention_prefill.cu",

@@ -40,6 +40,9 @@ SIGNATURES: dict[str, tuple[str, list]] = {
     "pyre_sample_slices": ("sampling", [I]),
     "pyre_paged_attention_generic": ("attention_generic", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, F, F, P, I, LL, P, I, I, P]),
     "pyre_sgemm_nt": ("gemm_f32", [P, LL, P, LL, P, LL, P, I, I, I, P]),
+    "pyre_fixed_exponents": ("gemm_fixed", [P, LL, I, I, P, P]),
+    "pyre_fixed_workspace": ("gemm_fixed", [I, I, I, I, I]),
+    "pyre_fixed_linear": ("gemm_fixed", [P, LL, P, LL, P, P, LL, I, I, I, P, LL, I, I, P, P]),
     "pyre_paged_attention_mma": ("attention_mma", [P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, LL, I, P, P]),
     "pyre_attention_prefill_tc": ("attention_tc", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, LL, I, I, F, F, P, I, I, P, P, P, P]),
     "pyre_attention_prefill": ("attention_prefill", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, LL, P, P]),
@@ -86,6 +89,9 @@ SIGNATURES: dict[str, tuple[str, list]] = {
     "pyre_token_gate_add": ("seqmix", [P, P, P, P, I, I, I, I, P]),
 }
 
+#: functions that return a number of another type than int (sizes; see ``call_value``)
+RESULTS = {"pyre_fixed_workspace": c_longlong}
+
 _ERRORS = {100001: "bad argument", 100002: "unsupported size"}
 
 
@@ -100,7 +106,7 @@ class KernelError(RuntimeError):
 DEFAULT_CLASS = {
     "pyre_embedding": "embed", "pyre_add_rmsnorm": "norm", "pyre_add_residual": "norm", "pyre_rope_table": "rotary+write",
     "pyre_qkv_rope_write": "rotary+write", "pyre_silu_mul": "activation", "pyre_sum_partials": "sum_partials",
-    "pyre_feed_tokens": "feed", "pyre_delay": "delay", "pyre_gemm_tc": "product", "pyre_sgemm_nt": "product", "pyre_scale_rows": "norm", "pyre_sample": "sampler",
+    "pyre_feed_tokens": "feed", "pyre_delay": "delay", "pyre_gemm_tc": "product", "pyre_sgemm_nt": "product", "pyre_fixed_linear": "product", "pyre_scale_rows": "norm", "pyre_sample": "sampler",
     "pyre_paged_attention_generic": "attention", "pyre_paged_attention_mma": "attention",
     "pyre_attention_prefill_tc": "attention", "pyre_attention_prefill": "attention",
     "pyre_cast_rows": "norm", "pyre_norm_add": "norm", "pyre_activation": "activation", "pyre_qk_norm_rope_write": "rotary+write",
@@ -230,7 +236,7 @@ def function(name: str):
         libname, argtypes = SIGNATURES[name]
         fn = getattr(load_library(libname), name)
         fn.argtypes = argtypes
-        fn.restype = c_int
+        fn.restype = RESULTS.get(name, c_int)
         _funcs[name] = fn
     return fn
 

@@ -5,7 +5,7 @@ kernel on torch's current stream.  A size the kernels do not take is refused wit
 clear error; nothing here computes on the CPU or falls back to a library.
 
 The matrix products are the package's own kernels too (``gemm_tc`` on the tcgen05 tensor
-cores for bfloat16, ``sgemm_nt`` for float32).  One case goes to a library (cuBLAS through
+cores for bfloat16, ``fixed_linear`` and ``sgemm_nt`` for float32).  One case goes to a library (cuBLAS through
 ``torch``): a bfloat16 product whose rows are no multiple of 16 bytes, which a TMA copy
 cannot fetch; the reference's engine uses a library for every projection (``nn.Linear``,
 pyre/model.py:84-87,133-135,172).  See ``linear``.
@@ -776,6 +776,75 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, bias: "torch.Tensor | None" = Non
     return out
 
 
+# Rows this long go to the fixed-point product: below, its conversions and its second kernel cost more than the CUDA cores' sums.
+FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_N = 512, 40960, 128
+
+
+class FixedWeight:
+    """A float32 weight [N, K] and the exponent of each row's largest element (int32 [N]), which ``fixed_linear`` puts the
+    row on a fixed-point scale with.  The exponents are worked out once, when a part takes its tensors (``linear_weight``); the weight
+    itself stays as it is and is shared, not copied."""
+
+    def __init__(self, w: torch.Tensor):
+        self.w = w
+        self.exponents = torch.empty(w.shape[0], dtype=torch.int32, device=w.device)
+        with torch.cuda.device(w.device):      # a model may be loaded while another device is current
+            lib.call("pyre_fixed_exponents", w.data_ptr(), w.stride(0), w.shape[0], w.shape[1], self.exponents.data_ptr(), _stream())
+            # products read weights and exponents before they wait for the kernels in front of them (programmatic dependent launch)
+            torch.cuda.current_stream().synchronize()
+
+    @property
+    def shape(self):
+        return self.w.shape
+
+    @property
+    def dtype(self):
+        return self.w.dtype
+
+    @property
+    def device(self):
+        return self.w.device
+
+
+def fixed_supported(w: torch.Tensor) -> bool:
+    """Does ``fixed_linear`` take this weight?  The rule knows the weight alone, never the number of rows that meet it: a row's
+    result is the same in every batch."""
+    return (w.is_cuda and w.dtype == torch.float32 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0
+            and FIXED_MIN_K <= w.shape[1] <= FIXED_MAX_K and w.shape[0] >= FIXED_MIN_N)
+
+
+def linear_weight(w: torch.Tensor) -> "torch.Tensor | FixedWeight":
+    """A weight as ``linear`` wants it: float32 matrices that the fixed-point product takes with their rows' exponents, others as
+    they are."""
+    return FixedWeight(w) if fixed_supported(w) else w
+
+
+def product_libraries(dtype: torch.dtype) -> "list[str]":
+    """The kernel libraries that ``linear`` launches from for weights of ``linear_weight``."""
+    return ["gemm_f32", "gemm_fixed"] if dtype == torch.float32 else ["gemm_tc"]
+
+
+def fixed_linear(a: torch.Tensor, w: FixedWeight, plan: "tuple[int, int]" = (0, 0)) -> torch.Tensor:
+    """C = A W^T of float32 operands on the tensor cores in fixed point: rows on power-of-two scales, integers of 31 bits as
+    four bytes, exact sums, one rounding (csrc/gemm_fixed.cu).  A row's result is bit-identical for any number of rows.
+    ``plan``: (tokens per tile, shares of K), 0 for the kernel's own choice."""
+    if not a.is_cuda or a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1:
+        raise ValueError("a must be a CUDA float32 matrix with contiguous rows")
+    require_current_device(a.device, "a")
+    M, K = a.shape
+    N, K2 = w.shape
+    if K != K2:
+        raise ValueError(f"inner sizes differ: a is [{M}, {K}], w is [{N}, {K2}]")
+    out = torch.empty((M, N), dtype=torch.float32, device=a.device)
+    size = lib.call_value("pyre_fixed_workspace", M, N, K, plan[0], plan[1])
+    if size < 0:
+        raise UnsupportedSize(f"no plan {plan} for a product of {M} rows")
+    work = torch.empty(size, dtype=torch.uint8, device=a.device)
+    lib.call("pyre_fixed_linear", a.data_ptr(), a.stride(0), w.w.data_ptr(), w.w.stride(0), w.exponents.data_ptr(), out.data_ptr(), out.stride(0),
+             M, N, K, work.data_ptr(), size, plan[0], plan[1], device_error_flag(a.device).data_ptr(), _stream())
+    return out
+
+
 _error_flags: dict = {}
 
 
@@ -1134,7 +1203,7 @@ def linear(x: "torch.Tensor | ScaledRows", w: torch.Tensor, out_dtype: "torch.dt
            deferred_ok: "bool | str | tuple" = False):
     """y = x W^T for a weight in the linear-layer layout [out, in].
 
-    float32: the package's own fp32 kernel (no reduced-precision matrix mode).
+    float32: the package's own kernels: ``fixed_linear`` for a weight of ``linear_weight`` that it takes, else ``sgemm_nt``.
     bfloat16: the package's tcgen05 kernel (``gemm_tc``); rows that are no 16-byte multiple
     (K not a multiple of 8) go to a library product instead, as the reference uses a library
     for every projection.  ``out_dtype=torch.float32`` keeps the accumulator's precision
@@ -1147,7 +1216,7 @@ def linear(x: "torch.Tensor | ScaledRows", w: torch.Tensor, out_dtype: "torch.dt
     ``deferred_ok=("rope", head_dim)``: the consumer is a position encoding that may fold bias, rotation and the cache
     write into the stacked q/k/v product (``folds_rope``)."""
     if x.dtype == torch.float32:
-        return sgemm_nt(x, w)
+        return fixed_linear(x, w) if isinstance(w, FixedWeight) else sgemm_nt(x, w)
     if x.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:
         raise ValueError(f"linear: unsupported dtypes {x.dtype} x {w.dtype}")
     rows = x.rows if isinstance(x, ScaledRows) else x

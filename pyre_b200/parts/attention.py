@@ -184,17 +184,17 @@ class Attention(StackedMixer):
             if self.learned_sink:
                 self.sink = tensors[n["sink"]]
             return
-        self.w_qkv = torch.cat([tensors[f"{n[k]}.weight"] for k in "qkv"], dim=0).contiguous()
+        self.w_qkv = ops.linear_weight(torch.cat([tensors[f"{n[k]}.weight"] for k in "qkv"], dim=0).contiguous())
         if self.qkv_bias:
             self.b_qkv = torch.cat([tensors[f"{n[k]}.bias"] for k in "qkv"]).contiguous()
-        self.w_o = tensors[f"{n['o']}.weight"]
+        self.w_o = ops.linear_weight(tensors[f"{n['o']}.weight"])
 
     def kernel_libraries(self):
         libs = ["elementwise"]      # the position encoding, a sub-part, names its own
         if self.general:
             libs.append("blockops")
         libs += attention_libraries(self.dtype, self.row_dim)
-        libs.append("gemm_f32" if self.dtype == torch.float32 else "gemm_tc")
+        libs += ops.product_libraries(self.dtype)
         return libs
 
     def cache_spec(self):

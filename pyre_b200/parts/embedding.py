@@ -66,10 +66,10 @@ class LinearHead(Part):
         return {self.tensor_name: TensorSpec((self.vocab, self.width), optional_alias=self.tied_to)}
 
     def load(self, tensors):
-        self.weight = tensors[self.tensor_name]
+        self.weight = ops.linear_weight(tensors[self.tensor_name])
 
     def kernel_libraries(self):
-        return (["gemm_f32"] if self.dtype == torch.float32 else ["gemm_tc"]) + (["seqmix"] if self._shaped() else [])
+        return ops.product_libraries(self.dtype) + (["seqmix"] if self._shaped() else [])
 
     def _shaped(self) -> bool:
         return self.logit_scale != 1.0 or self.softcap > 0.0

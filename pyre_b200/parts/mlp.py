@@ -70,12 +70,12 @@ class GatedMLP(Part):
         if self.interleaved:
             self.w_gate_up = ops.interleave_gate_up(gate, up)
         else:
-            self.w_gate_up = torch.cat([gate, up], dim=0).contiguous()
-        self.w_down = tensors[n["down"] + sfx]
+            self.w_gate_up = ops.linear_weight(torch.cat([gate, up], dim=0).contiguous())
+        self.w_down = ops.linear_weight(tensors[n["down"] + sfx])
 
     def kernel_libraries(self):
         return ["elementwise"] + (["parallel_block"] if not self.in_product else []) + \
-            (["gemm_f32"] if self.dtype == torch.float32 else ["gemm_tc"])
+            ops.product_libraries(self.dtype)
 
     def forward(self, ctx, h):
         with lib.section("gate_up"):
@@ -120,12 +120,12 @@ class DenseMLP(Part):
         return t
 
     def load(self, tensors):
-        self.w_up, self.w_down = tensors[self.names["up"]], tensors[self.names["down"]]
+        self.w_up, self.w_down = (ops.linear_weight(tensors[self.names[t]]) for t in ("up", "down"))
         if self.bias:
             self.b_up, self.b_down = tensors[self.names["up_bias"]], tensors[self.names["down_bias"]]
 
     def kernel_libraries(self):
-        return ["blockops", "elementwise"] + (["gemm_f32"] if self.dtype == torch.float32 else ["gemm_tc"])
+        return ["blockops", "elementwise"] + ops.product_libraries(self.dtype)
 
     def forward(self, ctx, h):
         with lib.section("up"):

@@ -1,0 +1,99 @@
+"""The fixed-point product of float32 operands against an evaluation in 64 bits: tile edges in every dimension, every tile
+width and split of K with the same bits, rows of any scale, rows that hold infinities or NaNs."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from pyre_b200.kernels import build, ops
+    build.ensure_built(["gemm_fixed", "gemm_f32"])
+    return ops
+
+
+def bound(a, w, c):
+    """One rounding to float; half a unit of 2^-29 of a row's leading power of two per factor; the products of byte planes 2 x 3, 3 x 2 and
+    3 x 3 that are left out (K terms of at most 2^15 2^8 and 2^14 units of 2^-58)."""
+    a, w = a.double(), w.double()
+    ta, tw = a.abs().amax(1, keepdim=True), w.abs().amax(1, keepdim=True).t()
+    steps = 2.0 ** -30 * (ta * w.abs().sum(1)[None] + a.abs().sum(1, keepdim=True) * tw)
+    return 2.0 ** -24 * c.abs() + steps + 2.0 ** -34 * a.shape[1] * ta * tw + 2.0 ** -149
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (7, 129, 516), (8, 1000, 640), (9, 300, 2052), (17, 128, 3584), (33, 255, 544), (65, 384, 1000),
+                                   (130, 777, 900), (200, 256, 18944), (3, 3584, 40960)])
+def test_against_64_bits(ops, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a = torch.randn(M, K, device="cuda", generator=g) * torch.exp2(torch.randint(-30, 30, (M, 1), device="cuda", generator=g))
+    w = torch.randn(N, K, device="cuda", generator=g) * torch.exp2(torch.randint(-20, 20, (N, 1), device="cuda", generator=g))
+    a[M // 2, :] = 0
+    w[N // 2, ::3] *= 1e-3
+    W = ops.FixedWeight(w)
+    got = ops.fixed_linear(a, W)
+    ops.check_device_errors()
+    want = a.double() @ w.double().t()
+    assert ((got.double() - want).abs() <= bound(a, w, want)).all()
+    # whatever the tile, the split of K and the rows beside it: the same bits; rows off 16-byte boundaries too
+    for tn, shares in [(8, 1), (16, 2), (32, 3), (48, 1), (64, 4)]:
+        steps = -(-K // 32)
+        if (shares - 1) * (-(-(-(-steps // shares)) // 4) * 4) >= steps:
+            continue      # fewer shares than that: none may be empty
+        assert torch.equal(ops.fixed_linear(a, W, (tn, shares)), got), (tn, shares)
+    odd = torch.empty(M, K + 1, device="cuda")
+    odd[:, :K] = a
+    assert torch.equal(ops.fixed_linear(odd[:, :K], W), got)
+    for r in {0, M // 2, M - 1}:
+        assert torch.equal(ops.fixed_linear(a[r:r + 1], W), got[r:r + 1])
+    ops.check_device_errors()
+
+
+def test_rows_of_any_scale(ops):
+    """Outliers, the smallest and the largest numbers: within the bound, and infinite where the result is."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a, w = torch.randn(12, 1024, device="cuda", generator=g), torch.randn(256, 1024, device="cuda", generator=g)
+    a[0, 5] = 3e3
+    a[1] *= 1e-38
+    a[2] *= 1e-44
+    a[3] *= 1e37
+    a[4, ::2] *= 1e-6
+    w[0] *= 1e-38
+    w[1] *= 1e30
+    w[2, 7] = 1e6
+    w[3] = 0
+    got, want = ops.fixed_linear(a, ops.FixedWeight(w)).double(), a.double() @ w.double().t()
+    fits = want.abs() < 3.4e38
+    assert (((got - want).abs() <= bound(a, w, want)) | ~fits).all()
+    assert torch.isinf(got[~fits]).all()
+
+
+def test_infinities_and_nans(ops):
+    """Rows without a scale give what an IEEE sum gives; the rows and features beside them keep their bits."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    a, w = torch.randn(20, 700, device="cuda", generator=g), torch.randn(256, 700, device="cuda", generator=g)
+    clean = ops.fixed_linear(a, ops.FixedWeight(w))
+    inf = float("inf")
+    a[3, 5], a[4, 6], a[5, 7], a[5, 9], a[6, 11] = inf, float("nan"), -inf, inf, inf
+    w[10, 11], w[12, 13], w[20, 5] = inf, float("nan"), 0
+    for plan in [(0, 0), (32, 2)]:
+        got, want = ops.fixed_linear(a, ops.FixedWeight(w), plan), ops.sgemm_nt(a, w)
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+        assert torch.equal(got[torch.isinf(got)], want[torch.isinf(want)])
+        rows = [r for r in range(20) if r not in (3, 4, 5, 6)]
+        cols = [c for c in range(256) if c not in (10, 12, 20)]
+        assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
+
+
+def test_which_weights_take_it(ops):
+    """The rule knows the weight alone: short rows, few features and rows off 16-byte boundaries stay with the CUDA cores' product."""
+    def weight(N, K, ld=0):
+        return torch.zeros(N, ld or K, device="cuda")[:, :K]
+    assert isinstance(ops.linear_weight(weight(128, 512)), ops.FixedWeight)
+    for w in (weight(128, 508), weight(127, 512), weight(128, 600, 601), weight(128, 512).to(torch.bfloat16), weight(128, 40964)):
+        assert ops.linear_weight(w) is w
+    W = ops.linear_weight(weight(128, 512))
+    with pytest.raises(ValueError):
+        ops.fixed_linear(torch.zeros(2, 516, device="cuda"), W)
+    assert ops.linear(torch.zeros(2, 512, device="cuda"), W).shape == (2, 128)
