@@ -555,7 +555,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             };
             if constexpr (!X_CONTIGUOUS_OUT && BN == 256) {
                 if (p.gated) {
-                    const bool live_row = xr < p.x_rows;
+                    // Rows beyond the tokens are all zeros, and silu's 0 / 2 takes the division's slow path: one such warp held its whole
+                    // tile up (500 x 37888 x 3584: 157 us against 105 for 512 rows, 107 so).
                     // the tile's columns are two blocks of 64 gate features followed by the 64 up features of the
                     // same indices: out[x, y0 / 2 + c] = silu(gate) * up, with the products rounded to bfloat16
                     // first (as a separate activation kernel would read them) and the rest in fp32
@@ -570,6 +571,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                             tmem_ld16(acc + blk * 128 + cc, g);
                             tmem_ld16(acc + blk * 128 + 64 + cc, u);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            if (xr >= p.x_rows) {
+#pragma unroll
+                                for (int q = 0; q < 16; ++q) g[q] = __float_as_uint(1.f);
+                            }
 #pragma unroll
                             for (int q = 0; q < 8; ++q) {
                                 float o[2];
@@ -577,9 +582,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                                 for (int e = 0; e < 2; ++e) {
                                     const float z = __bfloat162float(__float2bfloat16_rn(__uint_as_float(g[2 * q + e]) * row_scale));
                                     const float v = __bfloat162float(__float2bfloat16_rn(__uint_as_float(u[2 * q + e]) * row_scale));
-                                    // (a row beyond the tokens is all zeros, and 0 / 2 takes the division's slow path: it held the whole tile
-                                    // up, 500 x 37888 x 3584 157 us against 105 for 512 rows)
-                                    o[e] = gated_value(live_row ? z : 1.f, v, p.gated, p.gate_limit);
+                                    o[e] = gated_value(z, v, p.gated, p.gate_limit);
                                 }
                                 __nv_bfloat162 pr = __floats2bfloat162_rn(o[0], o[1]);
                                 w[cc / 2 + q] = *reinterpret_cast<uint32_t*>(&pr);
