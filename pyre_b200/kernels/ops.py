@@ -776,14 +776,16 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, bias: "torch.Tensor | None" = Non
     return out
 
 
-# Rows this long go to the fixed-point product: below, its conversions and its second kernel cost more than the CUDA cores' sums.
-FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_N = 512, 40960, 128
+# Weights this large go to the fixed-point product.  Its second kernel and the shares of K cost a few rows some 4 us, which weights of
+# 33 MB and more win back with the rows of a prompt or, from a hundred megabytes on, with their stream (us, CUDA cores / fixed
+# point: 4 x 4608 x 3584 15.7 / 19.8, 64 rows 81 / 34; 4 x 3584 x 3584 15.0 / 17.2, 64 rows 64 / 35; 4 x 37888 x 3584 118 / 95).
+FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_N, FIXED_MIN_SIZE = 512, 40960, 128, 1 << 23
 
 
 class FixedWeight:
     """A float32 weight [N, K] and the exponent of each row's largest element (int32 [N]), which ``fixed_linear`` puts the
     row on a fixed-point scale with.  The exponents are worked out once, when a part takes its tensors (``linear_weight``); the weight
-    itself stays as it is and is shared, not copied."""
+    itself stays as it is and is shared, not copied; one that is changed in place needs a new ``FixedWeight``."""
 
     def __init__(self, w: torch.Tensor):
         self.w = w
@@ -810,7 +812,7 @@ def fixed_supported(w: torch.Tensor) -> bool:
     """Does ``fixed_linear`` take this weight?  The rule knows the weight alone, never the number of rows that meet it: a row's
     result is the same in every batch."""
     return (w.is_cuda and w.dtype == torch.float32 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0
-            and FIXED_MIN_K <= w.shape[1] <= FIXED_MAX_K and w.shape[0] >= FIXED_MIN_N)
+            and FIXED_MIN_K <= w.shape[1] <= FIXED_MAX_K and w.shape[0] >= FIXED_MIN_N and w.numel() >= FIXED_MIN_SIZE)
 
 
 def linear_weight(w: torch.Tensor) -> "torch.Tensor | FixedWeight":

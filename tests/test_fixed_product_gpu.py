@@ -87,13 +87,14 @@ def test_infinities_and_nans(ops):
 
 
 def test_which_weights_take_it(ops):
-    """The rule knows the weight alone: short rows, few features and rows off 16-byte boundaries stay with the CUDA cores' product."""
+    """The rule knows the weight alone: small ones, short rows, few features and rows off 16-byte boundaries stay with the CUDA cores'
+    product."""
     def weight(N, K, ld=0):
         return torch.zeros(N, ld or K, device="cuda")[:, :K]
-    assert isinstance(ops.linear_weight(weight(128, 512)), ops.FixedWeight)
-    for w in (weight(128, 508), weight(127, 512), weight(128, 600, 601), weight(128, 512).to(torch.bfloat16), weight(128, 40964)):
+    assert isinstance(ops.linear_weight(weight(16384, 512)), ops.FixedWeight)
+    for w in (weight(16383, 512), weight(16600, 508), weight(127, 40960 * 2), weight(16384, 600, 601), weight(16384, 512).to(torch.bfloat16), weight(300, 40964)):
         assert ops.linear_weight(w) is w
-    W = ops.linear_weight(weight(128, 512))
+    W = ops.FixedWeight(weight(128, 512))
     with pytest.raises(ValueError):
         ops.fixed_linear(torch.zeros(2, 516, device="cuda"), W)
     assert ops.linear(torch.zeros(2, 512, device="cuda"), W).shape == (2, 128)
