@@ -424,10 +424,11 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
 }
 
-// A row's exponent, and (PLANES) its elements as four byte planes [4][rows][pitch].  A block per row, which it reads twice (the second time
-// out of the caches).
-constexpr int ROW_THREADS = 256;
-template <bool PLANES, bool VEC>
+// A row's exponent, and (PLANES) its elements as four byte planes [4][rows][pitch].  A block per row; what bounds it is the chain of
+// its latencies, so a thread asks for HELD pieces of four elements at once and keeps them (what a longer row has beyond them is read a second
+// time, out of the caches).
+constexpr int ROW_THREADS = 512;
+template <bool PLANES, bool VEC, int HELD>
 __global__ void __launch_bounds__(ROW_THREADS)
 fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* planes, long long plane_stride, int pitch, int* counters, int n_counters) {
     __shared__ uint32_t s_max[ROW_THREADS / 32];
@@ -437,17 +438,26 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* plan
     const float* a = A + (size_t)blockIdx.x * lda;
     if (PLANES)
         for (int i = blockIdx.x * ROW_THREADS + tid; i < n_counters; i += gridDim.x * ROW_THREADS) counters[i] = 0;
+    auto piece = [&](int k) {      // the four elements from k on, zeros beyond the row
+        if (VEC) return k < K ? *reinterpret_cast<const float4*>(a + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 v;
+        v.x = k < K ? a[k] : 0.f;
+        v.y = k + 1 < K ? a[k + 1] : 0.f;
+        v.z = k + 2 < K ? a[k + 2] : 0.f;
+        v.w = k + 3 < K ? a[k + 3] : 0.f;
+        return v;
+    };
     uint32_t most = 0;
-    if constexpr (VEC) {
-#pragma unroll 4
-        for (int k = 4 * tid; k < K; k += 4 * ROW_THREADS) {
-            const uint4 v = *reinterpret_cast<const uint4*>(a + k);
-            most = max(max(max(most, v.x & 0x7fffffffu), max(v.y & 0x7fffffffu, v.z & 0x7fffffffu)), v.w & 0x7fffffffu);
-        }
-    } else {
-#pragma unroll 4
-        for (int k = tid; k < K; k += ROW_THREADS) most = max(most, __float_as_uint(a[k]) & 0x7fffffffu);
-    }
+    auto look = [&](const float4& v) {
+        most = max(max(most, __float_as_uint(v.x) & 0x7fffffffu), max(__float_as_uint(v.y) & 0x7fffffffu, __float_as_uint(v.z) & 0x7fffffffu));
+        most = max(most, __float_as_uint(v.w) & 0x7fffffffu);
+    };
+    float4 held[HELD];
+#pragma unroll
+    for (int h = 0; h < HELD; ++h) held[h] = piece(4 * (tid + h * ROW_THREADS));
+#pragma unroll
+    for (int h = 0; h < HELD; ++h) look(held[h]);
+    for (int k = 4 * (tid + HELD * ROW_THREADS); k < K; k += 4 * ROW_THREADS) look(piece(k));
     most = __reduce_max_sync(0xffffffffu, most);
     if ((tid & 31) == 0) s_max[tid >> 5] = most;
     __syncthreads();
@@ -457,24 +467,21 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* plan
     if (tid == 0) exps[blockIdx.x] = E;
     if constexpr (PLANES) {
         const RowScale sc = row_scale(E);
+        const bool none = E >= E_INF;
         uint8_t* out = planes + (size_t)blockIdx.x * pitch;
-#pragma unroll 2
-        for (int k = 4 * tid; k < pitch; k += 4 * ROW_THREADS) {
-            float x[4];
-            if (VEC && k < K) {
-                const float4 v = *reinterpret_cast<const float4*>(a + k);
-                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) x[e] = k + e < K ? a[k + e] : 0.f;
-            }
-#pragma unroll
-            for (int e = 0; e < 4; ++e) x[e] = E >= E_INF ? 0.f : x[e] * sc.s2 * sc.s1;
+        auto put = [&](int k, const float4& v) {
             uint32_t w[4];
-            bytes_of(x[0], x[1], x[2], x[3], w[0], w[1], w[2], w[3]);
+            bytes_of(none ? 0.f : v.x * sc.s2 * sc.s1, none ? 0.f : v.y * sc.s2 * sc.s1, none ? 0.f : v.z * sc.s2 * sc.s1, none ? 0.f : v.w * sc.s2 * sc.s1,
+                     w[0], w[1], w[2], w[3]);
 #pragma unroll
             for (int q = 0; q < 4; ++q) *reinterpret_cast<uint32_t*>(out + q * plane_stride + k) = w[q];
+        };
+#pragma unroll
+        for (int h = 0; h < HELD; ++h) {
+            const int k = 4 * (tid + h * ROW_THREADS);
+            if (k < pitch) put(k, held[h]);
         }
+        for (int k = 4 * (tid + HELD * ROW_THREADS); k < pitch; k += 4 * ROW_THREADS) put(k, piece(k));
     }
 }
 
@@ -545,6 +552,16 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mb, const FixedParams& p, c
     const int items = p.tiles * p.splits, sms = pyre_sm_count();
     return (int)pyre_launch(fixed_gemm_kernel<TN>, dim3(items < sms ? items : sms), dim3(THREADS), (size_t)L::TOTAL, stream, mw, mb, p);
 }
+
+// Rows of up to 4,096 elements hold two pieces a thread (three blocks fit on an SM), longer ones ten.
+template <bool PLANES>
+cudaError_t launch_rows(bool vec, const float* a, long long lda, int rows, int K, int* exps, uint8_t* planes, long long plane_stride, int pitch,
+                        int* counters, int n_counters, cudaStream_t stream) {
+    const bool brief = K <= 2 * 4 * ROW_THREADS;
+    auto kernel = vec ? (brief ? fixed_rows_kernel<PLANES, true, 2> : fixed_rows_kernel<PLANES, true, 10>)
+                      : (brief ? fixed_rows_kernel<PLANES, false, 2> : fixed_rows_kernel<PLANES, false, 10>);
+    return pyre_launch(kernel, dim3(rows), dim3(ROW_THREADS), (size_t)0, stream, a, lda, K, exps, planes, plane_stride, pitch, counters, n_counters);
+}
 }  // namespace
 
 // The sizes that `pyre_fixed_linear` takes: sums of at most 3 K 2^14 in 32 bits, TMA rows on 16-byte boundaries.
@@ -554,9 +571,7 @@ static bool fixed_ok(const void* w, long long ldw, int K) { return K > 0 && K <=
 PYRE_API int pyre_fixed_exponents(const float* w, long long ldw, int N, int K, int* exps, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (!fixed_ok(w, ldw, K)) return PYRE_ERR_UNSUPPORTED;
-    const bool vec = K % 4 == 0;
-    const cudaError_t e = pyre_launch(vec ? fixed_rows_kernel<false, true> : fixed_rows_kernel<false, false>, dim3(N), dim3(ROW_THREADS), (size_t)0, stream,
-                                      w, ldw, K, exps, (uint8_t*)nullptr, 0ll, 0, (int*)nullptr, 0);
+    const cudaError_t e = launch_rows<false>(K % 4 == 0, w, ldw, N, K, exps, nullptr, 0, 0, nullptr, 0, stream);
     if (e != cudaSuccess) return (int)e;
     PYRE_LAUNCH_CHECK();
     return 0;
@@ -596,8 +611,7 @@ PYRE_API int pyre_fixed_linear(const float* A, long long lda, const float* W, lo
     const bool vec = K % 4 == 0 && lda % 4 == 0 && !((uintptr_t)A & 15);
     int* a_exp = (int*)(ws + pl.exps);
     int* counters = (int*)(ws + pl.counters);
-    const cudaError_t e = pyre_launch(vec ? fixed_rows_kernel<true, true> : fixed_rows_kernel<true, false>, dim3(M), dim3(ROW_THREADS), (size_t)0, stream,
-                                      A, lda, K, a_exp, ws + pl.planes, (long long)pl.pitch * M, pl.pitch, counters, pl.splits > 1 ? pl.tiles : 0);
+    const cudaError_t e = launch_rows<true>(vec, A, lda, M, K, a_exp, ws + pl.planes, (long long)pl.pitch * M, pl.pitch, counters, pl.splits > 1 ? pl.tiles : 0, stream);
     if (e != cudaSuccess) return (int)e;
     FixedParams p = {A, W, w_exp, a_exp, C, lda, ldw, ldc, M, N, K, pl.tiles_m, pl.tiles, pl.splits, pl.steps_per_split,
                      (long long*)(ws + pl.partial), counters, err_flag};
