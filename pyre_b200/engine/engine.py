@@ -83,7 +83,7 @@ class Engine:
                                    self.max_model_len, admit_whole_prompts=ec.admit_whole_prompts)
         self.sampler = Sampler(ec.device)
         self._requests: dict[int, Request] = {}
-        self._flight = None      # (plan, sampling ticket, error word) of the step whose ids have not been read yet
+        self._flight = None      # (plan, sampling ticket, error word, kept logits) of the step whose ids have not been read yet
         pinned = self.model.device.type == "cuda"
         self._err_host = [torch.zeros(1, dtype=torch.int32, pin_memory=pinned) for _ in range(2)]
         self._err_turn = 0
@@ -173,16 +173,11 @@ class Engine:
                 self._err_turn ^= 1
                 err.copy_(self.stepper.error_flag, non_blocking=True)
                 sampling = [s for s in plan if s.samples]
-                keep = [k for k, s in enumerate(sampling) if s.request.params.return_logits]
-                if keep:
-                    # only requests that ask for their logits pay for this copy (and for the wait it brings)
-                    rows = logits[keep].to("cpu").numpy()
-                    for k, row in zip(keep, rows):
-                        sampling[k].request.logits[len(sampling[k].request.generated)] = row
+                kept = self._copy_logits(logits, sampling)
                 ticket = self.sampler.sample_async(logits, [s.request.params for s in sampling],
                                                    [len(s.request.generated) for s in sampling]) if sampling else None
             sched.launched(plan)
-            flight = (plan, ticket, err)
+            flight = (plan, ticket, err, kept)
         if self._flight is not None:
             self._land(self._flight)
         self._flight = flight
@@ -214,14 +209,36 @@ class Engine:
             outs.append(RequestOutput(r.seq_id, r.prompt_ids, list(r.generated), r.finish_reason or "", r.preemptions, kept))
         return outs
 
+    _logits_last = _logits_spare = None      # pinned memory for kept logits: of the latest step that had some, of the one before it
+
+    def _copy_logits(self, logits: torch.Tensor, sampling) -> "tuple | None":
+        """Start the copy of the rows that requests keep (only those that ask for their logits pay for it) to one of two pinned
+        buffers (two steps are open at a time): (host rows, [(request, index of the token they choose)]).  The rows are there once
+        the step's ids are."""
+        keep = [k for k, s in enumerate(sampling) if s.request.params.return_logits]
+        if not keep:
+            return None
+        rows = logits[:len(sampling)] if len(keep) == len(sampling) else logits[keep]
+        buffer, self._logits_spare = self._logits_spare, self._logits_last
+        if buffer is None or buffer.numel() < rows.numel():
+            buffer = torch.empty(rows.numel(), dtype=rows.dtype, pin_memory=rows.is_cuda)
+        self._logits_last = buffer
+        host = buffer[:rows.numel()].view(rows.shape)
+        host.copy_(rows, non_blocking=True)
+        return host, [(sampling[k].request, len(sampling[k].request.generated)) for k in keep]
+
     def _land(self, flight) -> None:
         """Read the ids of a started step and let the scheduler record them."""
-        plan, ticket, err = flight
+        plan, ticket, err, kept = flight
         t_wait = time.perf_counter()
         ids = self.sampler.read(ticket) if ticket is not None else []
         self._waited += time.perf_counter() - t_wait      # the host had nothing left to do but wait for the GPU
         if ticket is not None and int(err[0]) != 0:
             self.stepper.check_device_errors()      # raises with the kernel's reason
+        if kept is not None:
+            host, places = kept
+            for row, (request, index) in zip(host.numpy().copy(), places):      # the buffer is the next but one step's
+                request.logits[index] = row
         self.scheduler.resolve(plan, ids)
 
     def has_unfinished(self) -> bool:
