@@ -943,33 +943,21 @@ def _tc_gemm_plan(M: int, N: int, K: int, _SM_COUNT: int, pair: bool) -> tuple[b
         if cand > 128 and N < cand:
             continue
         cols = -(-N // cand)
-        if pair:
-            # An SM of a pair pulls 128 (128 + bn / 2) bytes per K block at some 95 GB/s whoever else loads, and a block takes no less
-            # than 0.32 us.  Measured (7B, 14B and 32B shapes, 256 to 2,322 tokens; us by this rule / by the latency and rate of
-            # 18 TB/s, which chose otherwise): 500 x 3584 x 3584 16.5 (208 wide, K in two) / 22.7 (128), 500 x 4608 x 3584 18.3 / 23.3,
-            # 1500 x 3584 x 18944 163 / 186, 500 x 5120 x 13824 62 / 74, 500 x 5120 x 27648 111 / 143, 1040 x 5120 x 27648 251 / 281.
-            per_block = max(0.32, 128 * (128 + cand / 2) / 95e3)
-        else:
-            per_block = max(cand * 2 / 1900.0, latency / (stages - 1))
-        nbytes = (128 + cand) * 128       # one K block of both operands, per worker
+        nbytes = ((256 + cand) if pair else (128 + cand)) * 128       # one K block of both operands, per worker
+        per_block = max(cand * 2 / 1900.0, latency / (stages - 1))
         for sp in (1, 2, 3, 4):
             if sp > 1 and kb // sp < 8:
                 break
             items = rows * cols * sp
             per_worker = -(-items // workers)
             blocks = -(-kb // sp)
-            cost = per_worker * blocks * per_block
-            if not pair:
-                cost = max(cost, items * blocks * nbytes / 18e6)
-            cost += per_worker * (1.5 + cand / 64.0 * (2 if sp > 1 else 1))
-            if pair and sp > 1:
-                # whoever takes the partial sums reads them again, in a kernel that costs some 4 us less than what a whole product folds in
-                cost += max(0.0, sp * M * N * 4 / 5e6 - 4.0)
-            # near-ties go to the wider tile; a split K (fp32 partials, estimated less surely) has to gain something
+            cost = max(per_worker * blocks * per_block, items * blocks * nbytes / 18e6) \
+                + per_worker * (1.5 + cand / 64.0 * (2 if sp > 1 else 1))
+            # near-ties go to the wider tile; a split K (fp32 partials, estimated less surely) has to gain a tenth
             if best[sp > 1] is None or cost < best[sp > 1][0] * 0.98:
                 best[sp > 1] = (cost, cand, sp)
     whole, split = best
-    if split is not None and split[0] < (0.95 if pair else 0.9) * whole[0]:
+    if split is not None and split[0] < 0.9 * whole[0]:
         return False, split[1], split[2]
     return False, whole[1], whole[2]
 

@@ -126,15 +126,3 @@ def test_latent_attention_shares():
     assert ops.latent_attention_splits(64, 64, 256, 100, 320) == 1       # 27.2 so, 30.1 with two: 4,096 rows make the trip through memory
     assert ops.latent_attention_splits(24, 72, 128, 100, 160) == 1       # 17.4 so, 18.6 with two
     assert ops.latent_attention_splits(32, 128, 512, 70, 576) == 1       # 31.3 so, 34.0 with two
-
-
-def test_measured_splits_of_prompt_products(monkeypatch):
-    """Products of 300 to 1,500 tokens whose best plan was measured: few tiles of a long K go in shares, full rounds stay whole."""
-    monkeypatch.setattr(ops, "CTA_PAIRS", True)
-    assert ops.tc_gemm_plan(500, 4608, 3584) == (False, 256, 2)          # 18.3 us; whole, 128 wide: 23.3
-    assert ops.tc_gemm_plan(500, 3584, 3584)[2] == 2                     # 16.5; 22.7
-    assert ops.tc_gemm_plan(500, 5120, 27648) == (False, 224, 3)         # 111; 208 wide: 143
-    assert ops.tc_gemm_plan(1040, 5120, 27648) == (False, 256, 2)        # 251; 281
-    assert ops.tc_gemm_plan(700, 3584, 18944) == (False, 224, 3)         # 80; 98
-    assert ops.tc_gemm_plan(1040, 3584, 18944) == (False, 256, 1)        # 112; in two shares 120
-    assert ops.tc_gemm_plan(2322, 5120, 13824) == (False, 256, 1)        # 243; 273
