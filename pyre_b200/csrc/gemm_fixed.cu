@@ -164,7 +164,11 @@ struct FixedParams {
 };
 
 template <int TN> struct Layout {
-    static constexpr int W_STAGES = TN <= 16 ? 12 : TN <= 48 ? 9 : 8;
+    // The groups of converting warps take a ring's steps in turn, and a wait by parity cannot tell a phase from the one two before it.  With a
+    // multiple of GROUPS stages a stage is always the same group's, which has waited for its last phase itself; with nine, a load that came
+    // late let the next group read the stage ahead of it.  (Tensor memory's A_STAGES: a group's wait at step - 4 has shown that the
+    // MMAs of step - 4 - A_STAGES are done, so those of step - 2 A_STAGES are.)
+    static constexpr int W_STAGES = TN <= 16 ? 12 : 8;
     static constexpr int B_BYTES = 4 * TN * BLOCK_K, B_STAGES = TN <= 16 ? 4 : 3;
     static constexpr int W_OFF = 0, B_OFF = W_STAGES * W_BYTES, BARS = B_OFF + B_STAGES * B_BYTES;
     static constexpr int N_BARS = 2 * W_STAGES + 2 * B_STAGES + 2 * A_STAGES + 2;
@@ -172,6 +176,7 @@ template <int TN> struct Layout {
     // an MMA of M = 128 takes N in sixteens: with eight tokens the third plane's product is one plane wider (its last sum is not read)
     static constexpr int SUMS = TN == 8 ? 6 : 5;
     static constexpr int A_COL0 = 512 - A_STAGES * A_COLS;
+    static_assert(W_STAGES % GROUPS == 0 && A_STAGES >= GROUPS, "a stage belongs to one group; see above");
     static_assert(TOTAL <= 232448 && SUMS * TN <= A_COL0 && (TN == 8 || TN % 16 == 0), "fits");
 };
 
