@@ -12,8 +12,8 @@
 //
 // Integers add up in any order: a row's result has the same bits for any M, tile, split of K or order of arrival.
 //
-// A row with an infinity or a NaN has no scale.  Its outputs are worked out from the float operands: NaN if the row holds
-// one, else the sum over the infinite elements, which is what an IEEE sum over all of them gives.
+// A row with an infinity or a NaN has no scale.  Its outputs are sums of the float operands in double precision, a warp per feature,
+// after the CTA's last tile: nothing waits for them under a bounded wait.
 //
 // Two kernels: the activations' exponents and byte planes (they are few), then the product.  The product's CTA (640 threads)
 // owns 128 output features (the weights on the MMA's rows) and TN tokens, K in steps of 32:
@@ -33,7 +33,7 @@
 
 namespace {
 constexpr int ERR_TIMEOUT = 2;
-constexpr int E_NAN = 2000, E_INF = 1000;      // exponents of rows without a scale: a NaN, an infinity
+constexpr int E_NONE = 1000;                   // of a row without a scale
 constexpr int E_MIN = -98;                     // of a row of zeros (its scale is a normal float)
 constexpr int FEATURES = 128, STEP = 32, BLOCK_K = 128;
 constexpr int CONV_WARP0 = 4, GROUPS = 4, CONV_THREADS = GROUPS * 128, THREADS = CONV_WARP0 * 32 + CONV_THREADS;
@@ -107,7 +107,7 @@ __device__ __forceinline__ float pow2f(int e) { return __uint_as_float((uint32_t
 
 // The exponent of a row from the largest |x| of its elements as bits (NaN above infinity above all numbers).
 __device__ __forceinline__ int row_exponent(uint32_t abs_bits) {
-    if (abs_bits >= 0x7f800000u) return abs_bits > 0x7f800000u ? E_NAN : E_INF;
+    if (abs_bits >= 0x7f800000u) return E_NONE;
     if (abs_bits == 0) return E_MIN;
     const int e = (int)(abs_bits >> 23);
     return e ? e - 127 : 31 - __clz(abs_bits) - 149;
@@ -117,7 +117,7 @@ struct RowScale {
     float s1, s2;
 };
 __device__ __forceinline__ RowScale row_scale(int E) {
-    if (E >= E_INF) return {0.f, 1.f};
+    if (E >= E_NONE) return {0.f, 1.f};
     const int t = 29 - E;
     return {pow2f(min(t, 127)), t > 127 ? pow2f(t - 127) : 1.f};
 }
@@ -134,20 +134,6 @@ __device__ __forceinline__ void bytes_of(float x0, float x1, float x2, float x3,
     p0 = __byte_perm(c, d, 0x7632);
 }
 
-// One output of rows of which at least one has no scale (rare: no attempt at speed).
-__device__ __noinline__ float unscaled_output(const float* a, const float* w, int K, int Ea, int Ew) {
-    if (Ea == E_NAN || Ew == E_NAN) return __uint_as_float(0x7fffffffu);
-    float sum = 0.f;
-    for (int k = 0; k < K; ++k) {
-        const float x = a[k], y = w[k];
-        if (isinf(x) || isinf(y)) {
-            sum += x * y;
-            if (isnan(sum)) break;
-        }
-    }
-    return sum;
-}
-
 struct FixedParams {
     const float* A;
     const float* W;
@@ -162,6 +148,36 @@ struct FixedParams {
     int* counters;                // [tiles], zero
     int* err_flag;
 };
+
+// The outputs of a tile's rows and features without a scale, by one of `warps` warps: sums in double precision, lanes over K, four tokens
+// at a time.  Rare: no attempt at speed beyond whole lines of the weights.
+__device__ __noinline__ void unscaled_outputs(const FixedParams& p, int f0, int t0, unsigned long long tokens, unsigned long long unscaled, int warp, int warps) {
+    const int lane = threadIdx.x & 31;
+    for (int f = f0 + warp; f < min(f0 + FEATURES, p.N); f += warps) {
+        const float* w = p.W + (size_t)f * p.ldw;
+        for (unsigned long long left = p.w_exp[f] >= E_NONE ? tokens : unscaled; left;) {
+            int t[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {      // fewer than four: the last one again
+                t[q] = left ? t0 + __ffsll((long long)left) - 1 : t[q ? q - 1 : 0];
+                left &= left - 1;
+            }
+            double sum[4] = {0., 0., 0., 0.};
+#pragma unroll 2
+            for (int k = lane; k < p.K; k += 32) {
+                const double y = w[k];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) sum[q] += (double)p.A[(size_t)t[q] * p.lda + k] * y;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], o);
+                if (lane == 0) p.C[(size_t)t[q] * p.ldc + f] = (float)sum[q];
+            }
+        }
+    }
+}
 
 template <int TN> struct Layout {
     // The groups of converting warps take a ring's steps in turn, and a wait by parity cannot tell a phase from the one two before it.  With a
@@ -182,7 +198,7 @@ template <int TN> struct Layout {
 
 template <int TN>
 __global__ void __launch_bounds__(THREADS, 1)
-fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_b, const FixedParams p) {
+fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ FixedParams p) {
     using L = Layout<TN>;
     static_assert(CONV_THREADS == 512, "the named barrier's count");
     extern __shared__ uint8_t smem_raw[];
@@ -195,11 +211,13 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::BARS + L::N_BARS * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 8);
     volatile int* last_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 16);
+    volatile int* unscaled_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 24);      // a tile has rows or features without a scale
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int items = p.tiles * p.splits, total_steps = (p.K + STEP - 1) / STEP;
 
     if (threadIdx.x == 0) {
         *abort_flag = 0;
+        *unscaled_flag = 0;
         for (int s = 0; s < L::W_STAGES; ++s) { mbar_init(w_full + 8 * s, 1); mbar_init(w_empty + 8 * s, 4); }
         for (int s = 0; s < L::B_STAGES; ++s) { mbar_init(b_full + 8 * s, 1); mbar_init(b_empty + 8 * s, 1); }
         for (int s = 0; s < A_STAGES; ++s) { mbar_init(a_full + 8 * s, 4); mbar_init(a_empty + 8 * s, 1); }
@@ -273,6 +291,7 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             constexpr uint32_t n4 = (uint32_t)(4 * TN >> 3) << 17, n3 = (uint32_t)((TN == 8 ? 32 : 3 * TN) >> 3) << 17, n2 = (uint32_t)(2 * TN >> 3) << 17;
             int it = 0, bt = 0, j = 0;
             bool ok = true;
+            pdl_wait();      // the tokens' planes come after it, and no bounded wait should have to last as long as the kernels before
             for (int item = blockIdx.x; item < items && ok; item += gridDim.x, ++j) {
                 int tile, split, first, n;
                 range(item, tile, split, first, n);
@@ -320,6 +339,13 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty);
         };
+        // the tokens and features of a tile that have no scale, as bits of its tokens (of all of them for a feature)
+        auto tokens_of = [&](int t0) { return p.M - t0 >= 64 ? ~0ull >> (64 - TN) : (1ull << min(TN, p.M - t0)) - 1; };
+        auto unscaled_tokens = [&](int t0) {
+            const int lo = t0 + lane, hi = lo + 32;
+            return __ballot_sync(0xffffffffu, lane < TN && lo < p.M && p.a_exp[lo] >= E_NONE) |
+                   (unsigned long long)__ballot_sync(0xffffffffu, 32 + lane < TN && hi < p.M && p.a_exp[hi] >= E_NONE) << 32;
+        };
         clear_last_sum();
         bool waited = false, ok = true;
         int it = 0, j = 0;
@@ -349,6 +375,7 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
                     bytes_of(v[q].x * sc.s1, v[q].y * sc.s1, v[q].z * sc.s1, v[q].w * sc.s1, pl[0][q], pl[1][q], pl[2][q], pl[3][q]);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(w_empty + 8 * s);
+                if (!waited && at >= A_STAGES) { pdl_wait(); waited = true; }      // from here on the MMAs have to run
                 ok = mbar_wait(a_empty + 8 * sa, ((at / A_STAGES) & 1) ^ 1, abort_flag, p.err_flag) && ok;
                 ok = __all_sync(0xffffffffu, ok);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -361,6 +388,7 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             it += n;
             if (!waited) { pdl_wait(); waited = true; }
+            if (split == 0 && (unscaled_tokens(t0) || (f < p.N && Ew >= E_NONE))) *unscaled_flag = 1;      // a warp looks at a quarter of the features
             ok = mbar_wait(acc_full, j & 1, abort_flag, p.err_flag) && ok && !*abort_flag;
             // all warps of the groups agree: they meet at a barrier below
             {
@@ -375,10 +403,8 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             auto finish = [&](int t, long long total) {
                 if (t >= p.M || f >= p.N) return;
                 const int Ea = p.a_exp[t];
-                float out;
-                if (Ea >= E_INF || Ew >= E_INF) out = unscaled_output(p.A + (size_t)t * p.lda, p.W + (size_t)f * p.ldw, p.K, Ea, Ew);
-                else out = (float)(__ll2double_rn(total) * __hiloint2double((Ea + Ew - 42 + 1023) << 20, 0));
-                p.C[(size_t)t * p.ldc + f] = out;
+                if (Ea >= E_NONE || Ew >= E_NONE) return;      // below
+                p.C[(size_t)t * p.ldc + f] = (float)(__ll2double_rn(total) * __hiloint2double((Ea + Ew - 42 + 1023) << 20, 0));
             };
             long long* const mine = p.partial + ((size_t)(split * p.tiles + tile) * TN) * FEATURES + row;
             if (has_cols) {
@@ -420,6 +446,14 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
         }
         if (!waited) pdl_wait();
+        asm volatile("bar.sync 1, 512;" ::: "memory");      // all warps have looked at their last tile
+        if (ok && *unscaled_flag) {
+            // each tile once: by the CTA that had its first share
+            for (int item = blockIdx.x; item < p.tiles; item += gridDim.x) {
+                const int t0 = item % p.tiles_m * TN;
+                unscaled_outputs(p, item / p.tiles_m * FEATURES, t0, tokens_of(t0), unscaled_tokens(t0), warp - CONV_WARP0, GROUPS * 4);
+            }
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -472,7 +506,7 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* plan
     if (tid == 0) exps[blockIdx.x] = E;
     if constexpr (PLANES) {
         const RowScale sc = row_scale(E);
-        const bool none = E >= E_INF;
+        const bool none = E >= E_NONE;
         uint8_t* out = planes + (size_t)blockIdx.x * pitch;
         auto put = [&](int k, const float4& v) {
             uint32_t w[4];

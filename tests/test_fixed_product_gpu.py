@@ -86,6 +86,31 @@ def test_infinities_and_nans(ops):
         assert torch.equal(got[rows][:, cols], clean[rows][:, cols])
 
 
+@pytest.mark.parametrize("M,N,K,plan", [(64, 300, 40960, (0, 0)), (130, 256, 4100, (64, 1)), (40, 384, 2048, (48, 2)), (5, 700, 1024, (8, 1))])
+def test_whole_tiles_without_a_scale(ops, M, N, K, plan):
+    """Nothing waits for rows and features that have no scale, however long their sums take; in double precision they are nearer
+    to 64 bits than any sum in 32."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, w = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    a[:, 3::17] = 0
+    a[torch.arange(M), torch.randint(0, K // 17, (M,)) * 17 + 3] = float("inf")      # one in every row
+    a[M // 2, 8] = -float("inf")
+    w[N // 3, 5], w[N - 1, 3::17] = float("nan"), 0
+    W = ops.FixedWeight(w)
+    for x in (a, a[::3]):
+        got, want = ops.fixed_linear(x, W, plan), x.double() @ w.double().t()
+        ops.check_device_errors()
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(torch.isinf(got), torch.isinf(want))
+        assert torch.equal(got[torch.isinf(got)].double(), want[torch.isinf(want)])
+    w[N // 3, 5] = 0
+    w[::50, 7] = float("inf")
+    a = torch.randn(M, K, device="cuda", generator=g).abs()
+    got, want = ops.fixed_linear(a, ops.FixedWeight(w), plan), a.double() @ w.double().t()
+    assert torch.equal(torch.isinf(got), torch.isinf(want)) and not torch.isnan(got).any()
+    assert torch.equal(got[:, ::50].double(), want[:, ::50])
+    ops.check_device_errors()
+
+
 def test_which_weights_take_it(ops):
     """The rule knows the weight alone: small ones, short rows, few features and rows off 16-byte boundaries stay with the CUDA cores'
     product."""
