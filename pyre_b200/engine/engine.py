@@ -87,6 +87,7 @@ class Engine:
         pinned = self.model.device.type == "cuda"
         self._err_host = [torch.zeros(1, dtype=torch.int32, pin_memory=pinned) for _ in range(2)]
         self._err_turn = 0
+        self._logits_free: list = []      # pinned memory for kept logits that no open step writes to (two steps are open at a time)
         self.step_log: "list[dict] | None" = [] if ec.record_steps else None
         self.kernel_times: dict = {}      # with time_kernels: class -> {"us": device time so far, "launches": n}
         self._waited = 0.0                # seconds of the current call spent waiting for a step's ids
@@ -209,23 +210,20 @@ class Engine:
             outs.append(RequestOutput(r.seq_id, r.prompt_ids, list(r.generated), r.finish_reason or "", r.preemptions, kept))
         return outs
 
-    _logits_last = _logits_spare = None      # pinned memory for kept logits: of the latest step that had some, of the one before it
-
     def _copy_logits(self, logits: torch.Tensor, sampling) -> "tuple | None":
-        """Start the copy of the rows that requests keep (only those that ask for their logits pay for it) to one of two pinned
-        buffers (two steps are open at a time): (host rows, [(request, index of the token they choose)]).  The rows are there once
-        the step's ids are."""
+        """Start the copy of the rows that requests keep (only those that ask for their logits pay for it) to pinned memory: (buffer, host
+        rows in it, [(request, index of the token they choose)]).  The rows are there once the step's ids are; the buffer is the step's
+        until it has landed, and goes with it if it never does."""
         keep = [k for k, s in enumerate(sampling) if s.request.params.return_logits]
         if not keep:
             return None
         rows = logits[:len(sampling)] if len(keep) == len(sampling) else logits[keep]
-        buffer, self._logits_spare = self._logits_spare, self._logits_last
+        buffer = self._logits_free.pop() if self._logits_free else None
         if buffer is None or buffer.numel() < rows.numel():
             buffer = torch.empty(rows.numel(), dtype=rows.dtype, pin_memory=rows.is_cuda)
-        self._logits_last = buffer
         host = buffer[:rows.numel()].view(rows.shape)
         host.copy_(rows, non_blocking=True)
-        return host, [(sampling[k].request, len(sampling[k].request.generated)) for k in keep]
+        return buffer, host, [(sampling[k].request, len(sampling[k].request.generated)) for k in keep]
 
     def _land(self, flight) -> None:
         """Read the ids of a started step and let the scheduler record them."""
@@ -236,9 +234,10 @@ class Engine:
         if ticket is not None and int(err[0]) != 0:
             self.stepper.check_device_errors()      # raises with the kernel's reason
         if kept is not None:
-            host, places = kept
-            for row, (request, index) in zip(host.numpy().copy(), places):      # the buffer is the next but one step's
+            buffer, host, places = kept
+            for row, (request, index) in zip(host.numpy().copy(), places):      # the buffer is a later step's
                 request.logits[index] = row
+            self._logits_free.append(buffer)
         self.scheduler.resolve(plan, ids)
 
     def has_unfinished(self) -> bool:

@@ -434,6 +434,33 @@ def test_logits_come_back_with_the_tokens_when_asked_for(models, monkeypatch, lo
         assert o.logits.argmax(axis=1).tolist() == o.token_ids
 
 
+def test_kept_logits_of_an_open_step_outlive_one_that_failed():
+    """A step whose sampling raises after the copy of its logits was started must not hand an open step's buffer to the next one."""
+    from types import SimpleNamespace
+
+    from pyre_b200.engine.engine import Engine
+
+    def planned(n):
+        return [SimpleNamespace(request=SimpleNamespace(params=SimpleNamespace(return_logits=True), generated=[0] * n, logits={}))]
+
+    eng = object.__new__(Engine)
+    eng._logits_free, eng._waited = [], 0.0
+    eng.sampler, eng.scheduler = SimpleNamespace(read=lambda t: []), SimpleNamespace(resolve=lambda plan, ids: None)
+    rows = [torch.full((1, 6), float(k)) for k in range(6)]
+    open_step = planned(0)
+    kept = eng._copy_logits(rows[0], open_step)
+    eng._copy_logits(rows[1], planned(1))      # its sampling raised: no flight
+    later = planned(1)
+    kept2 = eng._copy_logits(rows[2], later)
+    eng._land((open_step, None, None, kept))
+    again = planned(2)
+    kept3 = eng._copy_logits(rows[3], again)
+    eng._land((later, None, None, kept2))
+    eng._land((again, None, None, kept3))
+    assert [s[0].request.logits[n].tolist() for n, s in enumerate((open_step, later, again))] == [[0.0] * 6, [2.0] * 6, [3.0] * 6]
+    assert len(eng._logits_free) == 2      # bounded by the steps that are open at a time
+
+
 def test_replay_answers_each_line_before_the_next_one_is_written(models, monkeypatch):
     """The next step of a trace may come only after ``done <step>``: the loop must answer a line as soon as it
     has it, without waiting for more input.  Lines go through a pipe one at a time; each answer is awaited."""
