@@ -3,17 +3,30 @@
 // A row of either operand is taken as 31-bit integers on a power-of-two scale of its own, x = X 2^(E - 29) with E the
 // exponent of the row's largest element (|X| <= 2^30), and X as four signed bytes, X = sum_p d_p 2^(8 (3 - p)).  Products of
 // byte planes are summed by tcgen05.mma kind::i8 in 32-bit integers, exactly, planes i and j into the sum i + j; the sums
-// 0 .. 4 (13 of the 16 products) make a 64-bit integer that is scaled and rounded to float once.  An output is therefore
-// off by one rounding to float, 2^-30 of the rows' largest elements per factor, and the products left out (some 2^-35 of the product of
-// the two largest elements per term), where a chain of fused multiply-adds rounds with every term.  Against 64 bits (2-norm of the
-// error over 2-norm of the result, this / the sums of gemm_f32.cu): normal operands, K = 512 .. 3,584 2.5e-8 / 0.9-1.2e-7; rows with one
-// element 3,000 times the others 3.4e-8 / 1.5e-7; log-normal operands 4.0e-8 / 4.1e-8; where one column of A is a thousand times the others
-// and that column of W a thousandth, so that the result does not see it, 3.0e-7 / 1.2e-7.
+// 0 .. 4 (13 of the 16 products) make a 64-bit integer that is scaled and rounded to float.  An output is therefore
+// off by the rounding to float, 2^-30 of the rows' largest elements per factor, and the products left out (some 2^-35 of the product of
+// the two largest elements per term), where a chain of fused multiply-adds rounds with every term.
+//
+// A scale gives every element the bits that are left below the row's largest one.  That costs nothing where the large elements make the
+// result, and everything where they meet small ones and the rest of the row makes it.  So:
+//   * A token's elements of more than 2^OUTLIER_BITS times the mean magnitude (2 to the mean exponent of the elements that are not zero;
+//     the mean is taken again without the ones found, until there are none) stay out of the integers as long as they are no more than
+//     MAX_OUTLIERS: they are listed, and the epilogue adds their products with the float weights in double precision.
+//   * A feature with an element of more than 2^WEIGHT_BITS times its mean magnitude has no scale; nor has a row with an infinity or a
+//     NaN.  A weight with many such features should not come here (ops.linear_weight).
+//   * The 128 outputs of a token in a tile are held against what the scales may have cost them (by the norms of the rows, see
+//     `result_holds`).  If that is more than 2^-23 of their 2-norm, or if the token or a feature has no scale, the outputs are made again from
+//     the float operands in double precision, after the CTA's last tile: nothing waits for them under a bounded wait.
+// All are facts of the row and the weight alone, so that a row's result does not depend on what else is in the batch.
+// Against 64 bits (2-norm of the error over 2-norm of the result, this / the sums of gemm_f32.cu): normal operands
+// 2.5e-8 / 1.0e-7 (K = 512), 1.2e-7 (3,584), 1.8e-7 (18,944); 1 to 200 columns of A 16 to 1e25 times the others and those of W by as much
+// less 2.5e-8 to 7.8e-8 / the same; log-normal activations up to e^(3 x) 2.4e-8 to 4.5e-8 / 0.8e-7 to 2.2e-7; where they come nearest, a share of 0.7 of A's
+// columns a hundredth and the rest of W's, 1.0e-7 / 1.0e-7 (512), 1.1e-7 / 1.2e-7 (3,584).
+// What it costs, us: ordinary and heavy-tailed rows nothing measurable from 64 rows on, 0.7 to 2.5 of 19 to 98 for 1 to 4 rows; per output and
+// outlier 7 ps (509 x 37,888 x 3,584: 770, with four columns of outliers 1,310); outputs made again some 13 multiplications a cycle and SM (all of the same
+// product: 20,400; one row in 64: 330 for 115).
 //
 // Integers add up in any order: a row's result has the same bits for any M, tile, split of K or order of arrival.
-//
-// A row with an infinity or a NaN has no scale.  Its outputs are sums of the float operands in double precision, a warp per feature,
-// after the CTA's last tile: nothing waits for them under a bounded wait.
 //
 // Two kernels: the activations' exponents and byte planes (they are few), then the product.  The product's CTA (640 threads)
 // owns 128 output features (the weights on the MMA's rows) and TN tokens, K in steps of 32:
@@ -35,6 +48,8 @@ namespace {
 constexpr int ERR_TIMEOUT = 2;
 constexpr int E_NONE = 1000;                   // of a row without a scale
 constexpr int E_MIN = -98;                     // of a row of zeros (its scale is a normal float)
+constexpr int OUTLIER_BITS = 7, WEIGHT_BITS = 6, MAX_OUTLIERS = 16;      // see above
+constexpr int ROW_THREADS = 512, ROW_WARPS = ROW_THREADS / 32;      // of the kernel in front
 constexpr int FEATURES = 128, STEP = 32, BLOCK_K = 128;
 constexpr int CONV_WARP0 = 4, GROUPS = 4, CONV_THREADS = GROUPS * 128, THREADS = CONV_WARP0 * 32 + CONV_THREADS;
 constexpr int W_BYTES = FEATURES * STEP * 4;   // a step's weights
@@ -112,6 +127,7 @@ __device__ __forceinline__ int row_exponent(uint32_t abs_bits) {
     const int e = (int)(abs_bits >> 23);
     return e ? e - 127 : 31 - __clz(abs_bits) - 149;
 }
+__device__ __forceinline__ double pow2d(int e) { return __hiloint2double((e + 1023) << 20, 0); }
 // x 2^(29 - E) as two factors: 29 - E reaches 178 for rows of the smallest numbers
 struct RowScale {
     float s1, s2;
@@ -134,11 +150,22 @@ __device__ __forceinline__ void bytes_of(float x0, float x1, float x2, float x3,
     p0 = __byte_perm(c, d, 0x7632);
 }
 
+// A token's word: its exponent in the lower half, the number of its outliers in the upper one.
+__device__ __forceinline__ int exponent_of(int word) { return (short)word; }
+__device__ __forceinline__ int outliers_of(int word) { return word >> 16; }
+
 struct FixedParams {
     const float* A;
     const float* W;
     const int* w_exp;             // [N]
-    const int* a_exp;             // [M]
+    const int* a_word;            // [M]
+    const int2* outliers;         // [M][MAX_OUTLIERS]: k and the element's bits, by ascending k
+    const float* w_norm;          // [N]: squares of the rows' 2-norms over those of their scales, 4^E
+    const float* a_norm;          // [M][ROW_WARPS]: the same in parts (without outliers)
+    float4* squares;              // [tiles][TN]: of the outputs over their scales, by quarters of the features (a CTA's last tile: in shared memory)
+    float2* features;             // [items][4]: by quarters of the features, their norms and, as bits, how many have a scale (the sign: some have none)
+    int* decided;                 // [items]: the item completed its tile (where K is split)
+    unsigned long long* again;    // [items]: the tokens whose outputs are made from the float operands
     float* C;
     long long lda, ldw, ldc;
     int M, N, K;
@@ -149,32 +176,109 @@ struct FixedParams {
     int* err_flag;
 };
 
-// The outputs of a tile's rows and features without a scale, by one of `warps` warps: sums in double precision, lanes over K, four tokens
-// at a time.  Rare: no attempt at speed beyond whole lines of the weights.
-__device__ __noinline__ void unscaled_outputs(const FixedParams& p, int f0, int t0, unsigned long long tokens, unsigned long long unscaled, int warp, int warps) {
-    const int lane = threadIdx.x & 31;
-    for (int f = f0 + warp; f < min(f0 + FEATURES, p.N); f += warps) {
-        const float* w = p.W + (size_t)f * p.ldw;
-        for (unsigned long long left = p.w_exp[f] >= E_NONE ? tokens : unscaled; left;) {
-            int t[4];
+// What a token's outliers add to an output, in the order of their list.
+__device__ __forceinline__ double outlier_sum(const int2* list, int n, const float* w) {
+    double sum = 0.;
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) sum += (double)__int_as_float(list[i].y) * (double)w[list[i].x];
+    return sum;
+}
+
+// Do a token's outputs in a tile, `squares` in all over 4^(Ea + Ew), have error enough to spare?  An element is off by 2^-29 / sqrt(12) of
+// its row's scale (2-norm), so an output by that times the other row's norm, and by 6.9e-12 sqrt(K) for the byte products left out.  The bound is 2^-23 of
+// the outputs' 2-norm, the size of the error that sums in 32 bits have; normal operands are off by 2^-28.  Rows of zeros have none.
+__device__ __forceinline__ bool result_holds(float squares, float a_norm, float w_norms, int features, int K) {
+    constexpr float SHARE = 70368744177664.f;      // 2^46
+    return squares >= SHARE * (2.9e-19f * ((float)features * a_norm + w_norms) + 4.8e-23f * (float)features * (float)K) || a_norm == 0.f || w_norms == 0.f;
+}
+
+// A token's norm, or -1 if it has no scale.
+__device__ __forceinline__ float token_norm(const FixedParams& p, int t) {
+    const int word = p.a_word[t];
+    float sum = 0.f;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {      // fewer than four: the last one again
-                t[q] = left ? t0 + __ffsll((long long)left) - 1 : t[q ? q - 1 : 0];
-                left &= left - 1;
+    for (int i = 0; i < ROW_WARPS; i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(p.a_norm + (size_t)t * ROW_WARPS + i);
+        sum += (v.x + v.y) + (v.z + v.w);
+    }
+    return exponent_of(word) < E_NONE ? sum : -1.f;
+}
+
+__device__ __forceinline__ void conv_barrier() { asm volatile("bar.sync 1, 512;" ::: "memory"); }      // of the converting warps
+
+// Outputs from the float operands, by all converting warps once the rings' shared memory is free: products of one row per thread of a
+// group (`mine`, if it has `some`) with n rows of the other operand, staged in shared memory, in double precision.  A group's threads take every
+// fourth block of 32 k in ascending order; the groups' sums are added in order.  AHEAD elements of a thread's own row are asked for at once: with
+// few rows opposite the chain of their latencies is the bound, with BATCH of them shared memory's reads.
+constexpr int UNSCALED_BYTES = CONV_THREADS * 16 * 8;      // staged rows and, after them, the groups' sums: a batch of 16
+template <int BATCH, int AHEAD>
+__device__ __noinline__ void double_products(const float* mine, bool some, const float* others, long long ld, const volatile int* list, int n, int K,
+                                             double* memory, float* out, long long out_ld) {
+    const int t = threadIdx.x - CONV_WARP0 * 32, lane = t & 31, group = t / FEATURES, row = t % FEATURES;
+    double* const stage = memory + (t >> 5) * (BATCH * 32);
+    const bool vec = !((uintptr_t)mine & 15);
+    double total[BATCH] = {};
+    for (int k0 = group * 32; k0 < K; k0 += GROUPS * 32) {
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < BATCH; ++j) stage[j * 32 + lane] = j < n && k0 + lane < K ? others[(size_t)list[j] * ld + k0 + lane] : 0.f;
+        __syncwarp();
+#pragma unroll 1
+        for (int k = 0; k < 32; k += AHEAD) {
+            float v[AHEAD];
+            if (some && vec && k0 + k + AHEAD <= K) {
+#pragma unroll
+                for (int i = 0; i < AHEAD; i += 4) *reinterpret_cast<float4*>(v + i) = *reinterpret_cast<const float4*>(mine + k0 + k + i);
+            } else {
+#pragma unroll
+                for (int i = 0; i < AHEAD; ++i) v[i] = some && k0 + k + i < K ? mine[k0 + k + i] : 0.f;
             }
-            double sum[4] = {0., 0., 0., 0.};
-#pragma unroll 2
-            for (int k = lane; k < p.K; k += 32) {
-                const double y = w[k];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) sum[q] += (double)p.A[(size_t)t[q] * p.lda + k] * y;
+            for (int i = 0; i < AHEAD; i += 2) {
+                const double a = v[i], b = v[i + 1];
+#pragma unroll
+                for (int j = 0; j < BATCH; ++j) {
+                    const double2 x = *reinterpret_cast<const double2*>(stage + j * 32 + k + i);
+                    total[j] = fma(b, x.y, fma(a, x.x, total[j]));
+                }
             }
+        }
+    }
+    conv_barrier();      // the sums take the place of the staged rows
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], o);
-                if (lane == 0) p.C[(size_t)t[q] * p.ldc + f] = (float)sum[q];
-            }
+    for (int j = 0; j < BATCH; ++j) memory[j * CONV_THREADS + t] = total[j];
+    conv_barrier();
+    if (some)
+        for (int j = group; j < n; j += GROUPS) {
+            const double* s = memory + j * CONV_THREADS + row;
+            out[(size_t)list[j] * out_ld] = (float)(((s[0] + s[FEATURES]) + s[2 * FEATURES]) + s[3 * FEATURES]);
+        }
+    conv_barrier();
+}
+// ... of a tile: `again` are the tokens.
+__device__ __noinline__ void unscaled_outputs(const FixedParams& p, uint8_t* smem, int f0, int t0, int tokens, unsigned long long again) {
+    const int t = threadIdx.x - CONV_WARP0 * 32, row = t % FEATURES;
+    double* const memory = reinterpret_cast<double*>(smem);
+    volatile int* const list = reinterpret_cast<volatile int*>(smem + UNSCALED_BYTES);
+    int* const count = reinterpret_cast<int*>(smem + UNSCALED_BYTES) + FEATURES;
+    const bool token = row < tokens && again >> row & 1, feature = f0 + row < p.N && p.w_exp[f0 + row] >= E_NONE;
+    // the tile's features by those tokens, then its other tokens by its features without a scale
+    for (int phase = 0; phase < 2; ++phase) {
+        conv_barrier();
+        if (t == 0) *count = 0;
+        conv_barrier();
+        if (t < FEATURES && (phase ? feature : token)) list[atomicAdd(count, 1)] = row;
+        conv_barrier();
+        const int listed = *const_cast<volatile int*>(count);
+        const bool some = phase ? row < tokens && !token : f0 + row < p.N;
+        const float* const mine = phase ? p.A + (size_t)(t0 + row) * p.lda : p.W + (size_t)(f0 + row) * p.ldw;
+        const float* const others = phase ? p.W + (size_t)f0 * p.ldw : p.A + (size_t)t0 * p.lda;
+        const long long ld = phase ? p.ldw : p.lda, out_ld = phase ? 1 : p.ldc;
+        float* const out = p.C + (phase ? (size_t)(t0 + row) * p.ldc + f0 : (size_t)t0 * p.ldc + f0 + row);
+        for (int at = 0; at < listed;) {
+            const int left = listed - at;
+            if (left > 2) double_products<16, 8>(mine, some, others, ld, list + at, min(left, 16), p.K, memory, out, out_ld), at += 16;
+            else double_products<2, 32>(mine, some, others, ld, list + at, left, p.K, memory, out, out_ld), at += 2;
         }
     }
 }
@@ -188,11 +292,13 @@ template <int TN> struct Layout {
     static constexpr int B_BYTES = 4 * TN * BLOCK_K, B_STAGES = TN <= 16 ? 4 : 3;
     static constexpr int W_OFF = 0, B_OFF = W_STAGES * W_BYTES, BARS = B_OFF + B_STAGES * B_BYTES;
     static constexpr int N_BARS = 2 * W_STAGES + 2 * B_STAGES + 2 * A_STAGES + 2;
-    static constexpr int TOTAL = BARS + N_BARS * 8 + 32 + 1024;
+    static constexpr int CHECK = BARS + N_BARS * 8 + 32;      // of the last tile: squares [TN], the tokens' norms [TN], the features' [4]
+    static constexpr int TOTAL = CHECK + 20 * TN + 32 + 1024;
     // an MMA of M = 128 takes N in sixteens: with eight tokens the third plane's product is one plane wider (its last sum is not read)
     static constexpr int SUMS = TN == 8 ? 6 : 5;
     static constexpr int A_COL0 = 512 - A_STAGES * A_COLS;
     static_assert(W_STAGES % GROUPS == 0 && A_STAGES >= GROUPS, "a stage belongs to one group; see above");
+    static_assert(B_OFF >= UNSCALED_BYTES + (FEATURES + 1) * 4 && CHECK % 16 == 0, "unscaled_outputs' memory");
     static_assert(TOTAL <= 232448 && SUMS * TN <= A_COL0 && (TN == 8 || TN % 16 == 0), "fits");
 };
 
@@ -211,7 +317,7 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::BARS + L::N_BARS * 8);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 8);
     volatile int* last_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 16);
-    volatile int* unscaled_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 24);      // a tile has rows or features without a scale
+    volatile int* unscaled_flag = reinterpret_cast<volatile int*>(gen + L::BARS + L::N_BARS * 8 + 24);      // some outputs are to be made from the float operands
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int items = p.tiles * p.splits, total_steps = (p.K + STEP - 1) / STEP;
 
@@ -339,12 +445,48 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty);
         };
-        // the tokens and features of a tile that have no scale, as bits of its tokens (of all of them for a feature)
-        auto tokens_of = [&](int t0) { return p.M - t0 >= 64 ? ~0ull >> (64 - TN) : (1ull << min(TN, p.M - t0)) - 1; };
-        auto unscaled_tokens = [&](int t0) {
-            const int lo = t0 + lane, hi = lo + 32;
-            return __ballot_sync(0xffffffffu, lane < TN && lo < p.M && p.a_exp[lo] >= E_NONE) |
-                   (unsigned long long)__ballot_sync(0xffffffffu, 32 + lane < TN && hi < p.M && p.a_exp[hi] >= E_NONE) << 32;
+        float4* const s_squares = reinterpret_cast<float4*>(gen + L::CHECK);
+        float* const s_tokens = reinterpret_cast<float*>(s_squares + TN);
+        float2* const s_features = reinterpret_cast<float2*>(s_tokens + TN);
+        // Do a tile's results hold?
+        auto check = [&](int item, bool last_tile) {
+            const int tile = item % p.tiles, t0 = tile % p.tiles_m * TN;
+            float2 part[4];      // (asked for before anything is used: one latency)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) part[r] = (last_tile ? s_features : p.features + (size_t)item * 4)[r];
+            float norm[(TN + 31) / 32];
+            float4 square[(TN + 31) / 32];
+#pragma unroll
+            for (int c = 0; c < TN; c += 32) {
+                norm[c / 32] = 0.f;
+                if (c + lane < TN && t0 + c + lane < p.M) {
+                    norm[c / 32] = last_tile ? s_tokens[c + lane] : token_norm(p, t0 + c + lane);
+                    square[c / 32] = last_tile ? s_squares[c + lane] : p.squares[(size_t)tile * TN + c + lane];
+                }
+            }
+            float w_norms = 0.f;
+            int features = 0;
+            bool odd = false;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                w_norms += part[r].x;
+                features += __float_as_int(part[r].y) & 0x7fffffff;
+                odd |= __float_as_int(part[r].y) < 0;
+            }
+            unsigned long long again = 0;
+#pragma unroll
+            for (int c = 0; c < TN; c += 32) {
+                bool holds = true;
+                if (c + lane < TN && t0 + c + lane < p.M) {
+                    const float4 s = square[c / 32];
+                    holds = norm[c / 32] >= 0.f && result_holds(((s.x + s.y) + s.z) + s.w, norm[c / 32], w_norms, features, p.K);
+                }
+                again |= (unsigned long long)__ballot_sync(0xffffffffu, !holds) << c;
+            }
+            if (lane == 0) {
+                if (odd || again) *unscaled_flag = 1;
+                p.again[item] = again;
+            }
         };
         clear_last_sum();
         bool waited = false, ok = true;
@@ -353,7 +495,9 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             int tile, split, first, n;
             range(item, tile, split, first, n);
             const int f = tile / p.tiles_m * FEATURES + row, t0 = tile % p.tiles_m * TN;
+            const bool last_tile = item + gridDim.x >= items;
             const int Ew = f < p.N ? p.w_exp[f] : E_MIN;
+            const float w_norm = group == 0 && f < p.N ? p.w_norm[f] : 0.f;      // (from memory: asked for well ahead)
             const RowScale sc = row_scale(Ew);
             const bool tiny = __any_sync(0xffffffffu, sc.s2 != 1.f);
             for (int i = (group - it) & (GROUPS - 1); i < n && ok; i += GROUPS) {
@@ -388,7 +532,13 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             it += n;
             if (!waited) { pdl_wait(); waited = true; }
-            if (split == 0 && (unscaled_tokens(t0) || (f < p.N && Ew >= E_NONE))) *unscaled_flag = 1;      // a warp looks at a quarter of the features
+            // what the tile's check needs, while the MMAs finish
+            if (group == 0) {
+                const bool scaled = f < p.N && Ew < E_NONE;
+                const float norm = warp_sum(scaled ? w_norm : 0.f);
+                const int count = __popc(__ballot_sync(0xffffffffu, scaled)) | (__any_sync(0xffffffffu, f < p.N && !scaled) ? 0x80000000 : 0);
+                if (lane == 0) (last_tile ? s_features : p.features + (size_t)item * 4)[quarter] = make_float2(norm, __int_as_float(count));
+            } else if (group == 1 && last_tile && row < TN && t0 + row < p.M) s_tokens[row] = token_norm(p, t0 + row);
             ok = mbar_wait(acc_full, j & 1, abort_flag, p.err_flag) && ok && !*abort_flag;
             // all warps of the groups agree: they meet at a barrier below
             {
@@ -399,28 +549,55 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             }
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            // sum s stands for 2^(8 (6 - s)); a row's scale is 2^(E - 29): C = total 2^(16 + Ea + Ew - 58)
-            auto finish = [&](int t, long long total) {
-                if (t >= p.M || f >= p.N) return;
-                const int Ea = p.a_exp[t];
-                if (Ea >= E_NONE || Ew >= E_NONE) return;      // below
-                p.C[(size_t)t * p.ldc + f] = (float)(__ll2double_rn(total) * __hiloint2double((Ea + Ew - 42 + 1023) << 20, 0));
+            if (last_tile)      // the tiles before it, a warp each, from those that may have no columns on
+                for (int q = CONV_WARP0 + 4 * GROUPS - 1 - warp; q < j; q += 4 * GROUPS) {
+                    const int earlier = (int)blockIdx.x + q * (int)gridDim.x;
+                    if (p.splits == 1 || p.decided[earlier]) check(earlier, false);
+                }
+            // sum s stands for 2^(8 (6 - s)); a row's scale is 2^(E - 29): C = total 2^(16 - 58) 2^(Ea + Ew).  Returns the square of C over 2^(Ea + Ew)
+            auto finish = [&](int t, int word, long long total) {
+                const int Ea = exponent_of(word);
+                if (t >= p.M || f >= p.N || Ea >= E_NONE || Ew >= E_NONE) return 0.f;
+                double x = __ll2double_rn(total) * 0x1p-42;
+                if (outliers_of(word)) x += outlier_sum(p.outliers + (size_t)t * MAX_OUTLIERS, outliers_of(word), p.W + (size_t)f * p.ldw) * pow2d(-Ea - Ew);
+                p.C[(size_t)t * p.ldc + f] = (float)(x * pow2d(Ea + Ew));
+                return (float)x * (float)x;
             };
+            float* const squares = reinterpret_cast<float*>(last_tile ? s_squares : p.squares + (size_t)tile * TN);
             long long* const mine = p.partial + ((size_t)(split * p.tiles + tile) * TN) * FEATURES + row;
             if (has_cols) {
 #pragma unroll 1
                 for (int c = 0; c < COLS; c += 8) {
-                    int s[5][8];
+                    int s[5][8], word[8];
+                    // (the words' memory goes on beyond the last token's)
+                    *reinterpret_cast<int4*>(word) = *reinterpret_cast<const int4*>(p.a_word + t0 + col0 + c);
+                    *reinterpret_cast<int4*>(word + 4) = *reinterpret_cast<const int4*>(p.a_word + t0 + col0 + c + 4);
                     __syncwarp();
 #pragma unroll
                     for (int q = 0; q < 5; ++q) tmem_ld8(tmem + lanes + q * TN + col0 + c, s[q]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float v[8];
 #pragma unroll
                     for (int e = 0; e < 8; ++e) {
                         const long long total = ((long long)s[0][e] << 32) + ((long long)s[1][e] << 24) + ((long long)s[2][e] << 16) +
                                                 ((long long)s[3][e] << 8) + s[4][e];
-                        if (p.splits == 1) finish(t0 + col0 + c + e, total);
+                        if (p.splits == 1) v[e] = finish(t0 + col0 + c + e, word[e], total);
                         else if (t0 + col0 + c + e < p.M) mine[(size_t)(col0 + c + e) * FEATURES] = total;
+                    }
+                    if (p.splits == 1) {
+                        // the warp's eight sums at once (the tree of warp_sum): half of them go to the other half of the lanes, ...
+#pragma unroll
+                        for (int half = 4, o = 16; half; half >>= 1, o >>= 1) {
+                            const bool upper = lane & o;
+#pragma unroll
+                            for (int i = 0; i < half; ++i) {
+                                const float sent = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[i + half], o);
+                                v[i] = (upper ? v[i + half] : v[i]) + sent;
+                            }
+                        }
+                        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+                        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+                        if ((lane & 3) == 0) squares[(col0 + c + (lane >> 2)) * 4 + quarter] = v[0];
                     }
                 }
             }
@@ -429,30 +606,45 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
             if (p.splits > 1) {
                 // whoever arrives last adds up the tile's shares
                 __threadfence();
-                asm volatile("bar.sync 1, 512;" ::: "memory");
-                if (threadIdx.x == CONV_WARP0 * 32) *last_flag = atomicAdd(p.counters + tile, 1) == p.splits - 1;
-                asm volatile("bar.sync 1, 512;" ::: "memory");
+                conv_barrier();
+                if (threadIdx.x == CONV_WARP0 * 32) p.decided[item] = *last_flag = atomicAdd(p.counters + tile, 1) == p.splits - 1;
+                conv_barrier();
                 if (*last_flag) {
                     __threadfence();
                     const int rows = min(TN, p.M - t0);
-                    for (int c = group; c < rows; c += GROUPS) {
-                        const long long* from = p.partial + ((size_t)tile * TN + c) * FEATURES + row;
-                        long long total = 0;
-                        for (int z = 0; z < p.splits; ++z) total += __ldcg(from + (size_t)z * p.tiles * TN * FEATURES);
-                        finish(t0 + c, total);
+                    for (int c = group; c < rows; c += 4 * GROUPS) {      // four tokens' shares asked for at once
+                        long long total[4] = {};
+                        int word[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) word[q] = p.a_word[t0 + min(c + q * GROUPS, rows - 1)];
+                        for (int z = 0; z < p.splits; ++z)
+#pragma unroll
+                            for (int q = 0; q < 4; ++q)
+                                total[q] += __ldcg(p.partial + ((size_t)(z * p.tiles + tile) * TN + min(c + q * GROUPS, rows - 1)) * FEATURES + row);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const int at = c + q * GROUPS;
+                            if (at < rows) {
+                                const float square = warp_sum(finish(t0 + at, word[q], total[q]));
+                                if (lane == 0) squares[at * 4 + quarter] = square;
+                            }
+                        }
                     }
                 }
-                asm volatile("bar.sync 1, 512;" ::: "memory");      // the flag is read before the next item writes it
+                conv_barrier();      // the flag is read before the next item writes it
             }
         }
         if (!waited) pdl_wait();
-        asm volatile("bar.sync 1, 512;" ::: "memory");      // all warps have looked at their last tile
-        if (ok && *unscaled_flag) {
-            // each tile once: by the CTA that had its first share
-            for (int item = blockIdx.x; item < p.tiles; item += gridDim.x) {
-                const int t0 = item % p.tiles_m * TN;
-                unscaled_outputs(p, item / p.tiles_m * FEATURES, t0, tokens_of(t0), unscaled_tokens(t0), warp - CONV_WARP0, GROUPS * 4);
-            }
+        if (p.splits == 1 || !ok) conv_barrier();
+        if (ok) {
+            if (warp == CONV_WARP0 && (p.splits == 1 || *last_flag)) check(items - 1 - (items - 1 - (int)blockIdx.x) % (int)gridDim.x, true);
+            conv_barrier();
+            if (*unscaled_flag)
+                for (int item = blockIdx.x; item < items; item += gridDim.x)
+                    if (p.splits == 1 || p.decided[item]) {
+                        const int tile = item % p.tiles, t0 = tile % p.tiles_m * TN;
+                        unscaled_outputs(p, gen, tile / p.tiles_m * FEATURES, t0, min(TN, p.M - t0), p.again[item]);
+                    }
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -463,20 +655,23 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
 }
 
-// A row's exponent, and (PLANES) its elements as four byte planes [4][rows][pitch].  A block per row; what bounds it is the chain of
-// its latencies, so a thread asks for HELD pieces of four elements at once and keeps them (what a longer row has beyond them is read a second
-// time, out of the caches).
-constexpr int ROW_THREADS = 512;
+// PLANES: a token's word, norm and outliers, and its other elements as four byte planes [4][rows][pitch]; else a feature's exponent and norm.  A block
+// per row; what bounds it is the chain of its latencies, so a thread asks for HELD pieces of four elements at once and keeps them (what a
+// longer row has beyond them is read again, out of the caches).
 template <bool PLANES, bool VEC, int HELD>
-__global__ void __launch_bounds__(ROW_THREADS)
-fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* planes, long long plane_stride, int pitch, int* counters, int n_counters) {
-    __shared__ uint32_t s_max[ROW_THREADS / 32];
+__global__ void __launch_bounds__(ROW_THREADS, HELD == 2 ? 3 : 1)
+fixed_rows_kernel(const float* A, long long lda, int K, int* words, float* norms, int2* outliers, uint8_t* planes, long long plane_stride, int pitch, int* counters, int n_counters) {
+    __shared__ int4 s_stats[ROW_WARPS];
+    __shared__ int2 s_list[MAX_OUTLIERS];
+    __shared__ int s_count;
     if (PLANES) pdl_trigger();      // a weight's exponents: no product may start beside them (it reads them ahead of its own wait)
     pdl_wait();
     const int tid = threadIdx.x;
     const float* a = A + (size_t)blockIdx.x * lda;
-    if (PLANES)
+    if (PLANES) {
         for (int i = blockIdx.x * ROW_THREADS + tid; i < n_counters; i += gridDim.x * ROW_THREADS) counters[i] = 0;
+        if (tid == 0) s_count = 0;
+    }
     auto piece = [&](int k) {      // the four elements from k on, zeros beyond the row
         if (VEC) return k < K ? *reinterpret_cast<const float4*>(a + k) : make_float4(0.f, 0.f, 0.f, 0.f);
         float4 v;
@@ -486,32 +681,95 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* plan
         v.w = k + 3 < K ? a[k + 3] : 0.f;
         return v;
     };
-    uint32_t most = 0;
-    auto look = [&](const float4& v) {
-        most = max(max(most, __float_as_uint(v.x) & 0x7fffffffu), max(__float_as_uint(v.y) & 0x7fffffffu, __float_as_uint(v.z) & 0x7fffffffu));
-        most = max(most, __float_as_uint(v.w) & 0x7fffffffu);
-    };
     float4 held[HELD];
 #pragma unroll
     for (int h = 0; h < HELD; ++h) held[h] = piece(4 * (tid + h * ROW_THREADS));
+    auto magnitude = [](float x) { return __float_as_uint(x) & 0x7fffffffu; };
+    uint32_t limit = 0xffffffffu;      // elements from here on have been listed
+    int E, listed = 0;
+    for (;;) {
+        // of the others: the largest, the sum of their exponents, how many are not zero
+        uint32_t most = 0, both = 0;      // the sum below the count: a warp has at most 2,560 elements
+        auto look = [&](float x) {
+            const uint32_t u = magnitude(x);
+            most = max(most, u);
+            both += (u >> 23) + (u ? 1u << 20 : 0u);
+        };
+        if (limit == 0xffffffffu) {
 #pragma unroll
-    for (int h = 0; h < HELD; ++h) look(held[h]);
-    for (int k = 4 * (tid + HELD * ROW_THREADS); k < K; k += 4 * ROW_THREADS) look(piece(k));
-    most = __reduce_max_sync(0xffffffffu, most);
-    if ((tid & 31) == 0) s_max[tid >> 5] = most;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < ROW_THREADS / 32; ++i) most = max(most, s_max[i]);
-    const int E = row_exponent(most);
-    if (tid == 0) exps[blockIdx.x] = E;
-    if constexpr (PLANES) {
-        const RowScale sc = row_scale(E);
-        const bool none = E >= E_NONE;
+            for (int h = 0; h < HELD; ++h) { look(held[h].x); look(held[h].y); look(held[h].z); look(held[h].w); }
+#pragma unroll 1
+            for (int k = 4 * (tid + HELD * ROW_THREADS); k < K; k += 4 * ROW_THREADS) {
+                const float4 v = piece(k);
+                look(v.x); look(v.y); look(v.z); look(v.w);
+            }
+        } else
+            for (int k = tid; k < K; k += ROW_THREADS)
+                if (magnitude(a[k]) < limit) look(a[k]);
+        most = __reduce_max_sync(0xffffffffu, most);
+        both = __reduce_add_sync(0xffffffffu, both);
+        int sum, n;
+        if ((tid & 31) == 0) s_stats[tid >> 5] = make_int4((int)most, (int)(both & 0xfffff), (int)(both >> 20), 0);
+        __syncthreads();
+        const int4 others = (tid & 31) < ROW_WARPS ? s_stats[tid & 31] : make_int4(0, 0, 0, 0);
+        most = __reduce_max_sync(0xffffffffu, (uint32_t)others.x);
+        sum = __reduce_add_sync(0xffffffffu, others.y);
+        n = __reduce_add_sync(0xffffffffu, others.z);
+        E = row_exponent(most);
+        if (E >= E_NONE || n == 0) break;
+        const int bound = sum / n + (PLANES ? OUTLIER_BITS : WEIGHT_BITS);
+        if ((int)(most >> 23) <= bound) break;
+        if (!PLANES) {
+            E = E_NONE;
+            break;
+        }
+        const uint32_t from = (uint32_t)(bound + 1) << 23;      // at most the exponent of `most`
+        for (int k = tid; k < K; k += ROW_THREADS) {
+            const float x = a[k];
+            const uint32_t u = magnitude(x);
+            if (u >= from && u < limit) {
+                const int at = atomicAdd(&s_count, 1);
+                if (at < MAX_OUTLIERS) s_list[at] = make_int2(k, __float_as_int(x));
+            }
+        }
+        __syncthreads();
+        if (s_count > MAX_OUTLIERS) break;      // too many: these stay in the integers
+        listed = s_count;                       // (the next turn adds to it behind its own barrier)
+        limit = from;
+    }
+    const RowScale sc = row_scale(E);
+    const bool none = E >= E_NONE;
+    float norm = 0.f;
+    auto scaled = [&](float x) { return none || magnitude(x) >= limit ? 0.f : x * sc.s2 * sc.s1; };
+    auto square = [&](float x) { norm = fmaf(x, x, norm); };      // in units of 2^58
+    if constexpr (!PLANES) {
+        for (int k = tid; k < K; k += ROW_THREADS) square(scaled(a[k]));
+        norm = warp_sum(norm);
+        __syncthreads();
+        if ((tid & 31) == 0) s_stats[tid >> 5].x = __float_as_int(norm);
+        __syncthreads();
+        if (tid == 0) {
+            for (int i = 1; i < ROW_WARPS; ++i) norm += __int_as_float(s_stats[i].x);
+            norms[blockIdx.x] = norm * 0x1p-58f;
+            words[blockIdx.x] = E;
+        }
+    } else {
+        if (tid < 32) {
+            const int n = none ? 0 : listed;
+            if (tid == 0) words[blockIdx.x] = n << 16 | (E & 0xffff);
+            if (tid < n) {
+                const int2 mine = s_list[tid];
+                int rank = 0;
+                for (int i = 0; i < n; ++i) rank += s_list[i].x < mine.x;
+                outliers[(size_t)blockIdx.x * MAX_OUTLIERS + rank] = mine;
+            }
+        }
         uint8_t* out = planes + (size_t)blockIdx.x * pitch;
         auto put = [&](int k, const float4& v) {
             uint32_t w[4];
-            bytes_of(none ? 0.f : v.x * sc.s2 * sc.s1, none ? 0.f : v.y * sc.s2 * sc.s1, none ? 0.f : v.z * sc.s2 * sc.s1, none ? 0.f : v.w * sc.s2 * sc.s1,
-                     w[0], w[1], w[2], w[3]);
+            const float x = scaled(v.x), y = scaled(v.y), z = scaled(v.z), u = scaled(v.w);
+            square(x); square(y); square(z); square(u);
+            bytes_of(x, y, z, u, w[0], w[1], w[2], w[3]);
 #pragma unroll
             for (int q = 0; q < 4; ++q) *reinterpret_cast<uint32_t*>(out + q * plane_stride + k) = w[q];
         };
@@ -520,7 +778,10 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* exps, uint8_t* plan
             const int k = 4 * (tid + h * ROW_THREADS);
             if (k < pitch) put(k, held[h]);
         }
+#pragma unroll 1
         for (int k = 4 * (tid + HELD * ROW_THREADS); k < pitch; k += 4 * ROW_THREADS) put(k, piece(k));
+        norm = warp_sum(norm);
+        if ((tid & 31) == 0) norms[blockIdx.x * ROW_WARPS + (tid >> 5)] = norm * 0x1p-58f;      // whoever reads them adds them up: no barrier for it here
     }
 }
 
@@ -540,7 +801,7 @@ EncodeTiledFn encode_tiled() {
 
 struct Plan {
     int tn, tiles_m, tiles, splits, steps_per_split;
-    long long planes, exps, counters, partial, bytes;      // offsets into the workspace
+    long long planes, words, norms, outliers, squares, features, again, decided, counters, partial, bytes;      // offsets into the workspace
     int pitch;
 };
 // Tokens per tile and shares of K by estimated cycles of the busiest SM.
@@ -571,8 +832,14 @@ Plan make_plan(int M, int N, int K, int sms, int force_tn, int force_splits) {
     auto up = [](long long v) { return (v + 255) / 256 * 256; };
     best.pitch = (K + 15) / 16 * 16;
     best.planes = 0;
-    best.exps = up(4ll * M * best.pitch);
-    best.counters = best.exps + up(4ll * M);
+    best.words = up(4ll * M * best.pitch);
+    best.norms = best.words + up(4ll * best.tiles_m * best.tn);      // the epilogue reads the words of whole tiles
+    best.outliers = best.norms + up(4ll * ROW_WARPS * M);
+    best.squares = best.outliers + up(8ll * MAX_OUTLIERS * M);
+    best.features = best.squares + up(16ll * best.tiles * best.tn);
+    best.again = best.features + up(32ll * best.tiles * best.splits);
+    best.decided = best.again + up(8ll * best.tiles * best.splits);
+    best.counters = best.decided + up(best.splits > 1 ? 4ll * best.tiles * best.splits : 0);
     best.partial = best.counters + up(best.splits > 1 ? 4ll * best.tiles : 0);
     best.bytes = best.partial + (best.splits > 1 ? 8ll * best.splits * best.tiles * best.tn * FEATURES : 0);
     return best;
@@ -594,23 +861,23 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mb, const FixedParams& p, c
 
 // Rows of up to 4,096 elements hold two pieces a thread (three blocks fit on an SM), longer ones ten.
 template <bool PLANES>
-cudaError_t launch_rows(bool vec, const float* a, long long lda, int rows, int K, int* exps, uint8_t* planes, long long plane_stride, int pitch,
+cudaError_t launch_rows(bool vec, const float* a, long long lda, int rows, int K, int* words, float* norms, int2* outliers, uint8_t* planes, long long plane_stride, int pitch,
                         int* counters, int n_counters, cudaStream_t stream) {
     const bool brief = K <= 2 * 4 * ROW_THREADS;
     auto kernel = vec ? (brief ? fixed_rows_kernel<PLANES, true, 2> : fixed_rows_kernel<PLANES, true, 10>)
                       : (brief ? fixed_rows_kernel<PLANES, false, 2> : fixed_rows_kernel<PLANES, false, 10>);
-    return pyre_launch(kernel, dim3(rows), dim3(ROW_THREADS), (size_t)0, stream, a, lda, K, exps, planes, plane_stride, pitch, counters, n_counters);
+    return pyre_launch(kernel, dim3(rows), dim3(ROW_THREADS), (size_t)0, stream, a, lda, K, words, norms, outliers, planes, plane_stride, pitch, counters, n_counters);
 }
 }  // namespace
 
 // The sizes that `pyre_fixed_linear` takes: sums of at most 3 K 2^14 in 32 bits, TMA rows on 16-byte boundaries.
 static bool fixed_ok(const void* w, long long ldw, int K) { return K > 0 && K <= 40960 && ldw % 4 == 0 && !((uintptr_t)w & 15); }
 
-// The exponents of a weight's rows, worked out once: exps[N].
-PYRE_API int pyre_fixed_exponents(const float* w, long long ldw, int N, int K, int* exps, cudaStream_t stream) {
+// The exponents of a weight's rows, 1000 for one without a scale, and the squares of their norms over their scales, worked out once.
+PYRE_API int pyre_fixed_exponents(const float* w, long long ldw, int N, int K, int* exps, float* norms, cudaStream_t stream) {
     if (N <= 0) return 0;
     if (!fixed_ok(w, ldw, K)) return PYRE_ERR_UNSUPPORTED;
-    const cudaError_t e = launch_rows<false>(K % 4 == 0, w, ldw, N, K, exps, nullptr, 0, 0, nullptr, 0, stream);
+    const cudaError_t e = launch_rows<false>(K % 4 == 0, w, ldw, N, K, exps, norms, nullptr, nullptr, 0, 0, nullptr, 0, stream);
     if (e != cudaSuccess) return (int)e;
     PYRE_LAUNCH_CHECK();
     return 0;
@@ -623,7 +890,7 @@ PYRE_API long long pyre_fixed_workspace(int M, int N, int K, int tn, int splits)
     return pl.tn ? pl.bytes : -1;
 }
 
-PYRE_API int pyre_fixed_linear(const float* A, long long lda, const float* W, long long ldw, const int* w_exp, float* C, long long ldc,
+PYRE_API int pyre_fixed_linear(const float* A, long long lda, const float* W, long long ldw, const int* w_exp, const float* w_norm, float* C, long long ldc,
                                int M, int N, int K, void* workspace, long long workspace_bytes, int tn, int splits, int* err_flag, cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (!fixed_ok(W, ldw, K) || ((uintptr_t)workspace & 255)) return PYRE_ERR_UNSUPPORTED;
@@ -648,11 +915,13 @@ PYRE_API int pyre_fixed_linear(const float* A, long long lda, const float* W, lo
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) return PYRE_ERR_BAD_ARG;
     }
     const bool vec = K % 4 == 0 && lda % 4 == 0 && !((uintptr_t)A & 15);
-    int* a_exp = (int*)(ws + pl.exps);
+    int* words = (int*)(ws + pl.words);
+    float* norms = (float*)(ws + pl.norms);
+    int2* outliers = (int2*)(ws + pl.outliers);
     int* counters = (int*)(ws + pl.counters);
-    const cudaError_t e = launch_rows<true>(vec, A, lda, M, K, a_exp, ws + pl.planes, (long long)pl.pitch * M, pl.pitch, counters, pl.splits > 1 ? pl.tiles : 0, stream);
+    const cudaError_t e = launch_rows<true>(vec, A, lda, M, K, words, norms, outliers, ws + pl.planes, (long long)pl.pitch * M, pl.pitch, counters, pl.splits > 1 ? pl.tiles : 0, stream);
     if (e != cudaSuccess) return (int)e;
-    FixedParams p = {A, W, w_exp, a_exp, C, lda, ldw, ldc, M, N, K, pl.tiles_m, pl.tiles, pl.splits, pl.steps_per_split,
+    FixedParams p = {A, W, w_exp, words, outliers, w_norm, norms, (float4*)(ws + pl.squares), (float2*)(ws + pl.features), (int*)(ws + pl.decided), (unsigned long long*)(ws + pl.again), C, lda, ldw, ldc, M, N, K, pl.tiles_m, pl.tiles, pl.splits, pl.steps_per_split,
                      (long long*)(ws + pl.partial), counters, err_flag};
     int rc;
     switch (pl.tn) {

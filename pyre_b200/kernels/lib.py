@@ -40,9 +40,9 @@ SIGNATURES: dict[str, tuple[str, list]] = {
     "pyre_sample_slices": ("sampling", [I]),
     "pyre_paged_attention_generic": ("attention_generic", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, F, F, P, I, LL, P, I, I, P]),
     "pyre_sgemm_nt": ("gemm_f32", [P, LL, P, LL, P, LL, P, I, I, I, P]),
-    "pyre_fixed_exponents": ("gemm_fixed", [P, LL, I, I, P, P]),
+    "pyre_fixed_exponents": ("gemm_fixed", [P, LL, I, I, P, P, P]),
     "pyre_fixed_workspace": ("gemm_fixed", [I, I, I, I, I]),
-    "pyre_fixed_linear": ("gemm_fixed", [P, LL, P, LL, P, P, LL, I, I, I, P, LL, I, I, P, P]),
+    "pyre_fixed_linear": ("gemm_fixed", [P, LL, P, LL, P, P, P, LL, I, I, I, P, LL, I, I, P, P]),
     "pyre_paged_attention_mma": ("attention_mma", [P, P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, I, LL, I, P, P]),
     "pyre_attention_prefill_tc": ("attention_tc", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, LL, I, I, F, F, P, I, I, P, P, P, P]),
     "pyre_attention_prefill": ("attention_prefill", [P, P, P, P, I, P, P, I, I, I, I, I, I, I, I, F, F, P, I, LL, P, P]),

@@ -780,18 +780,21 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, bias: "torch.Tensor | None" = Non
 # 33 MB and more win back with the rows of a prompt or, from a hundred megabytes on, with their stream (us, CUDA cores / fixed
 # point: 4 x 4608 x 3584 15.7 / 19.8, 64 rows 81 / 34; 4 x 3584 x 3584 15.0 / 17.2, 64 rows 64 / 35; 4 x 37888 x 3584 118 / 95).
 FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_N, FIXED_MIN_SIZE = 512, 40960, 128, 1 << 23
+FIXED_NO_SCALE = 1000      # the exponent of a feature without a scale (csrc/gemm_fixed.cu)
 
 
 class FixedWeight:
-    """A float32 weight [N, K] and the exponent of each row's largest element (int32 [N]), which ``fixed_linear`` puts the
-    row on a fixed-point scale with.  The exponents are worked out once, when a part takes its tensors (``linear_weight``); the weight
+    """A float32 weight [N, K] and, of each row, the exponent of its largest element (int32 [N]), which ``fixed_linear`` puts the
+    row on a fixed-point scale with, and the square of its norm on that scale (float32 [N]).  They are worked out once, when a part takes its tensors (``linear_weight``); the weight
     itself stays as it is and is shared, not copied; one that is changed in place needs a new ``FixedWeight``."""
 
     def __init__(self, w: torch.Tensor):
         self.w = w
         self.exponents = torch.empty(w.shape[0], dtype=torch.int32, device=w.device)
+        self.norms = torch.empty(w.shape[0], dtype=torch.float32, device=w.device)
         with torch.cuda.device(w.device):      # a model may be loaded while another device is current
-            lib.call("pyre_fixed_exponents", w.data_ptr(), w.stride(0), w.shape[0], w.shape[1], self.exponents.data_ptr(), _stream())
+            lib.call("pyre_fixed_exponents", w.data_ptr(), w.stride(0), w.shape[0], w.shape[1], self.exponents.data_ptr(),
+                     self.norms.data_ptr(), _stream())
             # products read weights and exponents before they wait for the kernels in front of them (programmatic dependent launch)
             torch.cuda.current_stream().synchronize()
 
@@ -817,8 +820,11 @@ def fixed_supported(w: torch.Tensor) -> bool:
 
 def linear_weight(w: torch.Tensor) -> "torch.Tensor | FixedWeight":
     """A weight as ``linear`` wants it: float32 matrices that the fixed-point product takes with their rows' exponents, others as
-    they are."""
-    return FixedWeight(w) if fixed_supported(w) else w
+    they are; so are those of which more than one feature in 64 has no scale (an element far above the rest of its row)."""
+    if not fixed_supported(w):
+        return w
+    fixed = FixedWeight(w)
+    return fixed if int((fixed.exponents >= FIXED_NO_SCALE).sum()) <= w.shape[0] // 64 else w
 
 
 def product_libraries(dtype: torch.dtype) -> "list[str]":
@@ -842,8 +848,8 @@ def fixed_linear(a: torch.Tensor, w: FixedWeight, plan: "tuple[int, int]" = (0, 
     if size < 0:
         raise UnsupportedSize(f"no plan {plan} for a product of {M} rows")
     work = torch.empty(size, dtype=torch.uint8, device=a.device)
-    lib.call("pyre_fixed_linear", a.data_ptr(), a.stride(0), w.w.data_ptr(), w.w.stride(0), w.exponents.data_ptr(), out.data_ptr(), out.stride(0),
-             M, N, K, work.data_ptr(), size, plan[0], plan[1], device_error_flag(a.device).data_ptr(), _stream())
+    lib.call("pyre_fixed_linear", a.data_ptr(), a.stride(0), w.w.data_ptr(), w.w.stride(0), w.exponents.data_ptr(), w.norms.data_ptr(),
+             out.data_ptr(), out.stride(0), M, N, K, work.data_ptr(), size, plan[0], plan[1], device_error_flag(a.device).data_ptr(), _stream())
     return out
 
 

@@ -111,6 +111,70 @@ def test_whole_tiles_without_a_scale(ops, M, N, K, plan):
     ops.check_device_errors()
 
 
+def error(x, want):
+    return float((x.double() - want).norm() / want.norm())
+
+
+@pytest.mark.parametrize("r", [1.0, 30.0, 300.0, 1e3, 1e4, 1e6, 1e25])
+@pytest.mark.parametrize("columns", [1, 40])
+def test_outliers_cost_no_bits(ops, r, columns):
+    """Columns of the activations r times the others, those columns of the weights by as much less: the error of the sums in 32 bits bounds
+    it, whatever r and however many (as many as a row lists, and more); a row's bits depend on neither plan nor batch."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a, w = torch.randn(70, 3584, device="cuda", generator=g), torch.randn(512, 3584, device="cuda", generator=g)
+    a[:, 7:7 + columns] *= r
+    w[:, 7:7 + columns] /= r
+    W, want = ops.FixedWeight(w), a.double() @ w.double().t()
+    got, sums = ops.fixed_linear(a, W), ops.sgemm_nt(a, w)
+    assert error(got, want) <= error(sums, want)
+    assert max(error(x, y) for x, y in zip(got, want)) <= max(error(x, y) for x, y in zip(sums, want))
+    for plan in [(8, 1), (16, 3), (32, 1), (48, 2), (64, 7)]:
+        assert torch.equal(ops.fixed_linear(a, W, plan), got), plan
+    assert torch.equal(ops.fixed_linear(a[33:34], W), got[33:34])
+    ops.check_device_errors()
+
+
+def test_rows_of_wide_range(ops):
+    """Outliers of several magnitudes in one row, as many as a row's list holds and one more, rows of few elements, features with an
+    outlier of their own: each row within the error of the sums in 32 bits."""
+    g = torch.Generator(device="cuda").manual_seed(4)
+    K = 2052
+    a, w = torch.randn(12, K, device="cuda", generator=g), torch.randn(384, K, device="cuda", generator=g)
+    a[0, [5, 1700, 2051]] = torch.tensor([1e12, -1e3, 1e6], device="cuda")      # they never reach the result
+    w[:, [5, 1700, 2051]] *= torch.tensor([1e-12, 1e-3, 1e-6], device="cuda")
+    a[1, :16] = 1e9
+    a[2, :17] = 1e9
+    w[:, :17] *= 1e-9
+    a[3] = torch.where(torch.rand(K, device="cuda", generator=g) < 0.995, 0.0, a[3])
+    a[4] = 0
+    a[4, [40, 2000]] = torch.tensor([1.0, 1e-10], device="cuda")
+    a[5] = 0
+    a[5, 100] = 7.5
+    a[6] *= torch.exp(3 * torch.randn(K, device="cuda", generator=g))
+    a[7] *= torch.exp2(torch.randint(-30, 30, (K,), device="cuda", generator=g).float())
+    a[8, 1000:1010] *= 1e-30
+    w[200, 99], w[201, 1001] = 1e5, 1e-5
+    a[9, 99] = 1e-5
+    W, want = ops.FixedWeight(w), a.double() @ w.double().t()
+    assert int((W.exponents >= 1000).sum()) >= 1      # the feature with an outlier
+    got, sums = ops.fixed_linear(a, W), ops.sgemm_nt(a, w)
+    ops.check_device_errors()
+    for t in range(12):
+        assert error(got[t], want[t]) <= max(error(sums[t], want[t]), 4e-8), t
+    assert torch.equal(ops.fixed_linear(a, W, (16, 4)), got)
+    for t in range(12):
+        assert torch.equal(ops.fixed_linear(a[t:t + 1], W)[0], got[t]), t
+
+
+def test_weights_of_wide_range_stay_on_the_cuda_cores(ops):
+    """A few features without a scale are the kernel's to see to; a weight with more of them is not taken."""
+    w = torch.randn(16384, 512, device="cuda")
+    w[:256, 3] = 1e3
+    assert isinstance(ops.linear_weight(w), ops.FixedWeight)
+    w[256, 3] = 1e3
+    assert ops.linear_weight(w) is w
+
+
 def test_which_weights_take_it(ops):
     """The rule knows the weight alone: small ones, short rows, few features and rows off 16-byte boundaries stay with the CUDA cores'
     product."""
