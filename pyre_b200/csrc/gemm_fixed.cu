@@ -20,7 +20,7 @@
 // All are facts of the row and the weight alone, so that a row's result does not depend on what else is in the batch.
 // Against 64 bits (2-norm of the error over 2-norm of the result, this / the sums of gemm_f32.cu): normal operands
 // 2.5e-8 / 1.0e-7 (K = 512), 1.2e-7 (3,584), 1.8e-7 (18,944); 1 to 200 columns of A 16 to 1e25 times the others and those of W by as much
-// less 2.5e-8 to 7.8e-8 / the same; log-normal activations up to e^(3 x) 2.4e-8 to 4.5e-8 / 0.8e-7 to 2.2e-7; where they come nearest, a share of 0.7 of A's
+// less 2.5e-8 to 7.8e-8 / the same; log-normal activations up to e^(3 x) 2.5e-8 to 5.1e-8 / 0.9e-7 to 1.9e-7; where they come nearest, a share of 0.7 of A's
 // columns a hundredth and the rest of W's, 1.0e-7 / 1.0e-7 (512), 1.1e-7 / 1.2e-7 (3,584).
 // What it costs, us: ordinary and heavy-tailed rows nothing measurable from 64 rows on, 0.7 to 2.5 of 19 to 98 for 1 to 4 rows; per output and
 // outlier 7 ps (509 x 37,888 x 3,584: 770, with four columns of outliers 1,310); outputs made again some 13 multiplications a cycle and SM (all of the same

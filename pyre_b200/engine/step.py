@@ -99,6 +99,7 @@ class _DecodeGraph:
     ctx: StepContext
     graph: "torch.cuda.CUDAGraph"
     logits: torch.Tensor
+    weights: list = field(default_factory=list)      # ``FixedWeight``s that the launches read
     replays: int = 0
 
 
@@ -339,6 +340,7 @@ class Stepper:
 
     # ------------------------------------------------------------------ captured decode steps
     def _graph_step(self, entries: Sequence[StepEntry], reserve: bool, fed_from: "torch.Tensor | None" = None) -> torch.Tensor:
+        from ..kernels import ops
         cache = self.cache
         need = 1
         for e in entries:
@@ -366,14 +368,16 @@ class Stepper:
             if self._graph_pool is None:
                 self._graph_pool = torch.cuda.graph_pool_handle()
             torch.cuda.synchronize()
-            with torch.cuda.graph(graph, pool=self._graph_pool):
+            with ops.fixed_weights_used() as weights, torch.cuda.graph(graph, pool=self._graph_pool):
                 logits = self.model.forward(ctx)
             self.launches_per_graph[key] = lib.launch_count - before
-            self._graphs[key] = _DecodeGraph(flat_dev, ctx, graph, logits)
+            self._graphs[key] = _DecodeGraph(flat_dev, ctx, graph, logits, list(weights))
             result = eager_logits[:n]
             self.graph_captures += 1
             self.capture_seconds += time.perf_counter() - t_capture
         else:
+            for w in g.weights:
+                w.follow()
             self._copy_flat(g.flat_dev, flat)
             self._feed(g.ctx, entries, fed_from)     # outside the graph: writes the static token array before the replay
             g.graph.replay()

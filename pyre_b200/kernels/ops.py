@@ -13,8 +13,10 @@ pyre/model.py:84-87,133-135,172).  See ``linear``.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import functools
+import threading
 
 import torch
 
@@ -785,18 +787,30 @@ FIXED_NO_SCALE = 1000      # the exponent of a feature without a scale (csrc/gem
 
 class FixedWeight:
     """A float32 weight [N, K] and, of each row, the exponent of its largest element (int32 [N]), which ``fixed_linear`` puts the
-    row on a fixed-point scale with, and the square of its norm on that scale (float32 [N]).  They are worked out once, when a part takes its tensors (``linear_weight``); the weight
-    itself stays as it is and is shared, not copied; one that is changed in place needs a new ``FixedWeight``."""
+    row on a fixed-point scale with, and the square of its norm on that scale (float32 [N]).  They are worked out when a part takes its tensors (``linear_weight``); the weight
+    itself stays as it is and is shared, not copied.  One that is changed in place (its version counter says so) has them worked out again,
+    into the same memory, by the next product or replay of a captured step (``fixed_weights_used``) that reads it."""
 
     def __init__(self, w: torch.Tensor):
         self.w = w
         self.exponents = torch.empty(w.shape[0], dtype=torch.int32, device=w.device)
         self.norms = torch.empty(w.shape[0], dtype=torch.float32, device=w.device)
+        self.refresh()
+
+    def refresh(self) -> None:
+        """Work exponents and norms out from the weight as it is."""
+        w = self.w
+        self.version = w._version
         with torch.cuda.device(w.device):      # a model may be loaded while another device is current
             lib.call("pyre_fixed_exponents", w.data_ptr(), w.stride(0), w.shape[0], w.shape[1], self.exponents.data_ptr(),
                      self.norms.data_ptr(), _stream())
             # products read weights and exponents before they wait for the kernels in front of them (programmatic dependent launch)
             torch.cuda.current_stream().synchronize()
+
+    def follow(self) -> None:
+        """``refresh`` if the weight has been changed in place."""
+        if self.w._version != self.version:
+            self.refresh()
 
     @property
     def shape(self):
@@ -813,8 +827,8 @@ class FixedWeight:
 
 def fixed_supported(w: torch.Tensor) -> bool:
     """Does ``fixed_linear`` take this weight?  The rule knows the weight alone, never the number of rows that meet it: a row's
-    result is the same in every batch."""
-    return (w.is_cuda and w.dtype == torch.float32 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0
+    result is the same in every batch.  (A tensor made in inference mode has no version counter, so its exponents could not follow it.)"""
+    return (not w.is_inference() and w.is_cuda and w.dtype == torch.float32 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0
             and FIXED_MIN_K <= w.shape[1] <= FIXED_MAX_K and w.shape[0] >= FIXED_MIN_N and w.numel() >= FIXED_MIN_SIZE)
 
 
@@ -832,6 +846,23 @@ def product_libraries(dtype: torch.dtype) -> "list[str]":
     return ["gemm_f32", "gemm_fixed"] if dtype == torch.float32 else ["gemm_tc"]
 
 
+_fixed_used = threading.local()
+
+
+@contextlib.contextmanager
+def fixed_weights_used():
+    """``with fixed_weights_used() as weights:`` collects the ``FixedWeight``s of the products that this thread launches inside.  A captured
+    step keeps them: its products are not asked for again, so whoever replays it calls their ``follow`` first."""
+    outer = getattr(_fixed_used, "weights", None)
+    _fixed_used.weights = mine = {}
+    try:
+        yield mine.values()
+    finally:
+        _fixed_used.weights = outer
+        if outer is not None:
+            outer.update(mine)
+
+
 def fixed_linear(a: torch.Tensor, w: FixedWeight, plan: "tuple[int, int]" = (0, 0)) -> torch.Tensor:
     """C = A W^T of float32 operands on the tensor cores in fixed point: rows on power-of-two scales, integers of 31 bits as
     four bytes, exact sums, one rounding (csrc/gemm_fixed.cu).  A row's result is bit-identical for any number of rows.
@@ -843,6 +874,10 @@ def fixed_linear(a: torch.Tensor, w: FixedWeight, plan: "tuple[int, int]" = (0, 
     N, K2 = w.shape
     if K != K2:
         raise ValueError(f"inner sizes differ: a is [{M}, {K}], w is [{N}, {K2}]")
+    w.follow()
+    used = getattr(_fixed_used, "weights", None)
+    if used is not None:
+        used[id(w)] = w
     out = torch.empty((M, N), dtype=torch.float32, device=a.device)
     size = lib.call_value("pyre_fixed_workspace", M, N, K, plan[0], plan[1])
     if size < 0:

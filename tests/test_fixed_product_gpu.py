@@ -175,6 +175,49 @@ def test_weights_of_wide_range_stay_on_the_cuda_cores(ops):
     assert ops.linear_weight(w) is w
 
 
+def test_a_weight_changed_in_place(ops):
+    """The exponents follow the weight: elements that outgrow them, rows that get an infinity or lose their outlier, through a view too; a
+    tensor without a version counter is not taken."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    a, w = torch.randn(9, 1024, device="cuda", generator=g), torch.randn(8192, 1024, device="cuda", generator=g)
+    w[3, 4] = 1e4
+    W = ops.linear_weight(w)
+    ops.linear(a, W)
+    for change in (lambda: w[5].mul_(1e6), lambda: w.mul_(1e-5), lambda: w[7, 7].fill_(float("inf")), lambda: w[3, 4].zero_(), lambda: w.view(-1)[9].fill_(1e9)):
+        change()
+        assert torch.equal(ops.linear(a, W), ops.fixed_linear(a, ops.FixedWeight(w.clone())))
+    ops.check_device_errors()
+    with torch.inference_mode():
+        plain = torch.zeros(8192, 1024, device="cuda")
+    assert ops.linear_weight(plain) is plain
+
+
+def test_a_captured_step_follows_a_weight_changed_in_place(ops):
+    """Decode steps replayed from a graph against the same steps launched one by one, with weights edited between them."""
+    from pyre_b200 import Engine
+    from pyre_b200.config import config_from_dict
+    from pyre_b200.engine.step import StepEntry
+    raw = dict(architectures=["Qwen2ForCausalLM"], tie_word_embeddings=False, hidden_size=512, intermediate_size=16384, num_hidden_layers=1,
+               num_attention_heads=8, num_key_value_heads=2, head_dim=64, vocab_size=512, rope_theta=10000.0, rms_norm_eps=1e-6,
+               max_position_embeddings=256)
+    got = {}
+    for graphs in (True, False):
+        engine = Engine(config=config_from_dict(raw), seed=1, dtype="float32", max_cache_tokens=256, max_num_seqs=2, cuda_graphs=graphs)
+        ffn = engine.model.blocks[0].ffn
+        assert isinstance(ffn.w_down, ops.FixedWeight)
+        engine.cache.begin(0)
+        rows = got[graphs] = []
+        for k in range(6):
+            rows.append(engine.stepper.step([StepEntry(0, [k], [0])]).clone())
+            if k == 2:
+                ffn.w_down.w[:100].mul_(1e4)
+            if k == 4:
+                ffn.w_gate_up.w.mul_(0.01)
+        engine.stepper.check_device_errors()
+        assert (engine.stepper.graph_replays > 3) == graphs
+    assert all(torch.equal(x, y) for x, y in zip(got[True], got[False]))
+
+
 def test_which_weights_take_it(ops):
     """The rule knows the weight alone: small ones, short rows, few features and rows off 16-byte boundaries stay with the CUDA cores'
     product."""
