@@ -782,6 +782,7 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, bias: "torch.Tensor | None" = Non
 # 33 MB and more win back with the rows of a prompt or, from a hundred megabytes on, with their stream (us, CUDA cores / fixed
 # point: 4 x 4608 x 3584 15.7 / 19.8, 64 rows 81 / 34; 4 x 3584 x 3584 15.0 / 17.2, 64 rows 64 / 35; 4 x 37888 x 3584 118 / 95).
 FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_N, FIXED_MIN_SIZE = 512, 40960, 128, 1 << 23
+FIXED_SCRATCH = 256 << 20      # bytes of byte planes that a product may hold: more rows go in portions (of 3,500 rows where K is 18,944)
 FIXED_NO_SCALE = 1000      # the exponent of a feature without a scale (csrc/gemm_fixed.cu)
 
 
@@ -879,12 +880,17 @@ def fixed_linear(a: torch.Tensor, w: FixedWeight, plan: "tuple[int, int]" = (0, 
     if used is not None:
         used[id(w)] = w
     out = torch.empty((M, N), dtype=torch.float32, device=a.device)
-    size = lib.call_value("pyre_fixed_workspace", M, N, K, plan[0], plan[1])
-    if size < 0:
+    # the planes are four bytes an element; a portion is a multiple of 64 rows, the widest tile
+    most = max(64, FIXED_SCRATCH // (4 * K) // 64 * 64)
+    portions = [(0, M)] if M <= most else [(r, min(most, M - r)) for r in range(0, M, most)]
+    sizes = [lib.call_value("pyre_fixed_workspace", m, N, K, plan[0], plan[1]) for _, m in portions]
+    if min(sizes) < 0:
         raise UnsupportedSize(f"no plan {plan} for a product of {M} rows")
-    work = torch.empty(size, dtype=torch.uint8, device=a.device)
-    lib.call("pyre_fixed_linear", a.data_ptr(), a.stride(0), w.w.data_ptr(), w.w.stride(0), w.exponents.data_ptr(), w.norms.data_ptr(),
-             out.data_ptr(), out.stride(0), M, N, K, work.data_ptr(), size, plan[0], plan[1], device_error_flag(a.device).data_ptr(), _stream())
+    work = torch.empty(max(sizes), dtype=torch.uint8, device=a.device)
+    for (r, m), size in zip(portions, sizes):
+        lib.call("pyre_fixed_linear", a.data_ptr() + 4 * r * a.stride(0), a.stride(0), w.w.data_ptr(), w.w.stride(0), w.exponents.data_ptr(),
+                 w.norms.data_ptr(), out.data_ptr() + 4 * r * N, N, m, N, K, work.data_ptr(), size, plan[0], plan[1],
+                 device_error_flag(a.device).data_ptr(), _stream())
     return out
 
 

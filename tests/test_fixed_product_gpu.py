@@ -218,6 +218,16 @@ def test_a_captured_step_follows_a_weight_changed_in_place(ops):
     assert all(torch.equal(x, y) for x, y in zip(got[True], got[False]))
 
 
+def test_many_rows_go_in_portions(ops, monkeypatch):
+    """Scratch memory is bounded whatever the number of rows: portions give the same bits, of rows off 16-byte boundaries too."""
+    a, W = torch.randn(330, 1027, device="cuda")[:, 3:], ops.FixedWeight(torch.randn(300, 1024, device="cuda"))
+    whole = ops.fixed_linear(a, W)
+    for portion in (64, 128, 320):
+        monkeypatch.setattr(ops, "FIXED_SCRATCH", portion * 4 * 1024)
+        assert torch.equal(ops.fixed_linear(a, W), whole)
+    ops.check_device_errors()
+
+
 def test_which_weights_take_it(ops):
     """The rule knows the weight alone: small ones, short rows, few features and rows off 16-byte boundaries stay with the CUDA cores'
     product."""
