@@ -781,7 +781,7 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, bias: "torch.Tensor | None" = Non
 # Weights this large go to the fixed-point product.  Its second kernel and the shares of K cost a few rows some 4 us, which weights of
 # 33 MB and more win back with the rows of a prompt or, from a hundred megabytes on, with their stream (us, CUDA cores / fixed
 # point: 4 x 4608 x 3584 15.7 / 19.8, 64 rows 81 / 34; 4 x 3584 x 3584 15.0 / 17.2, 64 rows 64 / 35; 4 x 37888 x 3584 118 / 95).
-FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_N, FIXED_MIN_SIZE = 512, 40960, 128, 1 << 23
+FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_SIZE = 512, 40960, 1 << 23      # so at least 205 features
 FIXED_SCRATCH = 256 << 20      # bytes of byte planes that a product may hold: more rows go in portions (of 3,500 rows where K is 18,944)
 FIXED_NO_SCALE = 1000      # the exponent of a feature without a scale (csrc/gemm_fixed.cu)
 
@@ -830,7 +830,7 @@ def fixed_supported(w: torch.Tensor) -> bool:
     """Does ``fixed_linear`` take this weight?  The rule knows the weight alone, never the number of rows that meet it: a row's
     result is the same in every batch.  (A tensor made in inference mode has no version counter, so its exponents could not follow it.)"""
     return (not w.is_inference() and w.is_cuda and w.dtype == torch.float32 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 4 == 0 and w.data_ptr() % 16 == 0
-            and FIXED_MIN_K <= w.shape[1] <= FIXED_MAX_K and w.shape[0] >= FIXED_MIN_N and w.numel() >= FIXED_MIN_SIZE)
+            and w.stride(0) >= w.shape[1] and FIXED_MIN_K <= w.shape[1] <= FIXED_MAX_K and w.numel() >= FIXED_MIN_SIZE)
 
 
 def linear_weight(w: torch.Tensor) -> "torch.Tensor | FixedWeight":

@@ -111,6 +111,59 @@ def test_whole_tiles_without_a_scale(ops, M, N, K, plan):
     ops.check_device_errors()
 
 
+def digits(x):
+    """The signed bytes of a 31-bit integer, the largest first."""
+    out = []
+    for _ in range(3):
+        d = (x + 128) % 256 - 128
+        out.insert(0, d)
+        x = (x - d) // 256
+    return [x] + out
+
+
+@pytest.mark.parametrize("K", [512, 40960])
+def test_the_largest_sums_of_bytes(ops, K):
+    """Rows whose lower three bytes are all -128: the sums of 32 bits reach 3 K 2^14, 6 % below their limit at the longest K.  Compared with
+    exact integers."""
+    import numpy as np
+
+    one, rest = 1 << 29, -0x808080
+    assert digits(rest) == [0, -128, -128, -128] and digits(one) == [32, 0, 0, 0]
+    a, w = torch.full((3, K), rest * 2.0 ** -29, device="cuda"), torch.full((256, K), rest * 2.0 ** -29, device="cuda")
+    a[:, 5] = 1.0
+    w[:, 9] = 1.0
+    w[7] = -w[7]
+    w[7, 9] = 1.0
+
+    def total(rows):
+        s = [0] * 5
+        for x, y, times in rows:
+            for i, dx in enumerate(digits(x)):
+                for j, dy in enumerate(digits(y)):
+                    if i + j <= 4:
+                        s[i + j] += dx * dy * times
+        assert max(map(abs, s)) < 1 << 31
+        return sum(v << 8 * (4 - q) for q, v in enumerate(s))
+
+    want = [float(np.float32(total([(one, x, 1), (rest, one, 1), (rest, x, K - 2)]) * 2.0 ** -42)) for x in (rest, -rest)]
+    W = ops.FixedWeight(w)
+    assert not (W.exponents >= ops.FIXED_NO_SCALE).any()
+    for plan in [(0, 0), (64, 1)]:
+        got = ops.fixed_linear(a, W, plan)
+        assert (got[:, 7] == want[1]).all() and (got[:, torch.arange(256) != 7] == want[0]).all()
+    ops.check_device_errors()
+
+
+@pytest.mark.parametrize("K", [512, 3584, 18944])
+def test_error_of_normal_operands(ops, K):
+    """2-norm against 64 bits: 2.5e-8 is what the kernel's comment states, a quarter and less of what the sums in 32 bits have."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a, w = torch.randn(64, K, device="cuda", generator=g), torch.randn(512, K, device="cuda", generator=g)
+    want = a.double() @ w.double().t()
+    got = error(ops.fixed_linear(a, ops.FixedWeight(w)), want)
+    assert got < 2.7e-8 and got < 0.3 * error(ops.sgemm_nt(a, w), want)
+
+
 def error(x, want):
     return float((x.double() - want).norm() / want.norm())
 
@@ -229,12 +282,14 @@ def test_many_rows_go_in_portions(ops, monkeypatch):
 
 
 def test_which_weights_take_it(ops):
-    """The rule knows the weight alone: small ones, short rows, few features and rows off 16-byte boundaries stay with the CUDA cores'
-    product."""
+    """The rule knows the weight alone: small ones, short and overlong rows, rows off 16-byte boundaries and rows that overlap stay with the
+    CUDA cores' product."""
     def weight(N, K, ld=0):
         return torch.zeros(N, ld or K, device="cuda")[:, :K]
     assert isinstance(ops.linear_weight(weight(16384, 512)), ops.FixedWeight)
-    for w in (weight(16383, 512), weight(16600, 508), weight(127, 40960 * 2), weight(16384, 600, 601), weight(16384, 512).to(torch.bfloat16), weight(300, 40964)):
+    assert isinstance(ops.linear_weight(weight(205, 40960)), ops.FixedWeight)
+    for w in (weight(16383, 512), weight(16600, 508), weight(16384, 600, 601), weight(16384, 512).to(torch.bfloat16), weight(300, 40964),
+              weight(1, 1024).expand(8192, 1024)):
         assert ops.linear_weight(w) is w
     W = ops.FixedWeight(weight(128, 512))
     with pytest.raises(ValueError):
