@@ -22,7 +22,7 @@
 // 2.5e-8 / 1.0e-7 (K = 512), 1.2e-7 (3,584), 1.8e-7 (18,944); 1 to 200 columns of A 16 to 1e25 times the others and those of W by as much
 // less 2.5e-8 to 7.8e-8 / the same; log-normal activations up to e^(3 x) 2.5e-8 to 5.1e-8 / 0.9e-7 to 1.9e-7; where they come nearest, a share of 0.7 of A's
 // columns a hundredth and the rest of W's, 1.0e-7 / 1.0e-7 (512), 1.1e-7 / 1.2e-7 (3,584).
-// What it costs, us: ordinary and heavy-tailed rows nothing measurable from 64 rows on, 0.7 to 2.5 of 19 to 98 for 1 to 4 rows; per output and
+// What it costs, us: ordinary and heavy-tailed rows nothing measurable from 64 rows on, 0.5 to 2.3 of 18 to 97 for 1 to 4 rows; per output and
 // outlier 7 ps (509 x 37,888 x 3,584: 770, with four columns of outliers 1,310); outputs made again some 13 multiplications a cycle and SM (all of the same
 // product: 20,400; one row in 64: 330 for 115).
 //
@@ -49,7 +49,7 @@ constexpr int ERR_TIMEOUT = 2;
 constexpr int E_NONE = 1000;                   // of a row without a scale
 constexpr int E_MIN = -98;                     // of a row of zeros (its scale is a normal float)
 constexpr int OUTLIER_BITS = 7, WEIGHT_BITS = 6, MAX_OUTLIERS = 16;      // see above
-constexpr int ROW_THREADS = 512, ROW_WARPS = ROW_THREADS / 32;      // of the kernel in front
+constexpr int ROW_THREADS = 1024, ROW_WARPS = ROW_THREADS / 32;      // of the kernel in front
 constexpr int FEATURES = 128, STEP = 32, BLOCK_K = 128;
 constexpr int CONV_WARP0 = 4, GROUPS = 4, CONV_THREADS = GROUPS * 128, THREADS = CONV_WARP0 * 32 + CONV_THREADS;
 constexpr int W_BYTES = FEATURES * STEP * 4;   // a step's weights
@@ -659,7 +659,7 @@ fixed_gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 // per row; what bounds it is the chain of its latencies, so a thread asks for HELD pieces of four elements at once and keeps them (what a
 // longer row has beyond them is read again, out of the caches).
 template <bool PLANES, bool VEC, int HELD>
-__global__ void __launch_bounds__(ROW_THREADS, HELD == 2 ? 3 : 1)
+__global__ void __launch_bounds__(ROW_THREADS, HELD == 1 ? 2 : 1)
 fixed_rows_kernel(const float* A, long long lda, int K, int* words, float* norms, int2* outliers, uint8_t* planes, long long plane_stride, int pitch, int* counters, int n_counters) {
     __shared__ int4 s_stats[ROW_WARPS];
     __shared__ int2 s_list[MAX_OUTLIERS];
@@ -689,7 +689,7 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* words, float* norms
     int E, listed = 0;
     for (;;) {
         // of the others: the largest, the sum of their exponents, how many are not zero
-        uint32_t most = 0, both = 0;      // the sum below the count: a warp has at most 2,560 elements
+        uint32_t most = 0, both = 0;      // the sum below the count: a warp has at most 1,280 elements
         auto look = [&](float x) {
             const uint32_t u = magnitude(x);
             most = max(most, u);
@@ -711,19 +711,19 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* words, float* norms
         int sum, n;
         if ((tid & 31) == 0) s_stats[tid >> 5] = make_int4((int)most, (int)(both & 0xfffff), (int)(both >> 20), 0);
         __syncthreads();
-        const int4 others = (tid & 31) < ROW_WARPS ? s_stats[tid & 31] : make_int4(0, 0, 0, 0);
+        const int4 others = s_stats[tid & 31];
+        static_assert(ROW_WARPS == 32, "a lane for each warp's");
         most = __reduce_max_sync(0xffffffffu, (uint32_t)others.x);
         sum = __reduce_add_sync(0xffffffffu, others.y);
         n = __reduce_add_sync(0xffffffffu, others.z);
         E = row_exponent(most);
         if (E >= E_NONE || n == 0) break;
-        const int bound = sum / n + (PLANES ? OUTLIER_BITS : WEIGHT_BITS);
-        if ((int)(most >> 23) <= bound) break;
+        if (((int)(most >> 23) - (PLANES ? OUTLIER_BITS : WEIGHT_BITS)) * n <= sum) break;      // no more than the mean exponent and so many bits
         if (!PLANES) {
             E = E_NONE;
             break;
         }
-        const uint32_t from = (uint32_t)(bound + 1) << 23;      // at most the exponent of `most`
+        const uint32_t from = (uint32_t)(sum / n + OUTLIER_BITS + 1) << 23;      // at most the exponent of `most`
         for (int k = tid; k < K; k += ROW_THREADS) {
             const float x = a[k];
             const uint32_t u = magnitude(x);
@@ -859,13 +859,13 @@ int launch(const CUtensorMap& mw, const CUtensorMap& mb, const FixedParams& p, c
     return (int)pyre_launch(fixed_gemm_kernel<TN>, dim3(items < sms ? items : sms), dim3(THREADS), (size_t)L::TOTAL, stream, mw, mb, p);
 }
 
-// Rows of up to 4,096 elements hold two pieces a thread (three blocks fit on an SM), longer ones ten.
+// Rows of up to 4,096 elements hold a piece a thread (two blocks fit on an SM), longer ones five.
 template <bool PLANES>
 cudaError_t launch_rows(bool vec, const float* a, long long lda, int rows, int K, int* words, float* norms, int2* outliers, uint8_t* planes, long long plane_stride, int pitch,
                         int* counters, int n_counters, cudaStream_t stream) {
-    const bool brief = K <= 2 * 4 * ROW_THREADS;
-    auto kernel = vec ? (brief ? fixed_rows_kernel<PLANES, true, 2> : fixed_rows_kernel<PLANES, true, 10>)
-                      : (brief ? fixed_rows_kernel<PLANES, false, 2> : fixed_rows_kernel<PLANES, false, 10>);
+    const bool brief = K <= 4 * ROW_THREADS;
+    auto kernel = vec ? (brief ? fixed_rows_kernel<PLANES, true, 1> : fixed_rows_kernel<PLANES, true, 5>)
+                      : (brief ? fixed_rows_kernel<PLANES, false, 1> : fixed_rows_kernel<PLANES, false, 5>);
     return pyre_launch(kernel, dim3(rows), dim3(ROW_THREADS), (size_t)0, stream, a, lda, K, words, norms, outliers, planes, plane_stride, pitch, counters, n_counters);
 }
 }  // namespace
