@@ -743,7 +743,10 @@ fixed_rows_kernel(const float* A, long long lda, int K, int* words, float* norms
     auto scaled = [&](float x) { return none || magnitude(x) >= limit ? 0.f : x * sc.s2 * sc.s1; };
     auto square = [&](float x) { norm = fmaf(x, x, norm); };      // in units of 2^58
     if constexpr (!PLANES) {
-        for (int k = tid; k < K; k += ROW_THREADS) square(scaled(a[k]));
+        auto take = [&](const float4& v) { square(scaled(v.x)); square(scaled(v.y)); square(scaled(v.z)); square(scaled(v.w)); };
+#pragma unroll
+        for (int h = 0; h < HELD; ++h) take(held[h]);
+        for (int k = 4 * (tid + HELD * ROW_THREADS); k < K; k += 4 * ROW_THREADS) take(piece(k));
         norm = warp_sum(norm);
         __syncthreads();
         if ((tid & 31) == 0) s_stats[tid >> 5].x = __float_as_int(norm);

@@ -779,8 +779,10 @@ def sgemm_nt(a: torch.Tensor, w: torch.Tensor, bias: "torch.Tensor | None" = Non
 
 
 # Weights this large go to the fixed-point product.  Its second kernel and the shares of K cost a few rows some 4 us, which weights of
-# 33 MB and more win back with the rows of a prompt or, from a hundred megabytes on, with their stream (us, CUDA cores / fixed
-# point: 4 x 4608 x 3584 15.7 / 19.8, 64 rows 81 / 34; 4 x 3584 x 3584 15.0 / 17.2, 64 rows 64 / 35; 4 x 37888 x 3584 118 / 95).
+# 33 MB and more win back from 8 rows on, and those of some 200 MB and more with any (us, CUDA cores / fixed point).  4 rows: 3584 x 3584 14.6 / 16.2,
+# 4608 x 3584 15.1 / 19.1, 8192 x 2048 18.1 / 19.3, 10240 x 2560 30.0 / 32.6, 6144 x 2048 17.1 / 15.7, 3584 x 18944 69.7 / 55.3, 37888 x 3584 123 / 97;
+# 8 rows: 4608 x 3584 20.0 / 19.8, 3584 x 3584 19.6 / 17.1; 64 rows: 4608 x 3584 81 / 30.  So 1 to 4 rows lose up to 27 % on weights of 2^23 to 2^25 elements; which
+# kernel serves a product cannot depend on the number of rows (a row's bits would depend on the batch), and a prompt gains 3 to 4 times as much.
 FIXED_MIN_K, FIXED_MAX_K, FIXED_MIN_SIZE = 512, 40960, 1 << 23      # so at least 205 features
 FIXED_SCRATCH = 256 << 20      # bytes of byte planes that a product may hold: more rows go in portions (of 3,500 rows where K is 18,944)
 FIXED_NO_SCALE = 1000      # the exponent of a feature without a scale (csrc/gemm_fixed.cu)
@@ -792,13 +794,14 @@ class FixedWeight:
     itself stays as it is and is shared, not copied.  One that is changed in place (its version counter says so) has them worked out again,
     into the same memory, by the next product or replay of a captured step (``fixed_weights_used``) that reads it."""
 
-    def __init__(self, w: torch.Tensor):
+    def __init__(self, w: torch.Tensor, wait: bool = True):
+        """``wait=False``: the caller waits for the stream before any product takes the weight."""
         self.w = w
         self.exponents = torch.empty(w.shape[0], dtype=torch.int32, device=w.device)
         self.norms = torch.empty(w.shape[0], dtype=torch.float32, device=w.device)
-        self.refresh()
+        self.refresh(wait)
 
-    def refresh(self) -> None:
+    def refresh(self, wait: bool = True) -> None:
         """Work exponents and norms out from the weight as it is."""
         w = self.w
         self.version = w._version
@@ -806,7 +809,8 @@ class FixedWeight:
             lib.call("pyre_fixed_exponents", w.data_ptr(), w.stride(0), w.shape[0], w.shape[1], self.exponents.data_ptr(),
                      self.norms.data_ptr(), _stream())
             # products read weights and exponents before they wait for the kernels in front of them (programmatic dependent launch)
-            torch.cuda.current_stream().synchronize()
+            if wait:
+                torch.cuda.current_stream().synchronize()
 
     def follow(self) -> None:
         """``refresh`` if the weight has been changed in place."""
@@ -838,8 +842,9 @@ def linear_weight(w: torch.Tensor) -> "torch.Tensor | FixedWeight":
     they are; so are those of which more than one feature in 64 has no scale (an element far above the rest of its row)."""
     if not fixed_supported(w):
         return w
-    fixed = FixedWeight(w)
-    return fixed if int((fixed.exponents >= FIXED_NO_SCALE).sum()) <= w.shape[0] // 64 else w
+    with torch.cuda.device(w.device):
+        fixed = FixedWeight(w, wait=False)
+        return fixed if int((fixed.exponents >= FIXED_NO_SCALE).sum()) <= w.shape[0] // 64 else w      # reading the number waits
 
 
 def product_libraries(dtype: torch.dtype) -> "list[str]":
@@ -1061,8 +1066,9 @@ def gemm_tc(x: "torch.Tensor | ScaledRows", w: torch.Tensor, out_dtype: torch.dt
     if gated and gate not in GATE_KINDS:
         raise UnsupportedSize(f"gate activation {gate!r}: the product's epilogue knows {sorted(GATE_KINDS)}")
     if gated and plan is None and M == 128 and N % 256 == 0:
-        # exactly 128 tokens: 58.6 us with the weights on the rows, 52.4 so; with 72-120 tokens (a tile of token rows
-        # that is not full) this orientation takes 66 us and the other 54-58
+        # Exactly 128 tokens, us with the weights on the rows / so: 37888 x 3584 63.2 / 60.2, 27648 x 5120 74.5 / 63.2, 55296 x 5120
+        # 114.3 / 120.5.  With 65 it is 56.2 / 57.1, 65.0 / 61.0 and 104.6 / 115.7, with 120 63.5 / 60.8, 73.3 / 62.9 and 112.0 / 119.3: below 128 it goes by
+        # how the tiles of 256 features fill their rounds, which no rule here looks at.
         weights_as_rows, bn, splits = False, 256, 1
     if scaled is not None and weights_as_rows and (M > bn or bn > 128):      # more than one tile of at most 128 tokens on the narrow side: not served
         x, scaled = materialize(scaled), None
