@@ -555,8 +555,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
             };
             if constexpr (!X_CONTIGUOUS_OUT && BN == 256) {
                 if (p.gated) {
-                    // Rows beyond the tokens are all zeros, and silu's 0 / 2 takes the division's slow path: one such warp held its whole
-                    // tile up (500 x 37888 x 3584: 157 us against 105 for 512 rows, 107 so).
                     // the tile's columns are two blocks of 64 gate features followed by the 64 up features of the
                     // same indices: out[x, y0 / 2 + c] = silu(gate) * up, with the products rounded to bfloat16
                     // first (as a separate activation kernel would read them) and the rest in fp32
@@ -571,6 +569,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant_
                             tmem_ld16(acc + blk * 128 + cc, g);
                             tmem_ld16(acc + blk * 128 + 64 + cc, u);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                            // Rows beyond the tokens are all zeros, and silu's 0 / 2 takes the division's slow path: one such warp held its whole
+                            // tile up (500 x 37888 x 3584: 157 us against 105 for 512 rows, 107 so).
                             if (xr >= p.x_rows) {
 #pragma unroll
                                 for (int q = 0; q < 16; ++q) g[q] = __float_as_uint(1.f);
