@@ -871,7 +871,7 @@ def fixed_weights_used():
 
 def fixed_linear(a: torch.Tensor, w: FixedWeight, plan: "tuple[int, int]" = (0, 0)) -> torch.Tensor:
     """C = A W^T of float32 operands on the tensor cores in fixed point: rows on power-of-two scales, integers of 31 bits as
-    four bytes, exact sums, one rounding (csrc/gemm_fixed.cu).  A row's result is bit-identical for any number of rows.
+    four bytes, exact sums; outliers, and outputs that the scales would cost bits, from the float operands (csrc/gemm_fixed.cu).  A row's result is bit-identical for any number of rows.
     ``plan``: (tokens per tile, shares of K), 0 for the kernel's own choice."""
     if not a.is_cuda or a.dtype != torch.float32 or a.dim() != 2 or a.stride(1) != 1:
         raise ValueError("a must be a CUDA float32 matrix with contiguous rows")
