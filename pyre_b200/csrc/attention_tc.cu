@@ -54,7 +54,7 @@
 
 #include <cstring>
 
-#include "common.cuh"
+#include "tensor_core.cuh"
 
 namespace {
 
@@ -64,48 +64,8 @@ constexpr int THREADS = 224;   // warp 0: K producer, 1: MMA issuer, 2-5: one th
 constexpr int ERR_TIMEOUT = 4;
 constexpr float RESCALE_THRESHOLD = 8.0f;   // log2 units
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    for (uint32_t it = 1;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 63) == 0) {
-            if (*abort_flag) return false;
-            if (clock64() - t0 > PYRE_WAIT_CYCLES) break;
-        }
-    }
-    *abort_flag = 1;
-    if (err_flag) atomicExch(err_flag, ERR_TIMEOUT);
-    return false;
-}
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1) : "memory");
-}
-// K-major operand, 128-byte rows, 128B swizzle: LBO unused (1), SBO = 1024 B (eight rows).
-__device__ __forceinline__ uint64_t desc_k_major(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFF) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-           ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+    return mbar_wait_or<ERR_TIMEOUT>(bar, parity, abort_flag, err_flag);
 }
 // MN-major operand: each K row (a key) holds 64 MN elements (128 B, swizzled); eight rows form
 // an atom (SBO = 1024 B); the next 64 MN elements start `lbo` bytes further.
@@ -127,9 +87,6 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 // 32 bytes per thread in one request (sm_100: 256-bit global stores; the address is 32-byte aligned): whole sectors
 __device__ __forceinline__ void st_global_32B(void* ptr, const uint32_t* w) {
@@ -377,8 +334,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 for (int h = 0; h < HALVES; ++h)
 #pragma unroll
                     for (int j = 0; j < 4; ++j)   // HD / 16 steps of 16 dims; 4 steps per 128-byte column box
-                        umma_bf16(tmem_base + S_COL + st * BN, desc_k_major(base + L::OFF_Q + h * (BM * 128)) + 2 * j,
-                                  desc_k_major(kd + h * (BN * 128)) + 2 * j, idesc_s, (h > 0 || j > 0) ? 1u : 0u);
+                        umma_bf16(tmem_base + S_COL + st * BN, umma_desc(base + L::OFF_Q + h * (BM * 128)) + 2 * j,
+                                  umma_desc(kd + h * (BN * 128)) + 2 * j, idesc_s, (h > 0 || j > 0) ? 1u : 0u);
                 umma_commit(bar_s + 8 * st);
                 return true;
             };

@@ -46,7 +46,7 @@ LIBRARIES = {
     "matrix_state": "matrix_state.cu",
 }
 
-HEADERS = ["common.cuh", "attention_mma_noalloc.h"]
+HEADERS = ["common.cuh", "tensor_core.cuh", "attention_mma_noalloc.h"]
 # sources that a library's source includes (they count towards its fingerprint)
 INCLUDED_SOURCES = {"attention_mma_noalloc": ["attention_mma.cu"]}
 
